@@ -203,11 +203,13 @@ def run_steps(ctx, t0, n0, count, dt):
 
 def roofline(ctx, shape, nsteps):
     """Roofline of the dominant kernel class, the transport operator applications of the
-    inner BiCGStab (k_ti_v and k_ti_st). The library accumulates their algorithmic bytes per
-    launch: N x (six FP32 scaled off-diagonals 24 + per live right-hand side 4 bytes for each
-    vector read or written once: 12 for v = A p (p in, rhat in, v out; 16 on the first
-    iteration, which also stores p = r), 20 for s = r - alpha v, t = A s (r, v, rhat in; s, t
-    out)); one right-hand side is live in this workload (the acid field is zero)."""
+    inner BiCGStab on the red-black reduced system (two half sweeps each: k_rb_z + k_rb_v and
+    k_rb_zs + k_rb_t). The library accumulates their algorithmic bytes per application: N x (six
+    FP32 scaled off-diagonals 24 + per live right-hand side 2 bytes for each half-length vector
+    read or written once: 12 for z = O_r p, v = p - O_b z (p, z, rhat in twice or once; z, v
+    out; 14 on the first iteration, which also stores p = r), 18 for s = r - alpha v,
+    z = O_r s, t = s - O_b z); one right-hand side is live in this workload (the acid field is
+    zero)."""
     peaks_path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     peaks = json.load(open(peaks_path)) if os.path.exists(peaks_path) else None
     ms, cnt = ctx.timing_get("kry_apply")
@@ -217,13 +219,10 @@ def roofline(ctx, shape, nsteps):
     achieved = nbytes / (ms / 1e3) / 1e9
     peak, src = (peaks["hbm_gbs"], "measured") if peaks else (6800.0, "fallback")
     vox = shape[0] * shape[1] * shape[2]
-    # DRAM traffic per launch: dram__bytes_read.sum + dram__bytes_write.sum per voxel from one
-    # ncu capture of the 160x256x256 case (inputs > L2), k_ti_v_pair 35.13 B and k_ti_st_pair
-    # 42.42 B, scaled by the voxel count; the timed launches alternate the two kernels
-    traffic = 0.5 * (35.13 + 42.42) * vox
-    return {"bound": "hbm", "kernel": "transport operator apply (k_ti_v_pair, k_ti_st_pair)",
+    # no byte counters for these kernels: the traffic is taken as the algorithmic bytes
+    return {"bound": "hbm", "kernel": "transport operator apply (k_rb_z + k_rb_v, k_rb_zs + k_rb_t)",
             "achieved": round(achieved, 1), "peak": peak, "peak_source": src, "unit": "GB/s",
-            "frac": round(achieved / peak, 4), "traffic": round(traffic),
+            "frac": round(achieved / peak, 4), "traffic": round(nbytes / cnt),
             "bytes_per_launch": round(nbytes / cnt), "bytes_per_voxel": round(nbytes / cnt / vox, 2),
             "launches": cnt, "us_per_launch": round(ms * 1e3 / cnt, 2)}
 

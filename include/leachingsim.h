@@ -458,7 +458,7 @@ typedef enum ls_timer {
     LS_T_PRECIP = 7,
     LS_T_DISSOLVE = 8,
     LS_T_SNAPSHOT = 9,
-    LS_T_KRY_APPLY = 10,    /* each transport / implicit-saturation operator-apply launch */
+    LS_T_KRY_APPLY = 10,    /* each transport / implicit-saturation operator application */
     LS_T_CG_APPLY = 11,     /* each inner pressure operator-apply launch */
     LS_T_COUNT = 12
 } ls_timer;

@@ -265,11 +265,11 @@ static void lean_release_transport(ls_ctx* c) {
     const size_t n = (size_t)c->g.N;
     for (double*& q : c->tc) dfree_t(c, &q, n);
     for (double*& q : c->tb) dfree_t(c, &q, n);
-    for (float*& q : c->to) dfree_t(c, &q, n);
-    for (float*& q : c->trhs) dfree_t(c, &q, n);
+    for (float*& q : c->to) dfree_t(c, &q, 2 * (size_t)c->ti_half);
+    for (float*& q : c->trhs) dfree_t(c, &q, 2 * (size_t)c->ti_half + 2 * (size_t)c->ti_pad);
     dfree_t(c, &c->tinv, n);
     dfree_t(c, &c->tkind, n);
-    dfree_t(c, &c->ti, (size_t)c->ti_stride * 7);
+    dfree_t(c, &c->ti, (size_t)c->ti_stride * kTiVecs);
     c->t_valid = 0;
 }
 
@@ -690,7 +690,6 @@ ls_status ls_destroy(ls_ctx* c) {
     for (float* q : c->trhs) rel(q);
     rel(c->ti);
     rel(c->start_anchor);
-    rel(c->tcount);
     {
         void* lp[] = {c->lpc_c0, c->lpc_c1, c->lpc_c2, c->lpc_out, c->lpc_isd, c->lpc_anchor};
         for (void* q : lp) rel(q);

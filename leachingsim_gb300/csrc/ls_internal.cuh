@@ -26,6 +26,7 @@ __host__ __device__ __forceinline__ double smax(double a, double b) { return (a 
 
 constexpr int kBlock = 256;        // threads per block of the streaming kernels
 constexpr int kMaxPartials = 4096; // per-block partial results of one reduction
+constexpr int kTiVecs = 8;         // vectors of the transport's inner solve: r rh p v s t d z
 
 // Division of a 32-bit index by a fixed divisor through a multiply-high and a shift
 // (Granlund-Montgomery): q = umulhi(n, m) >> s, exact for every n < 2^31.
@@ -392,12 +393,12 @@ struct ls_ctx {
     // transport / implicit saturation (2 right-hand sides)
     double* tc[7];        // FP64 row coefficients: diagonal, then +i,-i,+j,-j,+k,-k
     double* tb[2];        // FP64 right-hand sides
-    float* to[6];         // FP32 off-diagonals scaled by the row diagonal
+    float* to[6];         // FP32 off-diagonals scaled by the row diagonal, black then red (ti_half each)
     double* tinv;         // FP64 1 / row diagonal
-    float* trhs[2];       // FP32 D^-1 (b - A x) per right-hand side
-    float* ti;            // FP32 inner vectors r rh p v s t d, padded, float or float2 rows
+    float* trhs[2];       // FP32 D^-1 (b - A x) per right-hand side, black then red, padded
+    float* ti;            // FP32 inner vectors r rh p v s t d z of one colour, padded, float or float2
+    long long ti_half;    // elements of one colour (virtual ones included)
     long long ti_pad, ti_stride;  // zero elements around each vector; floats per vector
-    unsigned int* tcount; // blocks done in the current transport reduction
     int8_t* tkind;        // 1 identity row, 2 coupled row
 
     // dissolution

@@ -19,7 +19,8 @@
 // once per solve, exactly as the reference assembles them; an FP64 refinement loop forms
 // the true residual r = b - A x and its Jacobi-scaled norm ||D^-1 r|| / ||D^-1 b|| (the
 // test PETSc applies to left-Jacobi GMRES); each correction comes from an FP32 BiCGStab on
-// the unit-diagonal system (D^-1 A) d = D^-1 r with FP32 scaled off-diagonals.
+// the red-black reduced form of the unit-diagonal system (D^-1 A) d = D^-1 r with FP32 scaled
+// off-diagonals.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -200,13 +201,60 @@ struct Rows {
     const double *fx, *fy, *fz, *s;
 };
 
+// Red-black layout of the inner FP32 system. The seven-point stencil couples a voxel only to
+// voxels of the other parity of i + j + k, so the voxels of each colour (0 black, 1 red) sit in
+// an array of their own, H = I J K2p elements: voxel (i, j, k) at (k >> 1) + K2p (j + J i),
+// K2p = ceil(K / 2) rounded up to 4 (16-byte chunks of a row never straddle rows; the elements
+// past a row's end are virtual: zero links, zero values). The neighbours of an element at h are
+// the other colour's elements at h -+ J K2p (i), h -+ K2p (j), and along k at h ("near") and at
+// h + 1 (odd k) or h - 1 (even k) ("far").
+struct RBGrid {
+    int I, J, K, K2p, JK2;
+    long long H;
+    FastDiv div4, div2, div_j;  // by K2p / 4, K2p / 2 and J
+};
+
+__host__ __device__ __forceinline__ int rb_index(const RBGrid& g, int i, int j, int k, int& colour) {
+    colour = (i + j + k) & 1;
+    return (k >> 1) + g.K2p * (j + g.J * i);
+}
+
+static RBGrid make_rb(const Grid& g) {
+    RBGrid r;
+    r.I = g.I;
+    r.J = g.J;
+    r.K = g.K;
+    r.K2p = (((g.K + 1) / 2 + 3) / 4) * 4;
+    r.JK2 = g.J * r.K2p;
+    r.H = (long long)g.I * r.JK2;
+    r.div4 = make_fastdiv((unsigned int)(r.K2p / 4));
+    r.div2 = make_fastdiv((unsigned int)(r.K2p / 2));
+    r.div_j = make_fastdiv((unsigned int)g.J);
+    return r;
+}
+
 struct TBuf {
     double* c[7];
     double* b[2];
-    float* o[6];
+    float* o[6];  // FP32 scaled links, black then red (H each): -i, -j, near, far, +j, +i
     double* inv;
     int8_t* kind;
+    RBGrid rb;
 };
+
+// the FP32 links of row (i, j, k) from its FP64 off-diagonals (+i,-i,+j,-j,+k,-k)
+__device__ __forceinline__ void store_links(const TBuf& tb, int i, int j, int k, const double off[6], float inv32) {
+    int colour;
+    const int h = rb_index(tb.rb, i, j, k, colour);
+    const long long at = colour * tb.rb.H + h;
+    const bool odd = k & 1;
+    tb.o[0][at] = d2f_rz(off[1]) * inv32;
+    tb.o[1][at] = d2f_rz(off[3]) * inv32;
+    tb.o[2][at] = d2f_rz(odd ? off[5] : off[4]) * inv32;
+    tb.o[3][at] = d2f_rz(odd ? off[4] : off[5]) * inv32;
+    tb.o[4][at] = d2f_rz(off[2]) * inv32;
+    tb.o[5][at] = d2f_rz(off[0]) * inv32;
+}
 
 template <typename L, bool EXPL>
 __global__ void __launch_bounds__(kBlock) k_t_setup(Rows<L> op, TBuf tb, int nrhs, const double* f0,
@@ -229,10 +277,8 @@ __global__ void __launch_bounds__(kBlock) k_t_setup(Rows<L> op, TBuf tb, int nrh
         tb.c[0][r] = dg;
         tb.inv[r] = inv;
 #pragma unroll
-        for (int d = 0; d < 6; ++d) {
-            tb.c[1 + d][r] = off[d];
-            tb.o[d][r] = d2f_rz(off[d]) * inv32;
-        }
+        for (int d = 0; d < 6; ++d) tb.c[1 + d][r] = off[d];
+        store_links(tb, i, j, k, off, inv32);
         tb.kind[r] = (int8_t)kind;
         for (int q = 0; q < nrhs; ++q) {
             tb.b[q][r] = rhs[q];
@@ -321,10 +367,8 @@ __global__ void __launch_bounds__(kBlock) k_t_rows(Rows<L> op, TBuf tb, const in
         tb.c[0][r] = dg;
         tb.inv[r] = inv;
 #pragma unroll
-        for (int d = 0; d < 6; ++d) {
-            tb.c[1 + d][r] = off[d];
-            tb.o[d][r] = d2f_rz(off[d]) * inv32;
-        }
+        for (int d = 0; d < 6; ++d) tb.c[1 + d][r] = off[d];
+        store_links(tb, i, j, k, off, inv32);
         tb.kind[r] = (int8_t)kind;
     }
 }
@@ -384,7 +428,8 @@ __device__ __forceinline__ double t_row_apply(const Grid& g, const TBuf& tb, lon
     return acc;
 }
 
-// outer residual: rhs32 = D^-1 (b - A x) in FP32; partials sum (D^-1 r)^2 and NaN count
+// outer residual: rhs32 = D^-1 (b - A x) in FP32 (red-black layout); partials sum (D^-1 r)^2
+// and NaN count
 __global__ void __launch_bounds__(kBlock) k_t_resid(Grid g, TBuf tb, double* x0, double* x1,
                                                     float* r0, float* r1, int mask,
                                                     double* __restrict__ partials) {
@@ -394,17 +439,20 @@ __global__ void __launch_bounds__(kBlock) k_t_resid(Grid g, TBuf tb, double* x0,
         int i, j, k;
         decode(g, r, i, j, k);
         const double inv = tb.inv[r];
+        int colour;
+        const int h = rb_index(tb.rb, i, j, k, colour);
+        const long long at = colour * tb.rb.H + h;
         // the inner right-hand side in FP32 rounded toward zero on the integer pipe (its
         // rounding is the inner solve's business; the FP64 pipe bounds this pass)
         if (mask & 1) {
             double rv = (tb.b[0][r] - t_row_apply(g, tb, r, i, j, k, x0)) * inv;
-            r0[r] = d2f_rz(rv);
+            r0[at] = d2f_rz(rv);
             acc[0] = __fma_rn(rv, rv, acc[0]);
             if (disnan(rv)) acc[2] += 1.0;
         }
         if (mask & 2) {
             double rv = (tb.b[1][r] - t_row_apply(g, tb, r, i, j, k, x1)) * inv;
-            r1[r] = d2f_rz(rv);
+            r1[at] = d2f_rz(rv);
             acc[1] = __fma_rn(rv, rv, acc[1]);
             if (disnan(rv)) acc[3] += 1.0;
         }
@@ -413,22 +461,35 @@ __global__ void __launch_bounds__(kBlock) k_t_resid(Grid g, TBuf tb, double* x0,
 }
 
 // ---------------------------------------------------------------------------
-// Inner FP32 BiCGStab on A^ = I + O (O: FP32 off-diagonals scaled by the row diagonal), for
-// NQ right-hand sides at once. With NQ = 2 both share the off-diagonal loads: each vector
-// element is a float2 with one lane per right-hand side. Every vector has `pad` zero
-// elements before and after its N rows, so the stencil needs no bounds tests (a link that
-// leaves the domain has a zero coefficient, and 0 * 0 adds nothing).
+// Inner FP32 BiCGStab. With the unit diagonal the system is, per colour (b black, r red; O: FP32
+// off-diagonals scaled by the row diagonal),
+//     x_b + O_b x_r = f_b,     x_r + O_r x_b = f_r,
+// and eliminating the red half (Hageman and Young's reduced system) leaves
+//     S x_b = f_b - O_b f_r,   S = I - O_b O_r,     x_r = f_r - O_r x_b.
+// S is applied by two half sweeps, z = O_r p then v = p - O_b z, which read every link once,
+// as one application of the whole matrix does, while the Krylov vectors are half as long, and
+// it takes about half the iterations (33 -> 16 to a residual of 1e-13 at 32x28x30): the
+// eigenvalues of I + O at 1 -+ mu fold onto 1 - mu^2. The residual of the whole system is the
+// reduced one (its red half is zero by construction), so the stopping test is unchanged: ||r||
+// against ||f||. An iteration moves 94 bytes per voxel for one right-hand side (whole matrix:
+// 112). Against BiCGStab on the whole matrix a two-species solve of 97x128x121 to 1e-12 takes
+// 2.2 ms (4.7), a step at 338x338x283 21.0 ms (29.1) and with acid flowing in 124 ms (151).
+//
+// NQ right-hand sides go together; with NQ = 2 they share the link loads and each vector
+// element is a float2 with one lane per right-hand side. Every vector has `pad` zero elements
+// before and after its H elements, so the stencil needs no bounds tests (a link that leaves
+// the domain has a zero coefficient, and 0 * 0 adds nothing). Each thread takes 16-byte chunks.
 //
 // Iteration n, with the per-lane scalars a (alpha), w (omega), b (beta) on the device:
 //   XP (n > 0): r = s - w t;  d += a p + w s;  p = r + b (p - w v)
-//   V         : v = A^ p (n = 0: p = r);              dots (rh, v)
-//   ST        : s = r - a v;  t = A^ s;               dots (t,s) (t,t) (rh,s) (rh,t) (s,s)
-// ST recomputes s at the six neighbours from r and v instead of reading a stored s. The
+//   Z, V      : z = O_r p, v = p - O_b z (n = 0: p = r);        dots (rh, v)
+//   ZS, T     : s = r - a v, z = O_r s, t = s - O_b z;          dots (t,s) (t,t) (rh,s) (rh,t) (s,s)
+// ZS recomputes s at the six neighbours from r and v, so s is stored once, by T. The
 // next rho = (rh, r) = (rh,s) - w (rh,t) and ||r||^2 = (s,s) - 2w (t,s) + w^2 (t,t) come from
-// the ST dots, so one iteration takes two reductions. Each reduction's last block updates
+// the T dots, so one iteration takes two reductions. Each reduction's one-block finalize updates
 // the scalars on the device; kernels return at once when no lane is active, so the host
 // launches iterations in batches and reads the state once per batch. The update a p + w s
-// still pending after the last iteration goes into the FP64 solution with d.
+// still pending after the last iteration goes into d before the red half is formed.
 
 enum {
     TI_BASE = 64,    // lane l: TI_BASE + TI_STRIDE * l + TI_*
@@ -443,354 +504,359 @@ enum {
     TI_ACT,          // 1 while the lane iterates
     TI_ITS,
     TI_REASON,       // 1 converged, -1 breakdown, -4 NaN/Inf
-    TI_ANY = 100,    // 1 while some lane iterates
-    TI_RED = 104     // reduced dots of the last reduction (up to 10)
+    TI_ANY = 100     // 1 while some lane iterates
 };
 __host__ __device__ __forceinline__ int tslot(int l, int v) { return TI_BASE + TI_STRIDE * l + v; }
-static_assert(TI_RED + 10 <= S_COUNT, "transport scalars exceed the scalar block");
+static_assert(TI_ANY < S_COUNT, "transport scalars exceed the scalar block");
 
 enum { PH_INIT = 0, PH_V = 1, PH_ST = 2 };
 
-template <int NQ>
-struct Lanes;
-template <>
-struct Lanes<1> {
-    using V = float;
-    static __device__ __forceinline__ V zero() { return 0.f; }
-    static __device__ __forceinline__ V fma_s(float a, V x, V y) { return __fmaf_rn(a, x, y); }
-    static __device__ __forceinline__ V fma_l(V a, V x, V y) { return __fmaf_rn(a, x, y); }
-    static __device__ __forceinline__ float lane(V v, int) { return v; }
-    static __device__ __forceinline__ V scal(const double* s, int v, float sign) {
-        return sign * (float)s[tslot(0, v)];
-    }
-    static __device__ __forceinline__ V gather(const float* const* f, int r) { return f[0][r]; }
-};
-template <>
-struct Lanes<2> {
-    using V = float2;
-    static __device__ __forceinline__ V zero() { return make_float2(0.f, 0.f); }
-    static __device__ __forceinline__ V fma_s(float a, V x, V y) {
-        return make_float2(__fmaf_rn(a, x.x, y.x), __fmaf_rn(a, x.y, y.y));
-    }
-    static __device__ __forceinline__ V fma_l(V a, V x, V y) {
-        return make_float2(__fmaf_rn(a.x, x.x, y.x), __fmaf_rn(a.y, x.y, y.y));
-    }
-    static __device__ __forceinline__ float lane(V v, int q) { return q ? v.y : v.x; }
-    static __device__ __forceinline__ V scal(const double* s, int v, float sign) {
-        return make_float2(sign * (float)s[tslot(0, v)], sign * (float)s[tslot(1, v)]);
-    }
-    static __device__ __forceinline__ V gather(const float* const* f, int r) {
-        return make_float2(f[0][r], f[1][r]);
-    }
-};
-
-// inner vectors: element pointers of row 0 in the active layout (float or float2)
+// inner vectors: pointers to element 0 in the active layout (float or float2 elements)
 struct TIVec {
-    float *r, *rh, *p, *v, *s, *t, *d;
-    const float* rhs[2];  // FP32 D^-1 (b - A x) per lane, unpadded
+    float *r, *rh, *p, *v, *s, *t, *d, *z;
+    const float* rhs[2];  // FP32 D^-1 (b - A x) per lane: black then red, H each, zero-padded
+    const float* o[6];    // links, black then red
 };
 
-struct TOff {
-    const float* o[6];  // +i,-i,+j,-j,+k,-k
-};
-
-// y = x + sum_d o_d x_nb, neighbours in the order -i, -j, -k, +k, +j, +i
+// A thread's 16-byte chunk: 4 / NQ elements of NQ lanes (value m: element m / NQ, lane m % NQ).
 template <int NQ>
-__device__ __forceinline__ typename Lanes<NQ>::V ti_apply(const TOff& op, int r, int JK, int K,
-                                                          const typename Lanes<NQ>::V* __restrict__ x) {
-    using L = Lanes<NQ>;
-    typename L::V acc = x[r];
-    acc = L::fma_s(__ldg(op.o[1] + r), x[r - JK], acc);
-    acc = L::fma_s(__ldg(op.o[3] + r), x[r - K], acc);
-    acc = L::fma_s(__ldg(op.o[5] + r), x[r - 1], acc);
-    acc = L::fma_s(__ldg(op.o[4] + r), x[r + 1], acc);
-    acc = L::fma_s(__ldg(op.o[2] + r), x[r + K], acc);
-    acc = L::fma_s(__ldg(op.o[0] + r), x[r + JK], acc);
+struct Chunk {
+    static constexpr int W = 4 / NQ;
+    float v[4];
+};
+
+template <int NQ>
+__device__ __forceinline__ Chunk<NQ> ld_chunk(const float* __restrict__ x, int h) {
+    const float4 q = *reinterpret_cast<const float4*>(x + (long long)NQ * h);
+    return {{q.x, q.y, q.z, q.w}};
+}
+template <int NQ>
+__device__ __forceinline__ void st_chunk(float* __restrict__ x, int h, const Chunk<NQ>& c) {
+    *reinterpret_cast<float4*>(x + (long long)NQ * h) = make_float4(c.v[0], c.v[1], c.v[2], c.v[3]);
+}
+// links of the W elements at h
+template <int NQ>
+__device__ __forceinline__ void ld_link(const float* __restrict__ o, int h, float (&l)[4 / NQ]) {
+    if (NQ == 1) {
+        const float4 q = __ldg(reinterpret_cast<const float4*>(o + h));
+        l[0] = q.x;
+        l[1 % (4 / NQ)] = q.y;
+        l[2 % (4 / NQ)] = q.z;
+        l[3 % (4 / NQ)] = q.w;
+    } else {
+        const float2 q = __ldg(reinterpret_cast<const float2*>(o + h));
+        l[0] = q.x;
+        l[1 % (4 / NQ)] = q.y;
+    }
+}
+
+// sources of the neighbour values: a vector, s = r - a v of two vectors, or the right-hand sides
+template <int NQ>
+struct SrcVec {
+    const float* x;
+    __device__ __forceinline__ Chunk<NQ> chunk(int h) const { return ld_chunk<NQ>(x, h); }
+    __device__ __forceinline__ void one(int h, float (&e)[NQ]) const {
+#pragma unroll
+        for (int l = 0; l < NQ; ++l) e[l] = x[(long long)NQ * h + l];
+    }
+};
+template <int NQ>
+struct SrcS {
+    const float *r, *v;
+    float na[NQ];  // -alpha per lane
+    __device__ __forceinline__ Chunk<NQ> chunk(int h) const {
+        Chunk<NQ> a = ld_chunk<NQ>(r, h);
+        const Chunk<NQ> b = ld_chunk<NQ>(v, h);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) a.v[m] = __fmaf_rn(na[m % NQ], b.v[m], a.v[m]);
+        return a;
+    }
+    __device__ __forceinline__ void one(int h, float (&e)[NQ]) const {
+#pragma unroll
+        for (int l = 0; l < NQ; ++l)
+            e[l] = __fmaf_rn(na[l], v[(long long)NQ * h + l], r[(long long)NQ * h + l]);
+    }
+};
+template <int NQ>
+struct SrcRhs {
+    const float *f0, *f1;
+    __device__ __forceinline__ Chunk<NQ> chunk(int h) const {
+        if (NQ == 1) return ld_chunk<NQ>(f0, h);
+        const float2 a = *reinterpret_cast<const float2*>(f0 + h), b = *reinterpret_cast<const float2*>(f1 + h);
+        return {{a.x, b.x, a.y, b.y}};
+    }
+    __device__ __forceinline__ void one(int h, float (&e)[NQ]) const {
+        e[0] = f0[h];
+        if (NQ > 1) e[NQ - 1] = f1[h];
+    }
+};
+
+// sum over the six links of the elements of colour COLOUR in chunk ch, times the other colour's
+// values; near = the other colour's chunk at the same place
+template <int NQ, int COLOUR, typename SRC>
+__device__ __forceinline__ Chunk<NQ> rb_links(const RBGrid& g, const TIVec& iv, int ch, const SRC& src,
+                                              Chunk<NQ>& near) {
+    constexpr int W = 4 / NQ;
+    const int h = ch * W;
+    const int row = (int)fdiv(NQ == 1 ? g.div4 : g.div2, (unsigned int)ch);
+    const int i = (int)fdiv(g.div_j, (unsigned int)row);
+    const bool odd = ((row - i * g.J + i) & 1) != COLOUR;  // odd k: the far neighbour is at h + 1
+    const long long base = COLOUR * g.H;
+    float l[6][W];
+#pragma unroll
+    for (int d = 0; d < 6; ++d) ld_link<NQ>(iv.o[d] + base, h, l[d]);
+    const Chunk<NQ> im = src.chunk(h - g.JK2), jm = src.chunk(h - g.K2p);
+    near = src.chunk(h);
+    const Chunk<NQ> jp = src.chunk(h + g.K2p), ip = src.chunk(h + g.JK2);
+    float e[NQ];
+    src.one(odd ? h + W : h - 1, e);
+    Chunk<NQ> far;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        const float up = m + NQ < 4 ? near.v[(m + NQ) % 4] : e[m % NQ];
+        const float dn = m >= NQ ? near.v[(m + 4 - NQ) % 4] : e[m % NQ];
+        far.v[m] = odd ? up : dn;
+    }
+    Chunk<NQ> acc;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        float a = l[0][m / NQ] * im.v[m];
+        a = __fmaf_rn(l[1][m / NQ], jm.v[m], a);
+        a = __fmaf_rn(l[2][m / NQ], near.v[m], a);
+        a = __fmaf_rn(l[3][m / NQ], far.v[m], a);
+        a = __fmaf_rn(l[4][m / NQ], jp.v[m], a);
+        a = __fmaf_rn(l[5][m / NQ], ip.v[m], a);
+        acc.v[m] = a;
+    }
     return acc;
 }
 
-// r = rh = rhs, d = 0, zero halos of r, p, v; dots (r, r)
-template <int NQ>
-__global__ void __launch_bounds__(kBlock) k_ti_init(int N, int pad, TIVec iv, double* __restrict__ partials) {
-    using L = Lanes<NQ>;
-    using V = typename L::V;
-    V* __restrict__ R = reinterpret_cast<V*>(iv.r);
-    V* __restrict__ RH = reinterpret_cast<V*>(iv.rh);
-    V* __restrict__ D = reinterpret_cast<V*>(iv.d);
-    V* __restrict__ P = reinterpret_cast<V*>(iv.p);
-    V* __restrict__ VV = reinterpret_cast<V*>(iv.v);
-    float acc[NQ];
+// block sums of the per-thread FP32 partials, value v of block b at partials[v gridDim + b]
+template <int NV>
+__device__ __forceinline__ void ti_block_sum(const float (&acc)[NV], double* __restrict__ partials) {
+    __shared__ double sh[NV][kBlock / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) acc[q] = 0.f;
-    const int stride = gridDim.x * blockDim.x;
-    const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
-    for (int r = t0; r < N; r += stride) {
-        V x = L::gather(iv.rhs, r);
-        R[r] = x;
-        RH[r] = x;
-        D[r] = L::zero();
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) acc[q] = __fmaf_rn(L::lane(x, q), L::lane(x, q), acc[q]);
+    for (int q = 0; q < NV; ++q) {
+        double x = (double)acc[q];
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        if (lane == 0) sh[q][warp] = x;
     }
-    for (int h = t0; h < pad; h += stride) {
-        R[-1 - h] = L::zero(); R[N + h] = L::zero();
-        P[-1 - h] = L::zero(); P[N + h] = L::zero();
-        VV[-1 - h] = L::zero(); VV[N + h] = L::zero();
+    __syncthreads();
+    if (threadIdx.x < NV) {
+        double s = 0.0;
+        for (int w = 0; w < kBlock / 32; ++w) s += sh[threadIdx.x][w];
+        partials[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = s;
     }
-    double a[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) a[q] = acc[q];
-    block_sum_store<NQ>(a, partials);
 }
 
-// v = A^ p (FIRST: p = r, stored); dots (rh, v)
+template <int NQ>
+__device__ __forceinline__ void ti_scal(const double* __restrict__ scal, int v, float (&out)[NQ]) {
+#pragma unroll
+    for (int l = 0; l < NQ; ++l) out[l] = (float)scal[tslot(l, v)];
+}
+
+// r = rh = f_b - O_b f_r, d = 0, zero halos of the vectors; dots (r, r) and (f, f) per lane
+template <int NQ>
+__global__ void __launch_bounds__(kBlock) k_rb_init(RBGrid g, int pad, TIVec iv, double* __restrict__ partials) {
+    float acc[2 * NQ];
+#pragma unroll
+    for (int q = 0; q < 2 * NQ; ++q) acc[q] = 0.f;
+    const int n = (int)(g.H / (4 / NQ)), stride = gridDim.x * blockDim.x;
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
+    const SrcRhs<NQ> black{iv.rhs[0], iv.rhs[1]}, red{iv.rhs[0] + g.H, iv.rhs[1] + g.H};
+    for (int ch = t0; ch < n; ch += stride) {
+        const int h = ch * (4 / NQ);
+        const Chunk<NQ> fb = black.chunk(h);
+        Chunk<NQ> fr;
+        const Chunk<NQ> y = rb_links<NQ, 0>(g, iv, ch, red, fr);
+        Chunk<NQ> r;
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            r.v[m] = fb.v[m] - y.v[m];
+            acc[m % NQ] = __fmaf_rn(r.v[m], r.v[m], acc[m % NQ]);
+            float f2 = __fmaf_rn(fb.v[m], fb.v[m], acc[NQ + m % NQ]);
+            acc[NQ + m % NQ] = __fmaf_rn(fr.v[m], fr.v[m], f2);
+        }
+        st_chunk<NQ>(iv.r, h, r);
+        st_chunk<NQ>(iv.rh, h, r);
+        st_chunk<NQ>(iv.d, h, Chunk<NQ>{{0.f, 0.f, 0.f, 0.f}});
+    }
+    float* const vecs[5] = {iv.r, iv.p, iv.v, iv.d, iv.z};
+    const long long end = (long long)NQ * g.H;
+    for (int q = t0; q < NQ * pad; q += stride)
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+            vecs[v][-1 - q] = 0.f;
+            vecs[v][end + q] = 0.f;
+        }
+    ti_block_sum<2 * NQ>(acc, partials);
+}
+
+// z = O_r x (x: p, or r on the first iteration)
+template <int NQ>
+__global__ void __launch_bounds__(kBlock) k_rb_z(RBGrid g, TIVec iv, const float* __restrict__ x,
+                                                 const double* __restrict__ scal) {
+    pdl_enter();
+    if (scal[TI_ANY] == 0.0) return;
+    const int n = (int)(g.H / (4 / NQ));
+    const SrcVec<NQ> src{x};
+    for (int ch = blockIdx.x * blockDim.x + threadIdx.x; ch < n; ch += gridDim.x * blockDim.x) {
+        Chunk<NQ> near;
+        st_chunk<NQ>(iv.z, ch * (4 / NQ), rb_links<NQ, 1>(g, iv, ch, src, near));
+    }
+}
+
+// v = p - O_b z (FIRST: p = r, stored); dots (rh, v)
 template <int NQ, bool FIRST>
-__global__ void __launch_bounds__(kBlock) k_ti_v(int N, int JK, int K, TOff op, TIVec iv,
-                                                 const double* __restrict__ scal,
+__global__ void __launch_bounds__(kBlock) k_rb_v(RBGrid g, TIVec iv, const double* __restrict__ scal,
                                                  double* __restrict__ partials) {
     pdl_enter();
     if (scal[TI_ANY] == 0.0) return;
-    using L = Lanes<NQ>;
-    using V = typename L::V;
-    const V* __restrict__ X = reinterpret_cast<const V*>(FIRST ? iv.r : iv.p);
-    const V* __restrict__ RH = reinterpret_cast<const V*>(iv.rh);
-    V* __restrict__ VV = reinterpret_cast<V*>(iv.v);
-    V* __restrict__ P = reinterpret_cast<V*>(iv.p);
     float acc[NQ];
 #pragma unroll
     for (int q = 0; q < NQ; ++q) acc[q] = 0.f;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < N; r += gridDim.x * blockDim.x) {
-        const V y = ti_apply<NQ>(op, r, JK, K, X);
-        VV[r] = y;
-        if (FIRST) P[r] = X[r];
-        const V h = RH[r];
+    const int n = (int)(g.H / (4 / NQ));
+    const SrcVec<NQ> src{iv.z};
+    for (int ch = blockIdx.x * blockDim.x + threadIdx.x; ch < n; ch += gridDim.x * blockDim.x) {
+        const int h = ch * (4 / NQ);
+        const Chunk<NQ> p = ld_chunk<NQ>(FIRST ? iv.r : iv.p, h), rh = ld_chunk<NQ>(iv.rh, h);
+        Chunk<NQ> near;
+        Chunk<NQ> y = rb_links<NQ, 0>(g, iv, ch, src, near);
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) acc[q] = __fmaf_rn(L::lane(h, q), L::lane(y, q), acc[q]);
+        for (int m = 0; m < 4; ++m) {
+            y.v[m] = p.v[m] - y.v[m];
+            acc[m % NQ] = __fmaf_rn(rh.v[m], y.v[m], acc[m % NQ]);
+        }
+        st_chunk<NQ>(iv.v, h, y);
+        if (FIRST) st_chunk<NQ>(iv.p, h, p);
     }
-    double a[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) a[q] = acc[q];
-    block_sum_store<NQ>(a, partials);
+    ti_block_sum<NQ>(acc, partials);
 }
 
-// s = r - a v (at the row and, recomputed, at its neighbours); t = A^ s;
-// dots (t,s) (t,t) (rh,s) (rh,t) (s,s) per lane
+// z = O_r s, s = r - a v formed at the neighbours
 template <int NQ>
-__global__ void __launch_bounds__(kBlock) k_ti_st(int N, int JK, int K, TOff op, TIVec iv,
-                                                  const double* __restrict__ scal,
-                                                  double* __restrict__ partials) {
+__global__ void __launch_bounds__(kBlock) k_rb_zs(RBGrid g, TIVec iv, const double* __restrict__ scal) {
     pdl_enter();
     if (scal[TI_ANY] == 0.0) return;
-    using L = Lanes<NQ>;
-    using V = typename L::V;
-    const V* __restrict__ R = reinterpret_cast<const V*>(iv.r);
-    const V* __restrict__ VV = reinterpret_cast<const V*>(iv.v);
-    const V* __restrict__ RH = reinterpret_cast<const V*>(iv.rh);
-    V* __restrict__ S = reinterpret_cast<V*>(iv.s);
-    V* __restrict__ T = reinterpret_cast<V*>(iv.t);
-    const V na = L::scal(scal, TI_ALPHA, -1.f);
+    const int n = (int)(g.H / (4 / NQ));
+    SrcS<NQ> src{iv.r, iv.v, {}};
+    ti_scal<NQ>(scal, TI_ALPHA, src.na);
+#pragma unroll
+    for (int l = 0; l < NQ; ++l) src.na[l] = -src.na[l];
+    for (int ch = blockIdx.x * blockDim.x + threadIdx.x; ch < n; ch += gridDim.x * blockDim.x) {
+        Chunk<NQ> near;
+        st_chunk<NQ>(iv.z, ch * (4 / NQ), rb_links<NQ, 1>(g, iv, ch, src, near));
+    }
+}
+
+// s = r - a v, t = s - O_b z; dots (t,s) (t,t) (rh,s) (rh,t) (s,s) per lane
+template <int NQ>
+__global__ void __launch_bounds__(kBlock) k_rb_t(RBGrid g, TIVec iv, const double* __restrict__ scal,
+                                                 double* __restrict__ partials) {
+    pdl_enter();
+    if (scal[TI_ANY] == 0.0) return;
+    float na[NQ];
+    ti_scal<NQ>(scal, TI_ALPHA, na);
     float acc[5 * NQ];
 #pragma unroll
     for (int q = 0; q < 5 * NQ; ++q) acc[q] = 0.f;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < N; r += gridDim.x * blockDim.x) {
-        const V s = L::fma_l(na, VV[r], R[r]);
-        V t = s;
-        t = L::fma_s(__ldg(op.o[1] + r), L::fma_l(na, VV[r - JK], R[r - JK]), t);
-        t = L::fma_s(__ldg(op.o[3] + r), L::fma_l(na, VV[r - K], R[r - K]), t);
-        t = L::fma_s(__ldg(op.o[5] + r), L::fma_l(na, VV[r - 1], R[r - 1]), t);
-        t = L::fma_s(__ldg(op.o[4] + r), L::fma_l(na, VV[r + 1], R[r + 1]), t);
-        t = L::fma_s(__ldg(op.o[2] + r), L::fma_l(na, VV[r + K], R[r + K]), t);
-        t = L::fma_s(__ldg(op.o[0] + r), L::fma_l(na, VV[r + JK], R[r + JK]), t);
-        S[r] = s;
-        T[r] = t;
-        const V h = RH[r];
+    const int n = (int)(g.H / (4 / NQ));
+    const SrcVec<NQ> src{iv.z};
+    for (int ch = blockIdx.x * blockDim.x + threadIdx.x; ch < n; ch += gridDim.x * blockDim.x) {
+        const int h = ch * (4 / NQ);
+        const Chunk<NQ> r = ld_chunk<NQ>(iv.r, h), v = ld_chunk<NQ>(iv.v, h), rh = ld_chunk<NQ>(iv.rh, h);
+        Chunk<NQ> near;
+        Chunk<NQ> t = rb_links<NQ, 0>(g, iv, ch, src, near);
+        Chunk<NQ> s;
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const float sq = L::lane(s, q), tq = L::lane(t, q), hq = L::lane(h, q);
-            acc[5 * q + 0] = __fmaf_rn(tq, sq, acc[5 * q + 0]);
-            acc[5 * q + 1] = __fmaf_rn(tq, tq, acc[5 * q + 1]);
-            acc[5 * q + 2] = __fmaf_rn(hq, sq, acc[5 * q + 2]);
-            acc[5 * q + 3] = __fmaf_rn(hq, tq, acc[5 * q + 3]);
-            acc[5 * q + 4] = __fmaf_rn(sq, sq, acc[5 * q + 4]);
+        for (int m = 0; m < 4; ++m) {
+            const int q = 5 * (m % NQ);
+            s.v[m] = __fmaf_rn(-na[m % NQ], v.v[m], r.v[m]);
+            t.v[m] = s.v[m] - t.v[m];
+            acc[q + 0] = __fmaf_rn(t.v[m], s.v[m], acc[q + 0]);
+            acc[q + 1] = __fmaf_rn(t.v[m], t.v[m], acc[q + 1]);
+            acc[q + 2] = __fmaf_rn(rh.v[m], s.v[m], acc[q + 2]);
+            acc[q + 3] = __fmaf_rn(rh.v[m], t.v[m], acc[q + 3]);
+            acc[q + 4] = __fmaf_rn(s.v[m], s.v[m], acc[q + 4]);
         }
+        st_chunk<NQ>(iv.s, h, s);
+        st_chunk<NQ>(iv.t, h, t);
     }
-    double a[5 * NQ];
-#pragma unroll
-    for (int q = 0; q < 5 * NQ; ++q) a[q] = acc[q];
-    block_sum_store<5 * NQ>(a, partials);
+    ti_block_sum<5 * NQ>(acc, partials);
 }
 
 // r = s - w t; d += a p + w s; p = r + b (p - w v)
 template <int NQ>
-__global__ void __launch_bounds__(kBlock) k_ti_xp(int N, TIVec iv, const double* __restrict__ scal) {
+__global__ void __launch_bounds__(kBlock) k_rb_xp(RBGrid g, TIVec iv, const double* __restrict__ scal) {
     pdl_enter();
     if (scal[TI_ANY] == 0.0) return;
-    using L = Lanes<NQ>;
-    using V = typename L::V;
-    const V* __restrict__ S = reinterpret_cast<const V*>(iv.s);
-    const V* __restrict__ T = reinterpret_cast<const V*>(iv.t);
-    const V* __restrict__ VV = reinterpret_cast<const V*>(iv.v);
-    V* __restrict__ R = reinterpret_cast<V*>(iv.r);
-    V* __restrict__ P = reinterpret_cast<V*>(iv.p);
-    V* __restrict__ D = reinterpret_cast<V*>(iv.d);
-    const V a = L::scal(scal, TI_ALPHA, 1.f);
-    const V w = L::scal(scal, TI_OMEGA, 1.f);
-    const V nw = L::scal(scal, TI_OMEGA, -1.f);
-    const V b = L::scal(scal, TI_BETA, 1.f);
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < N; r += gridDim.x * blockDim.x) {
-        const V s = S[r], t = T[r], p = P[r], v = VV[r];
-        const V rn = L::fma_l(nw, t, s);
-        D[r] = L::fma_l(a, p, L::fma_l(w, s, D[r]));
-        R[r] = rn;
-        P[r] = L::fma_l(b, L::fma_l(nw, v, p), rn);
+    float a[NQ], w[NQ], b[NQ];
+    ti_scal<NQ>(scal, TI_ALPHA, a);
+    ti_scal<NQ>(scal, TI_OMEGA, w);
+    ti_scal<NQ>(scal, TI_BETA, b);
+    const int n = (int)(g.H / (4 / NQ));
+    for (int ch = blockIdx.x * blockDim.x + threadIdx.x; ch < n; ch += gridDim.x * blockDim.x) {
+        const int h = ch * (4 / NQ);
+        const Chunk<NQ> s = ld_chunk<NQ>(iv.s, h), t = ld_chunk<NQ>(iv.t, h), v = ld_chunk<NQ>(iv.v, h);
+        Chunk<NQ> p = ld_chunk<NQ>(iv.p, h), d = ld_chunk<NQ>(iv.d, h), r;
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const int l = m % NQ;
+            r.v[m] = __fmaf_rn(-w[l], t.v[m], s.v[m]);
+            d.v[m] = __fmaf_rn(a[l], p.v[m], __fmaf_rn(w[l], s.v[m], d.v[m]));
+            p.v[m] = __fmaf_rn(b[l], __fmaf_rn(-w[l], v.v[m], p.v[m]), r.v[m]);
+        }
+        st_chunk<NQ>(iv.d, h, d);
+        st_chunk<NQ>(iv.r, h, r);
+        st_chunk<NQ>(iv.p, h, p);
     }
 }
 
-// Single right-hand side with an even row length K: each thread takes a pair of rows
-// (r, r+1), r even, with 8-byte loads (the +-j and +-i neighbours of an even row are even as
-// K and J*K are even; the -k neighbour of r and the +k neighbour of r+1 are single loads).
-// Same arithmetic per row as k_ti_v / k_ti_st / k_ti_xp, half the load instructions.
-
-__device__ __forceinline__ float2 ti_apply_pair(const TOff& op, int t, int JK2, int K2,
-                                                const float* __restrict__ x) {
-    const float2* __restrict__ x2 = reinterpret_cast<const float2*>(x);
-    const int r = 2 * t;
-    const float2 xc = x2[t], xim = x2[t - JK2], xjm = x2[t - K2], xjp = x2[t + K2], xip = x2[t + JK2];
-    const float xkm = x[r - 1], xkp = x[r + 2];
-    const float2 o0 = __ldg(reinterpret_cast<const float2*>(op.o[0]) + t);
-    const float2 o1 = __ldg(reinterpret_cast<const float2*>(op.o[1]) + t);
-    const float2 o2 = __ldg(reinterpret_cast<const float2*>(op.o[2]) + t);
-    const float2 o3 = __ldg(reinterpret_cast<const float2*>(op.o[3]) + t);
-    const float2 o4 = __ldg(reinterpret_cast<const float2*>(op.o[4]) + t);
-    const float2 o5 = __ldg(reinterpret_cast<const float2*>(op.o[5]) + t);
-    float y0 = xc.x, y1 = xc.y;
-    y0 = __fmaf_rn(o1.x, xim.x, y0); y1 = __fmaf_rn(o1.y, xim.y, y1);
-    y0 = __fmaf_rn(o3.x, xjm.x, y0); y1 = __fmaf_rn(o3.y, xjm.y, y1);
-    y0 = __fmaf_rn(o5.x, xkm, y0);   y1 = __fmaf_rn(o5.y, xc.x, y1);
-    y0 = __fmaf_rn(o4.x, xc.y, y0);  y1 = __fmaf_rn(o4.y, xkp, y1);
-    y0 = __fmaf_rn(o2.x, xjp.x, y0); y1 = __fmaf_rn(o2.y, xjp.y, y1);
-    y0 = __fmaf_rn(o0.x, xip.x, y0); y1 = __fmaf_rn(o0.y, xip.y, y1);
-    return make_float2(y0, y1);
-}
-
-template <bool FIRST>
-__global__ void __launch_bounds__(kBlock) k_ti_v_pair(int N2, int JK2, int K2, TOff op, TIVec iv,
-                                                      const double* __restrict__ scal,
-                                                      double* __restrict__ partials) {
-    pdl_enter();
-    if (scal[TI_ANY] == 0.0) return;
-    const float* __restrict__ X = FIRST ? iv.r : iv.p;
-    const float2* __restrict__ RH = reinterpret_cast<const float2*>(iv.rh);
-    float2* __restrict__ VV = reinterpret_cast<float2*>(iv.v);
-    float2* __restrict__ P = reinterpret_cast<float2*>(iv.p);
-    float acc = 0.f;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < N2; t += gridDim.x * blockDim.x) {
-        const float2 y = ti_apply_pair(op, t, JK2, K2, X);
-        VV[t] = y;
-        if (FIRST) P[t] = reinterpret_cast<const float2*>(X)[t];
-        const float2 h = RH[t];
-        acc = __fmaf_rn(h.x, y.x, acc);
-        acc = __fmaf_rn(h.y, y.y, acc);
-    }
-    double a[1] = {acc};
-    block_sum_store<1>(a, partials);
-}
-
-__global__ void __launch_bounds__(kBlock) k_ti_st_pair(int N2, int JK2, int K2, TOff op, TIVec iv,
-                                                       const double* __restrict__ scal,
-                                                       double* __restrict__ partials) {
-    pdl_enter();
-    if (scal[TI_ANY] == 0.0) return;
-    const float* __restrict__ R = iv.r;
-    const float* __restrict__ VV = iv.v;
-    const float2* __restrict__ R2 = reinterpret_cast<const float2*>(iv.r);
-    const float2* __restrict__ V2 = reinterpret_cast<const float2*>(iv.v);
-    const float2* __restrict__ RH = reinterpret_cast<const float2*>(iv.rh);
-    float2* __restrict__ S = reinterpret_cast<float2*>(iv.s);
-    float2* __restrict__ T = reinterpret_cast<float2*>(iv.t);
-    const float na = -(float)scal[tslot(0, TI_ALPHA)];
-    float acc[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < N2; t += gridDim.x * blockDim.x) {
-        const int r = 2 * t;
-        auto s2 = [&](int u) {
-            const float2 rv = R2[u], vv = V2[u];
-            return make_float2(__fmaf_rn(na, vv.x, rv.x), __fmaf_rn(na, vv.y, rv.y));
-        };
-        const float2 sc = s2(t), sim = s2(t - JK2), sjm = s2(t - K2), sjp = s2(t + K2), sip = s2(t + JK2);
-        const float skm = __fmaf_rn(na, VV[r - 1], R[r - 1]);
-        const float skp = __fmaf_rn(na, VV[r + 2], R[r + 2]);
-        const float2 o0 = __ldg(reinterpret_cast<const float2*>(op.o[0]) + t);
-        const float2 o1 = __ldg(reinterpret_cast<const float2*>(op.o[1]) + t);
-        const float2 o2 = __ldg(reinterpret_cast<const float2*>(op.o[2]) + t);
-        const float2 o3 = __ldg(reinterpret_cast<const float2*>(op.o[3]) + t);
-        const float2 o4 = __ldg(reinterpret_cast<const float2*>(op.o[4]) + t);
-        const float2 o5 = __ldg(reinterpret_cast<const float2*>(op.o[5]) + t);
-        float t0 = sc.x, t1 = sc.y;
-        t0 = __fmaf_rn(o1.x, sim.x, t0); t1 = __fmaf_rn(o1.y, sim.y, t1);
-        t0 = __fmaf_rn(o3.x, sjm.x, t0); t1 = __fmaf_rn(o3.y, sjm.y, t1);
-        t0 = __fmaf_rn(o5.x, skm, t0);   t1 = __fmaf_rn(o5.y, sc.x, t1);
-        t0 = __fmaf_rn(o4.x, sc.y, t0);  t1 = __fmaf_rn(o4.y, skp, t1);
-        t0 = __fmaf_rn(o2.x, sjp.x, t0); t1 = __fmaf_rn(o2.y, sjp.y, t1);
-        t0 = __fmaf_rn(o0.x, sip.x, t0); t1 = __fmaf_rn(o0.y, sip.y, t1);
-        S[t] = sc;
-        T[t] = make_float2(t0, t1);
-        const float2 h = RH[t];
-        acc[0] = __fmaf_rn(t0, sc.x, acc[0]); acc[0] = __fmaf_rn(t1, sc.y, acc[0]);
-        acc[1] = __fmaf_rn(t0, t0, acc[1]);   acc[1] = __fmaf_rn(t1, t1, acc[1]);
-        acc[2] = __fmaf_rn(h.x, sc.x, acc[2]); acc[2] = __fmaf_rn(h.y, sc.y, acc[2]);
-        acc[3] = __fmaf_rn(h.x, t0, acc[3]);  acc[3] = __fmaf_rn(h.y, t1, acc[3]);
-        acc[4] = __fmaf_rn(sc.x, sc.x, acc[4]); acc[4] = __fmaf_rn(sc.y, sc.y, acc[4]);
-    }
-    double a[5] = {acc[0], acc[1], acc[2], acc[3], acc[4]};
-    block_sum_store<5>(a, partials);
-}
-
-// k_ti_xp on pairs of rows (8-byte loads and stores)
-__global__ void __launch_bounds__(kBlock) k_ti_xp_pair(int N2, TIVec iv, const double* __restrict__ scal) {
-    pdl_enter();
-    if (scal[TI_ANY] == 0.0) return;
-    const float2* __restrict__ S = reinterpret_cast<const float2*>(iv.s);
-    const float2* __restrict__ T = reinterpret_cast<const float2*>(iv.t);
-    const float2* __restrict__ VV = reinterpret_cast<const float2*>(iv.v);
-    float2* __restrict__ R = reinterpret_cast<float2*>(iv.r);
-    float2* __restrict__ P = reinterpret_cast<float2*>(iv.p);
-    float2* __restrict__ D = reinterpret_cast<float2*>(iv.d);
-    const float a = (float)scal[tslot(0, TI_ALPHA)];
-    const float w = (float)scal[tslot(0, TI_OMEGA)];
-    const float b = (float)scal[tslot(0, TI_BETA)];
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < N2; t += gridDim.x * blockDim.x) {
-        const float2 s = S[t], tt = T[t], p = P[t], v = VV[t], d = D[t];
-        const float2 rn = make_float2(__fmaf_rn(-w, tt.x, s.x), __fmaf_rn(-w, tt.y, s.y));
-        D[t] = make_float2(__fmaf_rn(a, p.x, __fmaf_rn(w, s.x, d.x)), __fmaf_rn(a, p.y, __fmaf_rn(w, s.y, d.y)));
-        R[t] = rn;
-        P[t] = make_float2(__fmaf_rn(b, __fmaf_rn(-w, v.x, p.x), rn.x), __fmaf_rn(b, __fmaf_rn(-w, v.y, p.y), rn.y));
-    }
-}
-
-// x_lane += d + a p + w s (the pending update of the last iteration)
+// d += a p + w s: the pending update of the last iteration
 template <int NQ>
-__global__ void k_ti_accum(int N, TIVec iv, const double* __restrict__ scal, double* __restrict__ x0,
-                           double* __restrict__ x1) {
-    using L = Lanes<NQ>;
-    using V = typename L::V;
-    const V* __restrict__ S = reinterpret_cast<const V*>(iv.s);
-    const V* __restrict__ P = reinterpret_cast<const V*>(iv.p);
-    const V* __restrict__ D = reinterpret_cast<const V*>(iv.d);
+__global__ void __launch_bounds__(kBlock) k_rb_pending(RBGrid g, TIVec iv, const double* __restrict__ scal) {
+    pdl_enter();
     float a[NQ], w[NQ];
+    ti_scal<NQ>(scal, TI_ALPHA, a);
+    ti_scal<NQ>(scal, TI_OMEGA, w);
+    const int n = (int)(g.H / (4 / NQ));
+    for (int ch = blockIdx.x * blockDim.x + threadIdx.x; ch < n; ch += gridDim.x * blockDim.x) {
+        const int h = ch * (4 / NQ);
+        const Chunk<NQ> s = ld_chunk<NQ>(iv.s, h), p = ld_chunk<NQ>(iv.p, h);
+        Chunk<NQ> d = ld_chunk<NQ>(iv.d, h);
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-        a[q] = (float)scal[tslot(q, TI_ALPHA)];
-        w[q] = (float)scal[tslot(q, TI_OMEGA)];
+        for (int m = 0; m < 4; ++m) {
+            if (w[m % NQ] != 0.f) d.v[m] = __fmaf_rn(w[m % NQ], s.v[m], d.v[m]);
+            if (a[m % NQ] != 0.f) d.v[m] = __fmaf_rn(a[m % NQ], p.v[m], d.v[m]);
+        }
+        st_chunk<NQ>(iv.d, h, d);
     }
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < N; r += gridDim.x * blockDim.x) {
-        const V d = D[r];
+}
+
+// both halves of the correction into the FP64 solution: x_b += d, x_r += f_r - O_r d
+template <int NQ>
+__global__ void __launch_bounds__(kBlock) k_rb_accum(RBGrid g, TIVec iv, double* __restrict__ x0,
+                                                     double* __restrict__ x1) {
+    pdl_enter();
+    const int n = (int)(g.H / (4 / NQ));
+    const SrcVec<NQ> src{iv.d};
+    const SrcRhs<NQ> red{iv.rhs[0] + g.H, iv.rhs[1] + g.H};
+    for (int ch = blockIdx.x * blockDim.x + threadIdx.x; ch < n; ch += gridDim.x * blockDim.x) {
+        const int h = ch * (4 / NQ);
+        Chunk<NQ> d;
+        const Chunk<NQ> y = rb_links<NQ, 1>(g, iv, ch, src, d);
+        const Chunk<NQ> f = red.chunk(h);
+        const int row = h / g.K2p, k2 = h - row * g.K2p, i = row / g.J;
+        const int par = (row - i * g.J + i) & 1;  // black at k = 2 k2 + par, red at 2 k2 + 1 - par
+        const long long base = (long long)row * g.K;
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            float inc = L::lane(d, q);
-            if (w[q] != 0.f) inc = __fmaf_rn(w[q], L::lane(S[r], q), inc);
-            if (a[q] != 0.f) inc = __fmaf_rn(a[q], L::lane(P[r], q), inc);
-            double* x = q ? x1 : x0;
-            x[r] += (double)inc;
+        for (int m = 0; m < 4; ++m) {
+            double* x = (m % NQ) ? x1 : x0;
+            const int k0 = 2 * (k2 + m / NQ);
+            const float dr = f.v[m] - y.v[m];
+            if (k0 + par < g.K) x[base + k0 + par] += (double)d.v[m];
+            if (k0 + 1 - par < g.K) x[base + k0 + 1 - par] += (double)dr;
         }
     }
 }
@@ -805,16 +871,17 @@ __device__ void ti_phase(double* scal, const double* red, double tol2_0, double 
     for (int l = 0; l < NQ; ++l) {
         double* s = scal + tslot(l, 0);
         if (PH == PH_INIT) {
-            const double rr = red[l];
-            s[TI_RR0] = rr;
+            const double rr = red[l], ff = red[NQ + l];  // the reduced and the whole right-hand side
+            s[TI_RR0] = ff;
             s[TI_RHO] = rr;
             s[TI_R2] = rr;
             s[TI_TOL2] = l ? tol2_1 : tol2_0;
             s[TI_ALPHA] = s[TI_OMEGA] = s[TI_BETA] = 0.0;
             s[TI_ITS] = 0.0;
-            const bool ok = finite_d(rr) && rr > 0.0;
+            const bool fin = finite_d(rr) && finite_d(ff);
+            const bool ok = fin && rr > s[TI_TOL2] * ff;
             s[TI_ACT] = ok ? 1.0 : 0.0;
-            s[TI_REASON] = ok ? 0.0 : (finite_d(rr) ? 1.0 : -4.0);
+            s[TI_REASON] = ok ? 0.0 : (fin ? 1.0 : -4.0);
         } else if (PH == PH_V) {
             if (s[TI_ACT] != 0.0) {
                 const double rv = red[l];
@@ -863,40 +930,31 @@ __device__ void ti_phase(double* scal, const double* red, double tol2_0, double 
     scal[TI_ANY] = any ? 1.0 : 0.0;
 }
 
-// Fixed-order reduction of the per-block partials, one block per value (as k_finalize);
-// the last block to finish applies the scalar update of phase PH.
+__host__ __device__ constexpr int ti_values(int ph, int nq) { return ph == PH_ST ? 5 * nq : ph == PH_INIT ? 2 * nq : nq; }
+
+// Fixed-order reduction of the per-block partials by one block, a warp per value, and the scalar
+// update of phase PH by its first thread. One block needs no counter across blocks: 4 us where
+// a block per value and an atomic ticket took 9-11 us.
 template <int PH, int NQ>
-__global__ void __launch_bounds__(kFinalizeThreads) k_ti_fin(const double* __restrict__ partials, int nblocks,
-                                                             double* scal, unsigned int* counter,
-                                                             double tol2_0, double tol2_1) {
+__global__ void __launch_bounds__(32 * ti_values(PH, NQ)) k_ti_fin(const double* __restrict__ partials, int nblocks,
+                                                                   double* scal, double tol2_0, double tol2_1) {
     pdl_enter();
     if (PH != PH_INIT && scal[TI_ANY] == 0.0) return;
-    constexpr int NV = (PH == PH_ST) ? 5 * NQ : NQ;
-    __shared__ double sh[kFinalizeThreads];
-    __shared__ bool last;
-    const int v = blockIdx.x;
-    double acc = 0.0;
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) acc += partials[(size_t)b * NV + v];
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int w = kFinalizeThreads / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        scal[TI_RED + v] = sh[0];
-        __threadfence();
-        last = (atomicAdd(counter, 1u) == (unsigned int)(NV - 1));
-    }
-    __syncthreads();
-    if (last && threadIdx.x == 0) {
-        __threadfence();
-        double red[NV];
+    constexpr int NV = ti_values(PH, NQ);
+    __shared__ double red[NV];
+    const int v = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const double* __restrict__ mine = partials + (size_t)v * nblocks;
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int b = lane; b < nblocks; b += 128) {
 #pragma unroll
-        for (int q = 0; q < NV; ++q) red[q] = __ldcg(scal + TI_RED + q);
-        ti_phase<PH, NQ>(scal, red, tol2_0, tol2_1);
-        *counter = 0u;
+        for (int q = 0; q < 4; ++q)
+            if (b + 32 * q < nblocks) a[q] += mine[b + 32 * q];
     }
+    double x = (a[0] + a[1]) + (a[2] + a[3]);
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (lane == 0) red[v] = x;
+    __syncthreads();
+    if (threadIdx.x == 0) ti_phase<PH, NQ>(scal, red, tol2_0, tol2_1);
 }
 
 // min / max of x over the rows
@@ -943,29 +1001,36 @@ __global__ void k_zero_solid_flux(Grid g, const unsigned int* __restrict__ bits,
 
 static ls_status t_alloc(ls_ctx* c) {
     const size_t n = (size_t)c->g.N;
+    const RBGrid rb = make_rb(c->g);
     LS_TRY(lean_phase(c, kPhaseTransport));  // lean: the transport arrays take the pressure solve's memory
+    c->ti_half = rb.H;
+    // a plane and a chunk around each vector
+    c->ti_pad = ((rb.JK2 + 4 + 31) / 32) * 32;
     // largest first (lean: an arena sized for the other phase then wastes the least)
     if (!c->ti) {
-        // 7 inner vectors of up to N float2 each, with `pad` elements on both sides
-        c->ti_pad = ((c->g.JK + 31) / 32) * 32;
-        c->ti_stride = ((2 * (c->g.N + 2 * c->ti_pad) + 63) / 64) * 64;
-        LS_TRY(walloc_t(c, &c->ti, (size_t)c->ti_stride * 7));
-        LS_CUDA(c, cudaMemsetAsync(c->ti, 0, sizeof(float) * (size_t)c->ti_stride * 7, c->stream));
+        // inner vectors of up to H float2 each, with `pad` elements on both sides
+        c->ti_stride = ((2 * (rb.H + 2 * c->ti_pad) + 63) / 64) * 64;
+        LS_TRY(walloc_t(c, &c->ti, (size_t)c->ti_stride * kTiVecs));
+        LS_CUDA(c, cudaMemsetAsync(c->ti, 0, sizeof(float) * (size_t)c->ti_stride * kTiVecs, c->stream));
     }
     for (int q = 0; q < 7; ++q)
         if (!c->tc[q]) LS_TRY(walloc_t(c, &c->tc[q], n));
     for (int q = 0; q < 2; ++q)
         if (!c->tb[q]) LS_TRY(walloc_t(c, &c->tb[q], n));
     if (!c->tinv) LS_TRY(walloc_t(c, &c->tinv, n));
+    // the virtual elements of the links and right-hand sides hold zeros, and nothing writes them
     for (int q = 0; q < 6; ++q)
-        if (!c->to[q]) LS_TRY(walloc_t(c, &c->to[q], n));
+        if (!c->to[q]) {
+            LS_TRY(walloc_t(c, &c->to[q], 2 * (size_t)rb.H));
+            LS_CUDA(c, cudaMemsetAsync(c->to[q], 0, sizeof(float) * 2 * (size_t)rb.H, c->stream));
+        }
     for (int q = 0; q < 2; ++q)
-        if (!c->trhs[q]) LS_TRY(walloc_t(c, &c->trhs[q], n));
+        if (!c->trhs[q]) {
+            const size_t m = 2 * (size_t)rb.H + 2 * (size_t)c->ti_pad;
+            LS_TRY(walloc_t(c, &c->trhs[q], m));
+            LS_CUDA(c, cudaMemsetAsync(c->trhs[q], 0, sizeof(float) * m, c->stream));
+        }
     if (!c->tkind) LS_TRY(walloc_t(c, &c->tkind, n));
-    if (!c->tcount) {
-        LS_TRY(dalloc_t(c, &c->tcount, 1));
-        LS_CUDA(c, cudaMemsetAsync(c->tcount, 0, sizeof(unsigned int), c->stream));
-    }
     return LS_OK;
 }
 
@@ -976,6 +1041,7 @@ static TBuf make_tbuf(ls_ctx* c) {
     for (int q = 0; q < 6; ++q) tb.o[q] = c->to[q];
     tb.inv = c->tinv;
     tb.kind = c->tkind;
+    tb.rb = make_rb(c->g);
     return tb;
 }
 
@@ -986,68 +1052,49 @@ template <int NQ>
 static ls_status inner_solve(ls_ctx* c, const TBuf& tb, const int lane_q[NQ], const double tol[NQ],
                              int max_it, double* x[2], int its[NQ]) {
     const Grid g = c->g;
-    const int N = (int)g.N, JK = (int)g.JK, K = g.K;
-    const int grid = grid_for(c, g.N);
+    const RBGrid rb = tb.rb;
+    const int grid = grid_for(c, rb.H / (4 / NQ));
     TIVec iv;
-    float** vecs[7] = {&iv.r, &iv.rh, &iv.p, &iv.v, &iv.s, &iv.t, &iv.d};
-    for (int v = 0; v < 7; ++v) *vecs[v] = c->ti + (size_t)v * c->ti_stride + 2 * c->ti_pad;
-    iv.rhs[0] = c->trhs[lane_q[0]];
-    iv.rhs[1] = c->trhs[NQ > 1 ? lane_q[1] : lane_q[0]];
-    TOff op;
-    for (int d = 0; d < 6; ++d) op.o[d] = tb.o[d];
+    float** vecs[kTiVecs] = {&iv.r, &iv.rh, &iv.p, &iv.v, &iv.s, &iv.t, &iv.d, &iv.z};
+    for (int v = 0; v < kTiVecs; ++v) *vecs[v] = c->ti + (size_t)v * c->ti_stride + 2 * c->ti_pad;
+    iv.rhs[0] = c->trhs[lane_q[0]] + c->ti_pad;
+    iv.rhs[1] = c->trhs[NQ > 1 ? lane_q[1] : lane_q[0]] + c->ti_pad;
+    for (int d = 0; d < 6; ++d) iv.o[d] = tb.o[d];
     const double t0 = tol[0] * tol[0], t1 = NQ > 1 ? tol[1] * tol[1] : 0.0;
-    LS_LAUNCH(c, k_ti_init<NQ>, grid, kBlock, 0, N, (int)c->ti_pad, iv, c->partials);
-    LS_LAUNCH(c, (k_ti_fin<PH_INIT, NQ>), NQ, kFinalizeThreads, 0, (const double*)c->partials, grid, c->scal,
-              c->tcount, t0, t1);
+    LS_LAUNCH(c, k_rb_init<NQ>, grid, kBlock, 0, rb, (int)c->ti_pad, iv, c->partials);
+    LS_LAUNCH_PDL(c, (k_ti_fin<PH_INIT, NQ>), 1, 32 * ti_values(PH_INIT, NQ), 0, (const double*)c->partials, grid,
+                  c->scal, t0, t1);
     // algorithmic bytes of the two operator applications: FP32 off-diagonals (24 per row)
-    // plus per lane 4 bytes for each vector read or written once
+    // plus per lane 2 bytes for each half-length vector read or written once
     const double v_bytes = (double)g.N * (24.0 + 12.0 * NQ);
-    const double st_bytes = (double)g.N * (24.0 + 20.0 * NQ);
+    const double st_bytes = (double)g.N * (24.0 + 18.0 * NQ);
     int it = 0, batch = 4;
     double sc[TI_STRIDE * 2 + 8];
-    // one right-hand side and an even row length: paired-row kernels
-    const bool pair = (NQ == 1) && (K % 2 == 0);
-    const int N2 = N / 2, JK2 = JK / 2, K2 = K / 2;
-    const int kgrid = pair ? grid_for(c, N2) : grid;
     while (it < max_it) {
         const int nb = std::min(batch, max_it - it);
         for (int b = 0; b < nb; ++b, ++it) {
-            if (it > 0) {
-                if (pair) LS_LAUNCH_PDL(c, k_ti_xp_pair, kgrid, kBlock, 0, N2, iv, (const double*)c->scal);
-                else LS_LAUNCH_PDL(c, k_ti_xp<NQ>, grid, kBlock, 0, N, iv, (const double*)c->scal);
-            }
+            if (it > 0) LS_LAUNCH_PDL(c, k_rb_xp<NQ>, grid, kBlock, 0, rb, iv, (const double*)c->scal);
             {
                 Timed tm(c, LS_T_KRY_APPLY);
-                if (pair) {
-                    if (it == 0)
-                        LS_LAUNCH_PDL(c, k_ti_v_pair<true>, kgrid, kBlock, 0, N2, JK2, K2, op, iv,
-                                  (const double*)c->scal, c->partials);
-                    else
-                        LS_LAUNCH_PDL(c, k_ti_v_pair<false>, kgrid, kBlock, 0, N2, JK2, K2, op, iv,
-                                  (const double*)c->scal, c->partials);
-                } else if (it == 0) {
-                    LS_LAUNCH_PDL(c, (k_ti_v<NQ, true>), grid, kBlock, 0, N, JK, K, op, iv, (const double*)c->scal,
-                              c->partials);
-                } else {
-                    LS_LAUNCH_PDL(c, (k_ti_v<NQ, false>), grid, kBlock, 0, N, JK, K, op, iv, (const double*)c->scal,
-                              c->partials);
-                }
-                if (c->timing) c->timer_bytes[LS_T_KRY_APPLY] += v_bytes + (it == 0 ? 4.0 * NQ * g.N : 0.0);
-            }
-            LS_LAUNCH_PDL(c, (k_ti_fin<PH_V, NQ>), NQ, kFinalizeThreads, 0, (const double*)c->partials, kgrid,
-                      c->scal, c->tcount, 0.0, 0.0);
-            {
-                Timed tm(c, LS_T_KRY_APPLY);
-                if (pair)
-                    LS_LAUNCH_PDL(c, k_ti_st_pair, kgrid, kBlock, 0, N2, JK2, K2, op, iv, (const double*)c->scal,
-                              c->partials);
+                LS_LAUNCH_PDL(c, k_rb_z<NQ>, grid, kBlock, 0, rb, iv, (const float*)(it == 0 ? iv.r : iv.p),
+                              (const double*)c->scal);
+                if (it == 0)
+                    LS_LAUNCH_PDL(c, (k_rb_v<NQ, true>), grid, kBlock, 0, rb, iv, (const double*)c->scal, c->partials);
                 else
-                    LS_LAUNCH_PDL(c, k_ti_st<NQ>, grid, kBlock, 0, N, JK, K, op, iv, (const double*)c->scal,
-                              c->partials);
+                    LS_LAUNCH_PDL(c, (k_rb_v<NQ, false>), grid, kBlock, 0, rb, iv, (const double*)c->scal,
+                                  c->partials);
+                if (c->timing) c->timer_bytes[LS_T_KRY_APPLY] += v_bytes + (it == 0 ? 2.0 * NQ * g.N : 0.0);
+            }
+            LS_LAUNCH_PDL(c, (k_ti_fin<PH_V, NQ>), 1, 32 * ti_values(PH_V, NQ), 0, (const double*)c->partials, grid,
+                          c->scal, 0.0, 0.0);
+            {
+                Timed tm(c, LS_T_KRY_APPLY);
+                LS_LAUNCH_PDL(c, k_rb_zs<NQ>, grid, kBlock, 0, rb, iv, (const double*)c->scal);
+                LS_LAUNCH_PDL(c, k_rb_t<NQ>, grid, kBlock, 0, rb, iv, (const double*)c->scal, c->partials);
                 if (c->timing) c->timer_bytes[LS_T_KRY_APPLY] += st_bytes;
             }
-            LS_LAUNCH_PDL(c, (k_ti_fin<PH_ST, NQ>), 5 * NQ, kFinalizeThreads, 0, (const double*)c->partials, kgrid,
-                      c->scal, c->tcount, 0.0, 0.0);
+            LS_LAUNCH_PDL(c, (k_ti_fin<PH_ST, NQ>), 1, 32 * ti_values(PH_ST, NQ), 0, (const double*)c->partials, grid,
+                          c->scal, 0.0, 0.0);
         }
         LS_TRY(read_scalars(c, TI_BASE, TI_ANY - TI_BASE + 1, sc));
         if (sc[TI_ANY - TI_BASE] == 0.0) break;
@@ -1064,8 +1111,9 @@ static ls_status inner_solve(ls_ctx* c, const TBuf& tb, const int lane_q[NQ], co
             }
         }
     }
-    LS_LAUNCH(c, k_ti_accum<NQ>, grid, kBlock, 0, N, iv, (const double*)c->scal, x[lane_q[0]],
-              NQ > 1 ? x[lane_q[1]] : (double*)nullptr);
+    LS_LAUNCH_PDL(c, k_rb_pending<NQ>, grid, kBlock, 0, rb, iv, (const double*)c->scal);
+    LS_LAUNCH_PDL(c, k_rb_accum<NQ>, grid, kBlock, 0, rb, iv, x[lane_q[0]],
+                  NQ > 1 ? x[lane_q[1]] : (double*)nullptr);
     for (int l = 0; l < NQ; ++l) its[l] = (int)sc[TI_STRIDE * l + TI_ITS];
     return LS_OK;
 }
@@ -1128,10 +1176,11 @@ static ls_status mixed_solve(ls_ctx* c, const Rows<L>& rows, int nrhs, const dou
             if (den[2 + q] == 0.0) *zero_lanes |= 1 << q;
     }
     double rel[2] = {0.0, 0.0}, prev[2] = {INFINITY, INFINITY};
-    int stagnant[2] = {0, 0};
+    int stagnant[2] = {0, 0}, floored[2] = {0, 0};
     const int max_sweeps = 40;
+    const double inner_floor = 1e-6;
     while (mask) {
-        LS_LAUNCH(c, k_t_resid, grid, kBlock, 0, g, tb, x0, x1, c->trhs[0], c->trhs[1], mask,
+        LS_LAUNCH(c, k_t_resid, grid, kBlock, 0, g, tb, x0, x1, c->trhs[0] + c->ti_pad, c->trhs[1] + c->ti_pad, mask,
                   c->partials);
         LS_TRY(finalize_sum(c, grid, 4, S_RED0));
         double h[4];
@@ -1142,7 +1191,12 @@ static ls_status mixed_solve(ls_ctx* c, const Rows<L>& rows, int nrhs, const dou
             if (!((mask >> q) & 1)) continue;
             if (h[2 + q] > 0.0 || h[q] != h[q]) { reason[q] = -4; rel[q] = NAN; mask &= ~(1 << q); continue; }
             rel[q] = den[q] > 0.0 ? sqrt(h[q] / den[q]) : sqrt(h[q]);
-            if (rel[q] <= rtol || h[q] == 0.0) { reason[q] = 2; mask &= ~(1 << q); continue; }
+            // A sweep aims at 0.2 rtol. One that the floor of the inner tolerance stopped above
+            // that is followed by another (an iteration or two) while the residual still falls,
+            // so that the margin holds at tight tolerances too.
+            const bool refine = floored[q] && rel[q] > 0.3 * rtol && rel[q] <= 0.5 * prev[q] && its[q] < max_it &&
+                                sweeps[q] < max_sweeps;
+            if ((rel[q] <= rtol && !refine) || h[q] == 0.0) { reason[q] = 2; mask &= ~(1 << q); continue; }
             if (its[q] >= max_it || sweeps[q] >= max_sweeps) { reason[q] = -3; mask &= ~(1 << q); continue; }
             if (rel[q] > 0.5 * prev[q]) {
                 if (++stagnant[q] >= 6) { reason[q] = -3; mask &= ~(1 << q); continue; }
@@ -1152,7 +1206,9 @@ static ls_status mixed_solve(ls_ctx* c, const Rows<L>& rows, int nrhs, const dou
             prev[q] = rel[q];
             // inner tolerance: what reaches rtol from here (with a margin), floored at what
             // the FP32 inner system still resolves (a relative 1e-6 is ~17 FP32 ulps)
-            tol[q] = std::min(0.5, std::max(1e-6, 0.2 * rtol / std::max(rel[q], 1e-300)));
+            const double want = 0.2 * rtol / std::max(rel[q], 1e-300);
+            floored[q] = want < inner_floor;
+            tol[q] = std::min(0.5, std::max(inner_floor, want));
             solve_mask |= 1 << q;
         }
         if (!solve_mask) break;
