@@ -117,41 +117,82 @@ __global__ void k_dz_scatter(Grid g, const L* __restrict__ label, const float* _
     }
 }
 
-// One voxel of one sub-step (the body of src/Simulation.cpp:475-603).
+// a / b, correctly rounded, for several a and one b > 0, from y = 1 / b correctly rounded: with
+// the quotient within an ulp, one residual correction rounds it correctly (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev.
+// 34(1), 1990); a y is within two ulps, so two corrections. Five FP64 operations instead of a
+// division's dozen or so. For operands whose quotient and residuals stay normal (div_ok).
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+    double q = a * y;
+    q = __fma_rn(__fma_rn(-q, b, a), y, q);
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+__device__ __noinline__ double div_any(double a, double b) { return a / b; }
+__device__ __forceinline__ bool div_ok(double v, int lo, int hi) {  // zero, or 2^lo <= |v| < 2^hi
+    const unsigned int h = (unsigned int)__double2hiint(v) & 0x7fffffffu;
+    return h - ((unsigned int)(1023 + lo) << 20) < ((unsigned int)(hi - lo) << 20) || (h | (unsigned int)__double2loint(v)) == 0u;
+}
+
+// One voxel of one sub-step (the body of src/Simulation.cpp:475-603). A level's time is the
+// chain of one update, so its memory reads go out together: the six neighbours' labels and acid
+// beside the voxel's own state, whatever the labels turn out to be (indices outside the domain
+// read the voxel itself).
 template <typename L>
-__device__ __forceinline__ void dz_voxel(const Grid& g, const DzConst& dc, long long r, L* __restrict__ label,
-                                         float* __restrict__ frac, double* __restrict__ acid,
+__device__ __forceinline__ void dz_voxel(const Grid& g, const DzConst& dc, int r, int i, int j, int k,
+                                         L* __restrict__ label, float* __restrict__ frac, double* __restrict__ acid,
                                          double* __restrict__ precip, double* __restrict__ conc,
                                          int* __restrict__ leached, int* __restrict__ flips) {
-    if (!((int)label[r] >= kSulphide && frac[r] > 0.0f)) return;
-    int i, j, k;
-    decode(g, r, i, j, k);
-    const long long nbs[6] = {r + g.JK, r - g.JK, r + g.K, r - g.K, r + 1, r - 1};
+    const int JK = (int)g.JK;
     const bool val[6] = {i + 1 < g.I, i > 0, j + 1 < g.J, j > 0, k + 1 < g.K, k > 0};
-    double f[6];
+    const int off[6] = {JK, -JK, g.K, -g.K, 1, -1};
+    int nb[6], nt[6];
+    double av[6], f[6];
 #pragma unroll
-    for (int d = 0; d < 6; ++d) f[d] = dz_surface_flux(g, dc, label, acid, val[d], nbs[d]);
+    for (int d = 0; d < 6; ++d) nb[d] = val[d] ? r + off[d] : r;
+    const int t = (int)label[r];
+    const float fr0 = frac[r];
+#pragma unroll
+    for (int d = 0; d < 6; ++d) {
+        nt[d] = (int)label[nb[d]];
+        av[d] = acid[nb[d]];
+    }
+    if (!(t >= kSulphide && fr0 > 0.0f)) return;
+    // calc_surface_flux, src/Simulation.cpp:520-542
+#pragma unroll
+    for (int d = 0; d < 6; ++d) f[d] = (val[d] && (nt[d] == kPore || nt[d] == kRock)) ? dc.k_eff * av[d] : 0.0;
     double flux_sum = f[0] + f[1] + f[2] + f[3] + f[4] + f[5];
     double area_per_face = dc.dx * dc.dx;
     double mass_loss = flux_sum * area_per_face * dc.dt_sub;
     double fractional_loss = dc.vol.div(mass_loss);
-    float fr = (float)((double)frac[r] - (fractional_loss * dc.time_scalar));
-    frac[r] = fr;
-    if (flux_sum > 0.0) {
+    float fr = (float)((double)fr0 - (fractional_loss * dc.time_scalar));
+    if (dpos(flux_sum)) {
+        bool fast = div_ok(flux_sum, -300, 300);
+#pragma unroll
+        for (int d = 0; d < 6; ++d) fast = fast && div_ok(f[d], -600, 300);
+        double nv[6];
+        if (fast) {
+            const double y = __drcp_rn(flux_sum);
+#pragma unroll
+            for (int d = 0; d < 6; ++d) nv[d] = av[d] - fractional_loss * div_by(f[d], flux_sum, y);
+        } else {
+#pragma unroll
+            for (int d = 0; d < 6; ++d) nv[d] = av[d] - fractional_loss * div_any(f[d], flux_sum);
+        }
 #pragma unroll
         for (int d = 0; d < 6; ++d)
-            if (val[d]) acid[nbs[d]] -= fractional_loss * (f[d] / flux_sum);
+            if (val[d] && __double_as_longlong(nv[d]) != __double_as_longlong(av[d])) acid[nb[d]] = nv[d];
     }
-    if ((double)fr <= 1e-4) {
-        frac[r] = 0.0f;
-        if ((int)label[r] == kSulphide) {
+    if (fr <= 1e-4f) {  // (double)fr <= 1e-4: 1e-4f is the largest float below 1e-4
+        if (t == kSulphide) {
             label[r] = (L)kPore;
             precip[r] = 0.0;
             conc[r] = dc.c_sat;
             const int pos = atomicAdd(leached, 1);
-            if (flips) flips[pos] = (int)r;  // a voxel leaches at most once per call
+            if (flips) flips[pos] = r;  // a voxel leaches at most once per call
         }
+        fr = 0.0f;
     }
+    frac[r] = fr;
 }
 
 // Skewed wavefront over the sub-steps. A voxel's update reads and writes only itself and its
@@ -165,7 +206,16 @@ __device__ __forceinline__ void dz_voxel(const Grid& g, const DzConst& dc, long 
 constexpr int kDzSkew = 7;
 
 // The (sub-step, voxel) updates of one level are spread over all threads: the level holds
-// the slices w = level - kDzSkew s of the sub-steps s it covers; one thread per update.
+// the slices w = level - kDzSkew s of the sub-steps s it covers; one thread per update. The
+// schedule does not change during a call, so a thread finds its voxel while the level before
+// still runs (programmatic dependent launch: the state is read after griddepcontrol.wait; the
+// next level is let in only then, since levels queued further ahead take the slots of the SMs
+// that should share the current one: 46 ms a call against 25). What a level then takes is the
+// update's chain: one round trip to L2, some 60 FP64 operations of the warp or two that an SM
+// holds, the hand-over to the next launch. A call at 338x338x283 (1,900 levels of 9,000 updates,
+// 20 sub-steps): 36.7 ms with each face's label, acid and division in turn and ordinary
+// launches; 24.8 with the reads together and dependent launches; 12.7 with the quotients from
+// one reciprocal (670 instructions a warp instead of 1,620). At 64x64x64: 7.8 -> 2.2 ms.
 template <typename L>
 __global__ void __launch_bounds__(kBlock) k_dz_skew(Grid g, DzConst dc, int level, int num_steps, int nlev,
                                                     const int* __restrict__ list, const int* __restrict__ tab,
@@ -182,6 +232,7 @@ __global__ void __launch_bounds__(kBlock) k_dz_skew(Grid g, DzConst dc, int leve
     const int* __restrict__ cumg = tab + (nsk + 1) + __ldg(tab + level);
     constexpr int kDzSliceCap = 512;
     __shared__ int cum[kDzSliceCap + 1];
+    bool waited = false;
     for (int s0 = 0; s0 < ns; s0 += kDzSliceCap) {
         const int m = min(kDzSliceCap, ns - s0);
         const int base = __ldg(cumg + s0);
@@ -189,14 +240,23 @@ __global__ void __launch_bounds__(kBlock) k_dz_skew(Grid g, DzConst dc, int leve
         __syncthreads();
         const int total = cum[m];
         for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
-            int t = 0;
-            while (cum[t + 1] <= idx) ++t;
-            const int w = level - kDzSkew * (s_lo + s0 + t);
-            const long long r = __ldg(list + __ldg(start + w) + (idx - cum[t]));
-            dz_voxel<L>(g, dc, r, label, frac, acid, precip, conc, leached, flips);
+            int lo = 0, hi = m;  // the slice t with cum[t] <= idx < cum[t + 1]
+            while (hi - lo > 1) {
+                const int mid = (lo + hi) >> 1;
+                if (cum[mid] <= idx) lo = mid;
+                else hi = mid;
+            }
+            const int w = level - kDzSkew * (s_lo + s0 + lo);
+            const int r = __ldg(list + __ldg(start + w) + (idx - cum[lo]));
+            int i, j, k;
+            decode(g, r, i, j, k);
+            if (!waited) pdl_enter();
+            waited = true;
+            dz_voxel<L>(g, dc, r, i, j, k, label, frac, acid, precip, conc, leached, flips);
         }
         __syncthreads();
     }
+    if (!waited) pdl_enter();
 }
 
 // ---------------------------------------------------------------------------
@@ -421,7 +481,7 @@ static ls_status dissolve_t(ls_ctx* c, double dt, int* leached_out, ls_substep_i
     // threads per block of the level launches (LS_DZ_THREADS: 32 .. 256)
     static const int dz_threads = [] {
         const char* e = getenv("LS_DZ_THREADS");
-        int v = e ? atoi(e) : 64;
+        int v = e ? atoi(e) : 32;
         if (v < 32) v = 32;
         if (v > kBlock) v = kBlock;
         return (v / 32) * 32;
@@ -455,17 +515,25 @@ static ls_status dissolve_t(ls_ctx* c, double dt, int* leached_out, ls_substep_i
             c->dz_tab_cap = (long long)tab.size();
         }
         LS_CUDA(c, cudaMemcpyAsync(c->dz_tab, tab.data(), sizeof(int) * tab.size(), cudaMemcpyHostToDevice, c->stream));
-        // small blocks: a level holds tens to thousands of updates of ~100 FP64 operations
-        // each (six correctly rounded divisions among them), so its time is the FP64 issue of
-        // the busiest SM; blocks of one or two warps put every warp on its own SM
+        // small blocks: a level holds tens to thousands of updates of ~60 FP64 operations each, so
+        // its time is the chain and the FP64 issue of the busiest SM; blocks of one warp spread
+        // the warps evenly (64 threads: 13.0 against 12.7 ms a call at 338x338x283)
+        bool first = true;
         for (int l = 0; l < nsk; ++l) {
             const long long total = totals[l];
             if (total == 0) continue;
             const int bt = dz_threads;
             const int blocks = (int)std::min<long long>((total + bt - 1) / bt, (long long)c->num_sms * (kBlock / bt) * 8);
-            LS_LAUNCH(c, k_dz_skew<L>, blocks, bt, 0, g, dc, l, num_steps, nlev, (const int*)c->dz_list,
-                      (const int*)c->dz_tab, nsk, (const int*)c->dz_level_start, (L*)c->label, c->frac, c->acid,
-                      c->precip, c->conc, d_leached, flips);
+            // the first level follows the kernels and copies that made the schedule: an ordinary launch
+            if (first)
+                LS_LAUNCH(c, k_dz_skew<L>, blocks, bt, 0, g, dc, l, num_steps, nlev, (const int*)c->dz_list,
+                          (const int*)c->dz_tab, nsk, (const int*)c->dz_level_start, (L*)c->label, c->frac, c->acid,
+                          c->precip, c->conc, d_leached, flips);
+            else
+                LS_LAUNCH_PDL(c, k_dz_skew<L>, blocks, bt, 0, g, dc, l, num_steps, nlev, (const int*)c->dz_list,
+                              (const int*)c->dz_tab, nsk, (const int*)c->dz_level_start, (L*)c->label, c->frac,
+                              c->acid, c->precip, c->conc, d_leached, flips);
+            first = false;
         }
         // the host table must outlive the asynchronous copy: the call ends with a synchronisation
         LS_CUDA(c, cudaStreamSynchronize(c->stream));
