@@ -36,12 +36,25 @@ constexpr int kCoarseSweeps = 48;
 constexpr double kProlongScale = 1.8;
 constexpr int kKLevels = 3;   // levels 1..kKLevels take a K-cycle coarse correction
 constexpr int kKSlot0 = 32;   // device scalar slots of the K-cycle FCG (5 per level)
+// Levels up to these sizes run fused (k_mg_fused). Beyond them 16 SMs take longer for a step than
+// the whole GPU and a launch: with bounds of 3,000 / 9,000 / 30,000 / 50,000 cells a run at
+// 64x64x64 (levels of 32,768, 4,096 and 512) took 74.9 / 73.9 / 74.8 / 74.8 ms, a step of the
+// 224x320x320 flow-through model (44,800, 5,600, 700, 100) 103.7 / 104.3 / 104.5 / 104.5; in FP64 a run
+// at 48x64x64 (24,576, 3,072, 384) took 48.8 ms without the 3,072-cell level and 46.7 with it.
+constexpr long long kFuseCells32 = 9000;
+constexpr long long kFuseCells64 = 8192;
 constexpr int kUnionSpin = 1 << 20;  // bound on the union-find retry loop
 // learned coarse solver (LS_PRESS_LEARNED): the network solves level kLearnedLevel in place of
 // the V-cycle below the K-cycle levels
 constexpr int kLearnedLevel = kKLevels + 1;  // the level below the K-cycle levels
 constexpr float kLpcOutScale = 64.f;  // network output x this x max|D^-1/2 b| = D^1/2 x
 constexpr int kLpcSlot = 60;          // device scalar: max |D^-1/2 b| over the level's members
+
+}  // namespace ls
+
+#include "ls_mg_fused.cuh"
+
+namespace ls {
 
 __device__ __forceinline__ long long lidx(const Grid& g, int i, int j, int k) {
     return (long long)k + (long long)g.K * ((long long)j + (long long)g.J * i);
@@ -263,7 +276,7 @@ __global__ void k_mg_coarse_op(Grid f, Grid cg, const int* __restrict__ fcomp, c
 // ---------------------------------------------------------------------------
 // V-cycle kernels
 
-// One damped-Jacobi update of cell r (shared by the level kernels and the one-block tail)
+// One damped-Jacobi update of cell r
 template <typename T>
 __device__ __forceinline__ T smooth_cell(const Grid& g, long long r, const T* __restrict__ e,
                                          const T* __restrict__ f0, const T* __restrict__ f1,
@@ -562,64 +575,6 @@ __global__ void k_mg_coarsest(Grid g, const int* __restrict__ comp, const T* __r
     coarsest_block(g, comp, e, f0, f1, f2, invd, b, x, t, sweeps);
 }
 
-// The V-cycle over the small coarse levels in one block. The levels from `first` down hold
-// a few thousand cells at most, where a kernel per sweep costs more in launch than in work
-// (the cycle over levels 5-6 of the 338x338x283 workload: 7 launches of ~7 us); one block
-// of 1024 threads runs the same cycle -- the same per-cell updates in the same order, so
-// the same results bit for bit -- with a barrier between sweeps. Level q of the tail reads
-// its right-hand side from b[q] and leaves its correction in x[q] (t[q]: scratch), as the
-// kernels of cycle() do.
-constexpr int kMaxTail = 8;
-template <typename T>
-struct TailLevels {
-    Grid g[kMaxTail];
-    const int* comp[kMaxTail];
-    const T *e[kMaxTail], *f0[kMaxTail], *f1[kMaxTail], *f2[kMaxTail], *invd[kMaxTail];
-    T *x[kMaxTail], *b[kMaxTail], *t[kMaxTail];
-    int n;  // levels in the tail; the last is the coarsest
-};
-
-template <typename T>
-__global__ void __launch_bounds__(1024) k_mg_tail(TailLevels<T> L, T scale, int sweeps) {
-    pdl_enter();
-    const int n = L.n;
-    // down: two smoothing sweeps from zero, then the restricted residual
-    for (int q = 0; q + 1 < n; ++q) {
-        const Grid& g = L.g[q];
-        for (long long r = threadIdx.x; r < g.N; r += blockDim.x)
-            if (L.comp[q][r] >= 0) L.t[q][r] = smooth_cell(g, r, L.e[q], L.f0[q], L.f1[q], L.f2[q], L.invd[q],
-                                                          (const T*)L.b[q], (const T*)nullptr);
-        __syncthreads();
-        for (long long r = threadIdx.x; r < g.N; r += blockDim.x)
-            if (L.comp[q][r] >= 0) L.x[q][r] = smooth_cell(g, r, L.e[q], L.f0[q], L.f1[q], L.f2[q], L.invd[q],
-                                                          (const T*)L.b[q], (const T*)L.t[q]);
-        __syncthreads();
-        const Grid& cg = L.g[q + 1];
-        for (long long R = threadIdx.x; R < cg.N; R += blockDim.x)
-            L.b[q + 1][R] = restrict_cell(g, cg, R, L.comp[q], L.comp[q + 1], L.e[q], L.f0[q], L.f1[q], L.f2[q],
-                                          (const T*)L.b[q], (const T*)L.x[q]);
-        __syncthreads();
-    }
-    const int c = n - 1;
-    coarsest_block(L.g[c], L.comp[c], L.e[c], L.f0[c], L.f1[c], L.f2[c], L.invd[c], (const T*)L.b[c], L.x[c],
-                   L.t[c], sweeps);
-    // up: the scaled coarse correction, then two smoothing sweeps
-    for (int q = n - 2; q >= 0; --q) {
-        const Grid& g = L.g[q];
-        for (long long r = threadIdx.x; r < g.N; r += blockDim.x)
-            prolong_cell(g, L.g[q + 1], r, L.comp[q], L.comp[q + 1], (const T*)L.x[q + 1], L.x[q], scale);
-        __syncthreads();
-        for (long long r = threadIdx.x; r < g.N; r += blockDim.x)
-            if (L.comp[q][r] >= 0) L.t[q][r] = smooth_cell(g, r, L.e[q], L.f0[q], L.f1[q], L.f2[q], L.invd[q],
-                                                          (const T*)L.b[q], (const T*)L.x[q]);
-        __syncthreads();
-        for (long long r = threadIdx.x; r < g.N; r += blockDim.x)
-            if (L.comp[q][r] >= 0) L.x[q][r] = smooth_cell(g, r, L.e[q], L.f0[q], L.f1[q], L.f2[q], L.invd[q],
-                                                          (const T*)L.b[q], (const T*)L.t[q]);
-        __syncthreads();
-    }
-}
-
 // ---------------------------------------------------------------------------
 // learned coarse solver: the network maps (member mask, anchoring fraction e/d, D^-1/2 b / s)
 // on a D x H x W grid holding the level at its origin to D^1/2 x / (s kLpcOutScale), the
@@ -838,11 +793,116 @@ void mg_free(ls_ctx* c) {
     c->mg_is64 = -1;
 }
 
+// Coarse levels of at most this many cells are run by k_mg_fused (LS_MG_TAIL_CELLS overrides it,
+// 0: a kernel per step).
+template <typename T>
+static long long fuse_cells(const ls_ctx* c) {
+    const long long cap = (long long)c->num_sms * 8 * kBlock;  // one cell per thread of a level kernel
+    const long long want = c->mg_tail_cells >= 0 ? c->mg_tail_cells : sizeof(T) == 4 ? kFuseCells32 : kFuseCells64;
+    return std::min(want, cap);
+}
+
+constexpr size_t kFuseSmem = 227 * 1024;
+
+// Slabs and shared memory of the levels in fa; false when a slab would be thinner than a plane
+// (its halo would reach past the neighbouring slabs) or the levels do not fit.
+template <typename T>
+static bool fuse_plan(FuseArgs<T>& fa, int blocks, size_t* smem) {
+    const bool f64 = sizeof(T) == 8;
+    size_t at = 0;
+    fa.nc = 0;
+    for (int q = 0; q < fa.n; ++q)
+        if (f64 || fa.lv[q].g.N > kBlockCells) fa.nc = q + 1;
+    for (int q = 0; q < fa.n; ++q) {
+        FLevel<T>& L = fa.lv[q];
+        const long long N = L.g.N, JK = L.g.JK;
+        L.blk = q >= fa.nc;
+        const long long share = L.blk ? N : (N + blocks - 1) / blocks;
+        L.per = (int)((share + 255) / 256 * 256);
+        L.div_per = make_fastdiv((unsigned int)L.per);
+        auto take = [&](long long n) {
+            const int o = (int)at;
+            at += (size_t)n;
+            return o;
+        };
+        L.oM = (int)(at * sizeof(T));
+        if (q > 0) take((L.per + (long long)sizeof(T) - 1) / (long long)sizeof(T));
+        if (!(f64 && q + 1 == fa.n)) {  // (the coarsest FP64 iterate has its own place)
+            if (!L.blk && JK > L.per) return false;
+            L.oE = take(L.per);
+            L.oW = take(L.per);
+            L.oF0 = take(L.per + JK);
+            L.oF1 = take(L.per + L.g.K);
+            L.oF2 = take(L.per + 1);
+            L.oX = take(L.per + 2 * JK);
+            L.oT = take(L.per + 2 * JK);
+            L.oB = take(L.per);
+            if (q < fa.nk) {
+                L.oZ = take(L.per);
+                L.oQ = take(L.per);
+                L.oV = take(L.per);
+            }
+        }
+        if (at * sizeof(T) > kFuseSmem) return false;
+    }
+    int widest = 0;
+    for (int q = 0; q < fa.nk; ++q) widest = std::max(widest, fa.lv[q].per);
+    fa.oP = (int)at;
+    at += (size_t)widest;
+    *smem = fuse_fixed<T>() + sizeof(T) * at;
+    return *smem <= kFuseSmem;
+}
+
+static void fuse_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&at)[2], int blocks, size_t smem, int pdl) {
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kFuseThreads);
+    cfg.dynamicSmemBytes = smem;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {(unsigned)blocks, 1, 1};
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+}
+
+template <typename T>
+static ls_status fuse_launch(ls_ctx* c, const FuseArgs<T>& fa, size_t smem) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[2];
+    fuse_config(cfg, at, fa.nc > 0 ? c->mg_cluster : 1, smem, c->pdl);
+    cfg.stream = c->stream;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, k_mg_fused<T>, fa);
+    c->launches++;
+    if (e == cudaSuccess) e = cudaGetLastError();
+    return e == cudaSuccess ? LS_OK : check_cuda(c, e, "k_mg_fused");
+}
+
+// The cluster of k_mg_fused: 16 blocks where the device can hold such a cluster, else 8, else
+// none (0: the level kernels).
+template <typename T>
+static int fuse_cluster() {
+    if (cudaFuncSetAttribute(k_mg_fused<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaFuncSetAttribute(k_mg_fused<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFuseSmem) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    for (int blocks = 16; blocks >= 8; blocks /= 2) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[2];
+        fuse_config(cfg, at, blocks, kFuseSmem, 0);
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, k_mg_fused<T>, &cfg) == cudaSuccess && n > 0) return blocks;
+        cudaGetLastError();
+    }
+    return 0;
+}
+
 template <typename T>
 static ls_status mg_alloc(ls_ctx* c) {
     const int is64 = sizeof(T) == 8;
     if (c->mg_is64 == is64) return LS_OK;
     mg_free(c);
+    c->mg_cluster = fuse_cluster<T>();
     if (!c->comp) LS_TRY(walloc_t(c, &c->comp, (size_t)c->g.N));
     if (!c->cc_flag) LS_TRY(dalloc_t(c, &c->cc_flag, (size_t)4));
     LS_TRY(l0_alloc(c, 10, sizeof(T), &c->mg0_x));
@@ -1013,32 +1073,37 @@ ls_status mg_apply(ls_ctx* c, const T* r, T* z, const T* dotv2, int* nblocks_out
         LS_LAUNCH_PDL(c, k_kc_second<T>, gd, kBlock, 0, a.g, a.comp, s, (const T*)pd, e);
         return LS_OK;
     };
-    // the small coarse levels below the K-cycle run as one block (k_mg_tail)
-    size_t tail_start = L + 1;
-    if (c->mg_tail_cells > 0)
-        for (size_t l = L; l > (size_t)kKLevels && l >= 1 && lv[l].g.N <= c->mg_tail_cells; --l) tail_start = l;
-    if (tail_start <= L && L - tail_start + 1 > (size_t)kMaxTail) tail_start = L + 1 - kMaxTail;
+    // the levels from `fuse` down run as one launch each time they are visited (k_mg_fused)
+    size_t fuse = L + 1, fuse_smem = 0;
+    FuseArgs<T> fa = {};
+    if (!learned && c->mg_cluster > 0) {
+        for (size_t l = L >= (size_t)kMaxFuse ? L + 1 - kMaxFuse : 1; l <= L && fuse > L; ++l) {
+            if (lv[l].g.N > fuse_cells<T>(c)) continue;
+            fa = {};
+            fa.n = (int)(L - l + 1);
+            fa.sweeps = kCoarseSweeps;
+            fa.scale = (T)kProlongScale;
+            fa.partials = c->partials;
+            for (int q = 0; q < fa.n; ++q) {
+                const Lv& a = lv[l + q];
+                FLevel<T>& f = fa.lv[q];
+                f.g = a.g;
+                f.comp = a.comp;
+                f.e = a.e;
+                f.f0 = a.f0;
+                f.f1 = a.f1;
+                f.f2 = a.f2;
+                f.invd = a.invd;
+                f.x = a.x;
+                f.b = a.b;
+                f.ev = a.kv[6];
+                if (l + q <= (size_t)kKLevels && l + q < L) fa.nk = q + 1;
+            }
+            if (fuse_plan(fa, c->mg_cluster, &fuse_smem)) fuse = l;
+        }
+    }
     cycle = [&](size_t l, const T* b, T* out, const T* dv, const T* dv2, int* nb) -> ls_status {
         Lv& a = lv[l];
-        if (l >= tail_start && !dv && b == a.b && out == a.x) {
-            TailLevels<T> tl = {};
-            tl.n = (int)(L - l + 1);
-            for (int q = 0; q < tl.n; ++q) {
-                const Lv& m = lv[l + q];
-                tl.g[q] = m.g;
-                tl.comp[q] = m.comp;
-                tl.e[q] = m.e;
-                tl.f0[q] = m.f0;
-                tl.f1[q] = m.f1;
-                tl.f2[q] = m.f2;
-                tl.invd[q] = m.invd;
-                tl.x[q] = m.x;
-                tl.b[q] = m.b;
-                tl.t[q] = m.t;
-            }
-            LS_LAUNCH_PDL(c, k_mg_tail<T>, 1, 1024, 0, tl, (T)kProlongScale, kCoarseSweeps);
-            return LS_OK;
-        }
         if (l == L) {
             LS_LAUNCH_PDL(c, k_mg_coarsest<T>, 1, 1024, 0, a.g, a.comp, a.e, a.f0, a.f1, a.f2, a.invd, b, out, a.t,
                       kCoarseSweeps);
@@ -1061,7 +1126,12 @@ ls_status mg_apply(ls_ctx* c, const T* r, T* z, const T* dotv2, int* nblocks_out
         }
         const T* corr;
         T scale;
-        if (l + 1 <= (size_t)kKLevels && l + 1 < L) {
+        if (l + 1 >= fuse) {
+            LS_TRY(fuse_launch<T>(c, fa, fuse_smem));
+            const bool kc = l + 1 <= (size_t)kKLevels && l + 1 < L;
+            corr = kc ? cl.kv[6] : cl.x;
+            scale = kc ? (T)1 : (T)kProlongScale;
+        } else if (l + 1 <= (size_t)kKLevels && l + 1 < L) {
             LS_TRY(kfcg(l + 1));
             corr = cl.kv[6];
             scale = (T)1;  // the FCG steps carry the optimal scaling

@@ -507,7 +507,7 @@ enum {
     TI_ANY = 100     // 1 while some lane iterates
 };
 __host__ __device__ __forceinline__ int tslot(int l, int v) { return TI_BASE + TI_STRIDE * l + v; }
-static_assert(TI_ANY < S_COUNT, "transport scalars exceed the scalar block");
+static_assert((int)TI_ANY < (int)S_COUNT, "transport scalars exceed the scalar block");
 
 enum { PH_INIT = 0, PH_V = 1, PH_ST = 2 };
 
