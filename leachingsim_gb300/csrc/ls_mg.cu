@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(kBlock) k_mg_smooth(Grid g, const int* __restr
         if (dotv2) acc2 += dotv2[r] * out;
     }
     if (dotv) {
-        double a[2] = {(double)acc, (double)acc2};
+        double a[2] = {widen(acc), widen(acc2)};
         block_sum_store<2>(a, partials);
     }
 }
@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(kBlock) k_mg_smooth0_pair(int N2, int JK2, int
         }
     }
     if (dotv) {
-        double a[2] = {(double)acc, (double)acc2};
+        double a[2] = {widen(acc), widen(acc2)};
         block_sum_store<2>(a, partials);
     }
 }
@@ -500,7 +500,7 @@ __global__ void __launch_bounds__(kBlock) k_kc_apply(Grid g, const int* __restri
         a0 += pd[r] * qv;
         a1 += pd[r] * rr[r];
     }
-    double a[2] = {(double)a0, (double)a1};
+    double a[2] = {widen(a0), widen(a1)};
     block_sum_store<2>(a, partials);
 }
 

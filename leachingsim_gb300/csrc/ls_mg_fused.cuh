@@ -36,10 +36,6 @@ constexpr int kFuseThreads = 1024;
 constexpr int kMaxFuse = 10;
 constexpr int kBlockCells = 2048;
 
-// to double without the FP64 pipe, which a conversion would hold as long as an addition
-__device__ __forceinline__ double widen(float v) { return f2d_exact(v); }
-__device__ __forceinline__ double widen(double v) { return v; }
-
 template <typename T>
 struct FLevel {
     Grid g;

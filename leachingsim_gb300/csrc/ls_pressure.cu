@@ -647,7 +647,7 @@ __global__ void __launch_bounds__(kBlock) k_cg_apply(Grid g, const int8_t* __res
         q[r] = qv;
         a += p[r] * qv;
     }
-    double acc[1] = {(double)a};
+    double acc[1] = {widen(a)};
     block_sum_store<1>(acc, partials);
 }
 
@@ -668,7 +668,7 @@ __global__ void __launch_bounds__(kBlock) k_cg_apply0_pair(int N2, int JK2, int 
         if (l0) { q[2 * t] = qv.x; a += pv.x * qv.x; }
         if (l1) { q[2 * t + 1] = qv.y; a += pv.y * qv.y; }
     }
-    double acc[1] = {(double)a};
+    double acc[1] = {widen(a)};
     block_sum_store<1>(acc, partials);
 }
 
@@ -702,7 +702,7 @@ __global__ void __launch_bounds__(kBlock) k_cg_jacobi(Grid g, const T* __restric
         z[r] = zv;
         a += rv * zv;
     }
-    double acc[1] = {(double)a};
+    double acc[1] = {widen(a)};
     block_sum_store<1>(acc, partials);
 }
 

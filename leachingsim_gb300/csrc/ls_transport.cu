@@ -375,6 +375,11 @@ __global__ void __launch_bounds__(kBlock) k_t_rows(Rows<L> op, TBuf tb, const in
 
 // Also counts, per right-hand side, the rows where b or the solution after k_t_xid (b on
 // identity rows) is nonzero: a system with none has the exact solution x = 0 already.
+// 0.0 + v on the integer pipe: v, with -0.0 as +0.0
+__device__ __forceinline__ double plus_zero(double v) {
+    return __double_as_longlong(v) == (long long)0x8000000000000000ull ? 0.0 : v;
+}
+
 __global__ void __launch_bounds__(kBlock) k_t_rhs(Grid g, double inv_dt, double in0, double in1, TBuf tb,
                                                   int nrhs, const double* f0, const double* f1,
                                                   const double* __restrict__ x0, const double* __restrict__ x1,
@@ -388,13 +393,16 @@ __global__ void __launch_bounds__(kBlock) k_t_rhs(Grid g, double inv_dt, double 
             const double fv = (q ? f1 : f0)[r];
             // trans_row's right-hand side at theta = 1: 0.0 + c_old on Precipitate rows,
             // the inflow value on inflow rows, 0.0 + c_old * (1/dt) on every other row
-            const double rhs = (kind == 1) ? 0.0 + fv : (kind == 3) ? 0.0 + (q ? in1 : in0) : 0.0 + fv * inv_dt;
+            const double rhs = plus_zero(kind == 1 ? fv : kind == 3 ? (q ? in1 : in0) : fv * inv_dt);
             tb.b[q][r] = rhs;
-            double bt = rhs * inv;
-            acc[q] += bt * bt;
             const double xv = (kind == 1 || kind == 3) ? rhs : (q ? x1 : x0)[r];
             const long long m = 0x7fffffffffffffffll;
-            if ((__double_as_longlong(rhs) & m) != 0 || (__double_as_longlong(xv) & m) != 0) nz[q]++;
+            const bool nzb = (__double_as_longlong(rhs) & m) != 0;
+            if (nzb) {  // a zero adds nothing to the norm
+                const double bt = rhs * inv;
+                acc[q] = __fma_rn(bt, bt, acc[q]);
+            }
+            if (nzb || (__double_as_longlong(xv) & m) != 0) nz[q]++;
         }
     }
     acc[2] = (double)nz[0];
@@ -414,49 +422,81 @@ __global__ void k_t_xid(Grid g, TBuf tb, double* x0, double* x1, int nrhs) {
     }
 }
 
-// FP64 A x with the stored coefficients, ascending column order
-__device__ __forceinline__ double t_row_apply(const Grid& g, const TBuf& tb, long long r, int i, int j,
-                                              int k, const double* __restrict__ x) {
-    double acc = 0.0;
-    if (i > 0) acc = __fma_rn(tb.c[2][r], x[r - g.JK], acc);
-    if (j > 0) acc = __fma_rn(tb.c[4][r], x[r - g.K], acc);
-    if (k > 0) acc = __fma_rn(tb.c[6][r], x[r - 1], acc);
-    acc = __fma_rn(tb.c[0][r], x[r], acc);
-    if (k + 1 < g.K) acc = __fma_rn(tb.c[5][r], x[r + 1], acc);
-    if (j + 1 < g.J) acc = __fma_rn(tb.c[3][r], x[r + g.K], acc);
-    if (i + 1 < g.I) acc = __fma_rn(tb.c[1][r], x[r + g.JK], acc);
-    return acc;
+// Outer residual: rhs32 = D^-1 (b - A x) in FP32 (red-black layout); partials sum (D^-1 r)^2
+// and NaN count. MASK: the right-hand sides it runs for. HBM bounds it (84 bytes a row, 98 with
+// the neighbours' second reads) and FP64 issue comes close (nine operations a row, b - A x being
+// fused multiply-subtracts from b: 0.5 ms for 32.3 M rows). The coefficients of links that leave
+// the domain are zero, so their neighbour index is clamped to the row and nothing branches; with
+// an even row length (V = 2) a thread takes two neighbouring rows with 16-byte loads. One
+// right-hand side at 338x338x283: 0.58 ms at 5.4 TB/s (0.97 a row at a time with a branch per
+// link); two: 0.99 ms (1.50).
+struct alignas(16) D2 {
+    double v[2];
+};
+template <int V>
+__device__ __forceinline__ void ld_rows(const double* __restrict__ p, int r, double (&o)[V]) {
+    if (V == 2) {
+        const D2 q = *reinterpret_cast<const D2*>(p + r);
+        o[0] = q.v[0];
+        o[V - 1] = q.v[1];
+    } else {
+        o[0] = p[r];
+    }
 }
 
-// outer residual: rhs32 = D^-1 (b - A x) in FP32 (red-black layout); partials sum (D^-1 r)^2
-// and NaN count
-__global__ void __launch_bounds__(kBlock) k_t_resid(Grid g, TBuf tb, double* x0, double* x1,
-                                                    float* r0, float* r1, int mask,
+template <int MASK, int V>
+__global__ void __launch_bounds__(kBlock) k_t_resid(Grid g, TBuf tb, const double* x0, const double* x1,
+                                                    float* __restrict__ r0, float* __restrict__ r1,
                                                     double* __restrict__ partials) {
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
-         r += (long long)gridDim.x * blockDim.x) {
+    const int n = (int)(g.N / V), JK = (int)g.JK, K = g.K;
+    int nan[2] = {0, 0};
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        const int r = t * V;
         int i, j, k;
         decode(g, r, i, j, k);
-        const double inv = tb.inv[r];
+        const int im = i > 0 ? r - JK : r, ip = i + 1 < g.I ? r + JK : r;
+        const int jm = j > 0 ? r - K : r, jp = j + 1 < g.J ? r + K : r;
+        const int km = k > 0 ? r - 1 : r, kp = k + V < K ? r + V : r;
+        double c[7][V], inv[V];
+#pragma unroll
+        for (int d = 0; d < 7; ++d) ld_rows<V>(tb.c[d], r, c[d]);
+        ld_rows<V>(tb.inv, r, inv);
         int colour;
         const int h = rb_index(tb.rb, i, j, k, colour);
-        const long long at = colour * tb.rb.H + h;
-        // the inner right-hand side in FP32 rounded toward zero on the integer pipe (its
-        // rounding is the inner solve's business; the FP64 pipe bounds this pass)
-        if (mask & 1) {
-            double rv = (tb.b[0][r] - t_row_apply(g, tb, r, i, j, k, x0)) * inv;
-            r0[at] = d2f_rz(rv);
-            acc[0] = __fma_rn(rv, rv, acc[0]);
-            if (disnan(rv)) acc[2] += 1.0;
-        }
-        if (mask & 2) {
-            double rv = (tb.b[1][r] - t_row_apply(g, tb, r, i, j, k, x1)) * inv;
-            r1[at] = d2f_rz(rv);
-            acc[1] = __fma_rn(rv, rv, acc[1]);
-            if (disnan(rv)) acc[3] += 1.0;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            if (!(MASK >> q & 1)) continue;
+            const double* __restrict__ x = q ? x1 : x0;
+            double b[V], xc[V], xim[V], xip[V], xjm[V], xjp[V];
+            ld_rows<V>(tb.b[q], r, b);
+            ld_rows<V>(x, im, xim);
+            ld_rows<V>(x, jm, xjm);
+            ld_rows<V>(x, r, xc);
+            ld_rows<V>(x, jp, xjp);
+            ld_rows<V>(x, ip, xip);
+            const double xkm = x[km], xkp = x[kp];
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+                double a = __fma_rn(-c[0][e], xc[e], b[e]);
+                a = __fma_rn(-c[2][e], xim[e], a);
+                a = __fma_rn(-c[4][e], xjm[e], a);
+                a = __fma_rn(-c[6][e], e == 0 ? xkm : xc[0], a);
+                a = __fma_rn(-c[5][e], e == V - 1 ? xkp : xc[V - 1], a);
+                a = __fma_rn(-c[3][e], xjp[e], a);
+                a = __fma_rn(-c[1][e], xip[e], a);
+                const double rv = a * inv[e];
+                // the inner right-hand side in FP32 rounded toward zero on the integer pipe (its
+                // rounding is the inner solve's business); rows k and k + 1 differ in colour only
+                const long long at = (e ? colour ^ 1 : colour) * tb.rb.H + h;
+                (q ? r1 : r0)[at] = d2f_rz(rv);
+                acc[q] = __fma_rn(rv, rv, acc[q]);
+                nan[q] += disnan(rv) ? 1 : 0;
+            }
         }
     }
+    acc[2] = (double)nan[0];
+    acc[3] = (double)nan[1];
     block_sum_store<4>(acc, partials);
 }
 
@@ -634,20 +674,10 @@ __device__ __forceinline__ Chunk<NQ> rb_links(const RBGrid& g, const TIVec& iv, 
 // block sums of the per-thread FP32 partials, value v of block b at partials[v gridDim + b]
 template <int NV>
 __device__ __forceinline__ void ti_block_sum(const float (&acc)[NV], double* __restrict__ partials) {
-    __shared__ double sh[NV][kBlock / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double v[NV];
 #pragma unroll
-    for (int q = 0; q < NV; ++q) {
-        double x = (double)acc[q];
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-        if (lane == 0) sh[q][warp] = x;
-    }
-    __syncthreads();
-    if (threadIdx.x < NV) {
-        double s = 0.0;
-        for (int w = 0; w < kBlock / 32; ++w) s += sh[threadIdx.x][w];
-        partials[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = s;
-    }
+    for (int q = 0; q < NV; ++q) v[q] = widen(acc[q]);
+    block_sums<NV>(v, partials, (int)gridDim.x, 1);
 }
 
 template <int NQ>
@@ -834,8 +864,9 @@ __global__ void __launch_bounds__(kBlock) k_rb_pending(RBGrid g, TIVec iv, const
     }
 }
 
-// both halves of the correction into the FP64 solution: x_b += d, x_r += f_r - O_r d
-template <int NQ>
+// both halves of the correction into the FP64 solution: x_b += d, x_r += f_r - O_r d (EVEN: the
+// pairs of voxels are 16-byte aligned)
+template <int NQ, bool EVEN>
 __global__ void __launch_bounds__(kBlock) k_rb_accum(RBGrid g, TIVec iv, double* __restrict__ x0,
                                                      double* __restrict__ x1) {
     pdl_enter();
@@ -847,7 +878,8 @@ __global__ void __launch_bounds__(kBlock) k_rb_accum(RBGrid g, TIVec iv, double*
         Chunk<NQ> d;
         const Chunk<NQ> y = rb_links<NQ, 1>(g, iv, ch, src, d);
         const Chunk<NQ> f = red.chunk(h);
-        const int row = h / g.K2p, k2 = h - row * g.K2p, i = row / g.J;
+        const int ch4 = (int)fdiv(NQ == 1 ? g.div4 : g.div2, (unsigned int)ch);
+        const int row = ch4, k2 = h - row * g.K2p, i = (int)fdiv(g.div_j, (unsigned int)row);
         const int par = (row - i * g.J + i) & 1;  // black at k = 2 k2 + par, red at 2 k2 + 1 - par
         const long long base = (long long)row * g.K;
 #pragma unroll
@@ -855,21 +887,30 @@ __global__ void __launch_bounds__(kBlock) k_rb_accum(RBGrid g, TIVec iv, double*
             double* x = (m % NQ) ? x1 : x0;
             const int k0 = 2 * (k2 + m / NQ);
             const float dr = f.v[m] - y.v[m];
-            if (k0 + par < g.K) x[base + k0 + par] += (double)d.v[m];
-            if (k0 + 1 - par < g.K) x[base + k0 + 1 - par] += (double)dr;
+            const double e0 = widen(par ? dr : d.v[m]), e1 = widen(par ? d.v[m] : dr);  // at k0, k0 + 1
+            if (EVEN) {
+                if (k0 < g.K) {
+                    D2* q = reinterpret_cast<D2*>(x + base + k0);
+                    D2 w = *q;
+                    w.v[0] += e0;
+                    w.v[1] += e1;
+                    *q = w;
+                }
+            } else {
+                if (k0 < g.K) x[base + k0] += e0;
+                if (k0 + 1 < g.K) x[base + k0 + 1] += e1;
+            }
         }
     }
 }
 
 __device__ __forceinline__ bool finite_d(double v) { return v == v && fabs(v) < INFINITY; }
 
-// scalar update after a reduction (one thread)
+// scalar update of lane l after a reduction (a thread per lane); whether the lane goes on
 template <int PH, int NQ>
-__device__ void ti_phase(double* scal, const double* red, double tol2_0, double tol2_1) {
-    int any = 0;
-#pragma unroll
-    for (int l = 0; l < NQ; ++l) {
-        double* s = scal + tslot(l, 0);
+__device__ bool ti_phase(double* scal, const double* red, double tol2_0, double tol2_1, int l) {
+    double* s = scal + tslot(l, 0);
+    {
         if (PH == PH_INIT) {
             const double rr = red[l], ff = red[NQ + l];  // the reduced and the whole right-hand side
             s[TI_RR0] = ff;
@@ -925,36 +966,53 @@ __device__ void ti_phase(double* scal, const double* red, double tol2_0, double 
                 s[TI_ALPHA] = s[TI_OMEGA] = s[TI_BETA] = 0.0;
             }
         }
-        if (s[TI_ACT] != 0.0) any = 1;
     }
-    scal[TI_ANY] = any ? 1.0 : 0.0;
+    return s[TI_ACT] != 0.0;
 }
 
 __host__ __device__ constexpr int ti_values(int ph, int nq) { return ph == PH_ST ? 5 * nq : ph == PH_INIT ? 2 * nq : nq; }
+// up to four warps per value
+__host__ __device__ constexpr int ti_fin_threads(int nv) { return 32 * nv * (4 * nv <= 32 ? 4 : 32 / nv); }
 
-// Fixed-order reduction of the per-block partials by one block, a warp per value, and the scalar
-// update of phase PH by its first thread. One block needs no counter across blocks: 4 us where
-// a block per value and an atomic ticket took 9-11 us.
+// Fixed-order reduction of the per-block partials by one block, up to four warps per value, and
+// the scalar update of phase PH by one thread per lane. The block is bound by its SM's FP64 pipe
+// (two additions a clock over up to ten values of 608 partials) and by the update's chain: 7-8 us
+// under a profiler, against 9-11 with a block per value, or with one warp per value and 1,216
+// partials.
 template <int PH, int NQ>
-__global__ void __launch_bounds__(32 * ti_values(PH, NQ)) k_ti_fin(const double* __restrict__ partials, int nblocks,
-                                                                   double* scal, double tol2_0, double tol2_1) {
+__global__ void __launch_bounds__(ti_fin_threads(ti_values(PH, NQ)))
+    k_ti_fin(const double* __restrict__ partials, int nblocks, double* scal, double tol2_0, double tol2_1) {
     pdl_enter();
     if (PH != PH_INIT && scal[TI_ANY] == 0.0) return;
     constexpr int NV = ti_values(PH, NQ);
+    constexpr int WPV = ti_fin_threads(NV) / 32 / NV;  // warps per value
+    __shared__ double part[NV][4];
     __shared__ double red[NV];
-    const int v = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const double* __restrict__ mine = partials + (size_t)v * nblocks;
-    double a[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int b = lane; b < nblocks; b += 128) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if (b + 32 * q < nblocks) a[q] += mine[b + 32 * q];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int v = warp / WPV, w = warp - v * WPV;
+    if (v < NV) {
+        const double* __restrict__ mine = partials + (size_t)v * nblocks;
+        double a[2] = {0.0, 0.0};
+        for (int b = 32 * w + lane; b < nblocks; b += 64 * WPV) {
+            a[0] += mine[b];
+            if (b + 32 * WPV < nblocks) a[1] += mine[b + 32 * WPV];
+        }
+        double x[1] = {a[0] + a[1]};
+        warp_sums<1, 16>(x);
+        if (lane == 0) part[v][w] = x[0];
     }
-    double x = (a[0] + a[1]) + (a[2] + a[3]);
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) red[v] = x;
     __syncthreads();
-    if (threadIdx.x == 0) ti_phase<PH, NQ>(scal, red, tol2_0, tol2_1);
+    if (threadIdx.x < NV) {
+        double x = part[threadIdx.x][0];
+        for (int q = 1; q < WPV; ++q) x += part[threadIdx.x][q];
+        red[threadIdx.x] = x;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const bool on = threadIdx.x < NQ && ti_phase<PH, NQ>(scal, red, tol2_0, tol2_1, (int)threadIdx.x);
+        const bool any = __any_sync(0xffffffffu, on);
+        if (threadIdx.x == 0) scal[TI_ANY] = any ? 1.0 : 0.0;
+    }
 }
 
 // min / max of x over the rows
@@ -1054,6 +1112,9 @@ static ls_status inner_solve(ls_ctx* c, const TBuf& tb, const int lane_q[NQ], co
     const Grid g = c->g;
     const RBGrid rb = tb.rb;
     const int grid = grid_for(c, rb.H / (4 / NQ));
+    // the kernels with dots: four blocks per SM are resident together (up to 56 registers a
+    // thread), and more would only add partial sums
+    const int dgrid = std::min(grid, 4 * c->num_sms);
     TIVec iv;
     float** vecs[kTiVecs] = {&iv.r, &iv.rh, &iv.p, &iv.v, &iv.s, &iv.t, &iv.d, &iv.z};
     for (int v = 0; v < kTiVecs; ++v) *vecs[v] = c->ti + (size_t)v * c->ti_stride + 2 * c->ti_pad;
@@ -1061,8 +1122,8 @@ static ls_status inner_solve(ls_ctx* c, const TBuf& tb, const int lane_q[NQ], co
     iv.rhs[1] = c->trhs[NQ > 1 ? lane_q[1] : lane_q[0]] + c->ti_pad;
     for (int d = 0; d < 6; ++d) iv.o[d] = tb.o[d];
     const double t0 = tol[0] * tol[0], t1 = NQ > 1 ? tol[1] * tol[1] : 0.0;
-    LS_LAUNCH(c, k_rb_init<NQ>, grid, kBlock, 0, rb, (int)c->ti_pad, iv, c->partials);
-    LS_LAUNCH_PDL(c, (k_ti_fin<PH_INIT, NQ>), 1, 32 * ti_values(PH_INIT, NQ), 0, (const double*)c->partials, grid,
+    LS_LAUNCH(c, k_rb_init<NQ>, dgrid, kBlock, 0, rb, (int)c->ti_pad, iv, c->partials);
+    LS_LAUNCH_PDL(c, (k_ti_fin<PH_INIT, NQ>), 1, ti_fin_threads(ti_values(PH_INIT, NQ)), 0, (const double*)c->partials, dgrid,
                   c->scal, t0, t1);
     // algorithmic bytes of the two operator applications: FP32 off-diagonals (24 per row)
     // plus per lane 2 bytes for each half-length vector read or written once
@@ -1079,21 +1140,21 @@ static ls_status inner_solve(ls_ctx* c, const TBuf& tb, const int lane_q[NQ], co
                 LS_LAUNCH_PDL(c, k_rb_z<NQ>, grid, kBlock, 0, rb, iv, (const float*)(it == 0 ? iv.r : iv.p),
                               (const double*)c->scal);
                 if (it == 0)
-                    LS_LAUNCH_PDL(c, (k_rb_v<NQ, true>), grid, kBlock, 0, rb, iv, (const double*)c->scal, c->partials);
+                    LS_LAUNCH_PDL(c, (k_rb_v<NQ, true>), dgrid, kBlock, 0, rb, iv, (const double*)c->scal, c->partials);
                 else
-                    LS_LAUNCH_PDL(c, (k_rb_v<NQ, false>), grid, kBlock, 0, rb, iv, (const double*)c->scal,
+                    LS_LAUNCH_PDL(c, (k_rb_v<NQ, false>), dgrid, kBlock, 0, rb, iv, (const double*)c->scal,
                                   c->partials);
                 if (c->timing) c->timer_bytes[LS_T_KRY_APPLY] += v_bytes + (it == 0 ? 2.0 * NQ * g.N : 0.0);
             }
-            LS_LAUNCH_PDL(c, (k_ti_fin<PH_V, NQ>), 1, 32 * ti_values(PH_V, NQ), 0, (const double*)c->partials, grid,
+            LS_LAUNCH_PDL(c, (k_ti_fin<PH_V, NQ>), 1, ti_fin_threads(ti_values(PH_V, NQ)), 0, (const double*)c->partials, dgrid,
                           c->scal, 0.0, 0.0);
             {
                 Timed tm(c, LS_T_KRY_APPLY);
                 LS_LAUNCH_PDL(c, k_rb_zs<NQ>, grid, kBlock, 0, rb, iv, (const double*)c->scal);
-                LS_LAUNCH_PDL(c, k_rb_t<NQ>, grid, kBlock, 0, rb, iv, (const double*)c->scal, c->partials);
+                LS_LAUNCH_PDL(c, k_rb_t<NQ>, dgrid, kBlock, 0, rb, iv, (const double*)c->scal, c->partials);
                 if (c->timing) c->timer_bytes[LS_T_KRY_APPLY] += st_bytes;
             }
-            LS_LAUNCH_PDL(c, (k_ti_fin<PH_ST, NQ>), 1, 32 * ti_values(PH_ST, NQ), 0, (const double*)c->partials, grid,
+            LS_LAUNCH_PDL(c, (k_ti_fin<PH_ST, NQ>), 1, ti_fin_threads(ti_values(PH_ST, NQ)), 0, (const double*)c->partials, dgrid,
                           c->scal, 0.0, 0.0);
         }
         LS_TRY(read_scalars(c, TI_BASE, TI_ANY - TI_BASE + 1, sc));
@@ -1112,8 +1173,9 @@ static ls_status inner_solve(ls_ctx* c, const TBuf& tb, const int lane_q[NQ], co
         }
     }
     LS_LAUNCH_PDL(c, k_rb_pending<NQ>, grid, kBlock, 0, rb, iv, (const double*)c->scal);
-    LS_LAUNCH_PDL(c, k_rb_accum<NQ>, grid, kBlock, 0, rb, iv, x[lane_q[0]],
-                  NQ > 1 ? x[lane_q[1]] : (double*)nullptr);
+    double* const xl[2] = {x[lane_q[0]], NQ > 1 ? x[lane_q[1]] : (double*)nullptr};
+    if (g.K % 2 == 0) LS_LAUNCH_PDL(c, (k_rb_accum<NQ, true>), grid, kBlock, 0, rb, iv, xl[0], xl[1]);
+    else LS_LAUNCH_PDL(c, (k_rb_accum<NQ, false>), grid, kBlock, 0, rb, iv, xl[0], xl[1]);
     for (int l = 0; l < NQ; ++l) its[l] = (int)sc[TI_STRIDE * l + TI_ITS];
     return LS_OK;
 }
@@ -1180,8 +1242,17 @@ static ls_status mixed_solve(ls_ctx* c, const Rows<L>& rows, int nrhs, const dou
     const int max_sweeps = 40;
     const double inner_floor = 1e-6;
     while (mask) {
-        LS_LAUNCH(c, k_t_resid, grid, kBlock, 0, g, tb, x0, x1, c->trhs[0] + c->ti_pad, c->trhs[1] + c->ti_pad, mask,
-                  c->partials);
+        {
+            float *t0 = c->trhs[0] + c->ti_pad, *t1 = c->trhs[1] + c->ti_pad;
+            const bool two = g.K % 2 == 0;  // pairs of rows stay within a row of voxels, 16-byte aligned
+            const double *y0 = x0, *y1 = x1;
+            if (mask == 3 && two) LS_LAUNCH(c, (k_t_resid<3, 2>), grid, kBlock, 0, g, tb, y0, y1, t0, t1, c->partials);
+            else if (mask == 3) LS_LAUNCH(c, (k_t_resid<3, 1>), grid, kBlock, 0, g, tb, y0, y1, t0, t1, c->partials);
+            else if (mask == 1 && two) LS_LAUNCH(c, (k_t_resid<1, 2>), grid, kBlock, 0, g, tb, y0, y1, t0, t1, c->partials);
+            else if (mask == 1) LS_LAUNCH(c, (k_t_resid<1, 1>), grid, kBlock, 0, g, tb, y0, y1, t0, t1, c->partials);
+            else if (two) LS_LAUNCH(c, (k_t_resid<2, 2>), grid, kBlock, 0, g, tb, y0, y1, t0, t1, c->partials);
+            else LS_LAUNCH(c, (k_t_resid<2, 1>), grid, kBlock, 0, g, tb, y0, y1, t0, t1, c->partials);
+        }
         LS_TRY(finalize_sum(c, grid, 4, S_RED0));
         double h[4];
         LS_TRY(read_scalars(c, S_RED0, 4, h));
