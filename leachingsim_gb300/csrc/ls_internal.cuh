@@ -629,6 +629,17 @@ __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// A scalar of a solver step in every thread of the block, computed by one of them: a division in
+// FP64 by each thread holds the FP64 pipe for 10 us where an SM runs 64 warps (every thread of
+// the block calls it, once).
+template <typename T, typename F>
+__device__ __forceinline__ T block_scalar(F f) {
+    __shared__ T v;
+    if (threadIdx.x == 0) v = f();
+    __syncthreads();
+    return v;
+}
+
 // One block per value: a fixed-order tree reduction of the per-block partials (the
 // result does not depend on timing).
 constexpr int kFinalizeThreads = 256;

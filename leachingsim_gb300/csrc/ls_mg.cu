@@ -549,7 +549,7 @@ __global__ void k_kc_first(Grid g, const int* __restrict__ comp, const double* _
                            const T* __restrict__ pd, const T* __restrict__ q, T* __restrict__ e,
                            T* __restrict__ rr) {
     pdl_enter();
-    const T a = (T)((s[0] > 0.0) ? s[1] / s[0] : 0.0);
+    const T a = block_scalar<T>([=] { return (T)((s[0] > 0.0) ? s[1] / s[0] : 0.0); });
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
          r += (long long)gridDim.x * blockDim.x) {
         if (comp[r] < 0) continue;
@@ -563,7 +563,7 @@ template <typename T>
 __global__ void k_kc_dir(Grid g, const int* __restrict__ comp, const double* __restrict__ s,
                          const T* __restrict__ z, const T* __restrict__ pd0, T* __restrict__ pd1) {
     pdl_enter();
-    const T b = (T)((s[0] > 0.0) ? -s[2] / s[0] : 0.0);
+    const T b = block_scalar<T>([=] { return (T)((s[0] > 0.0) ? -s[2] / s[0] : 0.0); });
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
          r += (long long)gridDim.x * blockDim.x)
         if (comp[r] >= 0) pd1[r] = z[r] + b * pd0[r];
@@ -574,7 +574,7 @@ template <typename T>
 __global__ void k_kc_second(Grid g, const int* __restrict__ comp, const double* __restrict__ s,
                             const T* __restrict__ pd1, T* __restrict__ e) {
     pdl_enter();
-    const T a = (T)((s[3] > 0.0) ? s[4] / s[3] : 0.0);
+    const T a = block_scalar<T>([=] { return (T)((s[3] > 0.0) ? s[4] / s[3] : 0.0); });
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
          r += (long long)gridDim.x * blockDim.x)
         if (comp[r] >= 0) e[r] += a * pd1[r];

@@ -678,8 +678,10 @@ __global__ void k_cg_update(Grid g, const int8_t* __restrict__ kind, const doubl
                             const T* __restrict__ p, const T* __restrict__ q, T* __restrict__ x,
                             T* __restrict__ r_) {
     pdl_enter();
-    const double pq = scal[SP_PQ];
-    const T a = (T)((pq > 0.0) ? scal[SP_RZ] / pq : 0.0);
+    const T a = block_scalar<T>([=] {
+        const double pq = scal[SP_PQ];
+        return (T)((pq > 0.0) ? scal[SP_RZ] / pq : 0.0);
+    });
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
          r += (long long)gridDim.x * blockDim.x) {
         if (kind[r] != 2) continue;
@@ -712,8 +714,9 @@ template <typename T>
 __global__ void k_cg_dir(Grid g, const int8_t* __restrict__ kind, const double* __restrict__ scal,
                          const T* __restrict__ z, T* __restrict__ p, int flexible) {
     pdl_enter();
-    const T beta = (T)(flexible ? ((scal[SP_PQ] > 0.0) ? -scal[SP_ZQ] / scal[SP_PQ] : 0.0)
-                                : scal[SP_RZN] / scal[SP_RZ]);
+    const T beta = block_scalar<T>([=] {
+        return (T)(flexible ? ((scal[SP_PQ] > 0.0) ? -scal[SP_ZQ] / scal[SP_PQ] : 0.0) : scal[SP_RZN] / scal[SP_RZ]);
+    });
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
          r += (long long)gridDim.x * blockDim.x)
         if (kind[r] == 2) p[r] = z[r] + beta * p[r];

@@ -544,6 +544,8 @@ enum {
     TI_ACT,          // 1 while the lane iterates
     TI_ITS,
     TI_REASON,       // 1 converged, -1 breakdown, -4 NaN/Inf
+    TI_F32,          // three slots: alpha, omega and beta as FP32 (k_ti_fin rounds them once;
+                     // a conversion per thread would cost the passes 1-3 us of the FP64 pipe)
     TI_ANY = 100     // 1 while some lane iterates
 };
 __host__ __device__ __forceinline__ int tslot(int l, int v) { return TI_BASE + TI_STRIDE * l + v; }
@@ -680,10 +682,12 @@ __device__ __forceinline__ void ti_block_sum(const float (&acc)[NV], double* __r
     block_sums<NV>(v, partials, (int)gridDim.x, 1);
 }
 
+// v: TI_ALPHA, TI_OMEGA or TI_BETA
 template <int NQ>
 __device__ __forceinline__ void ti_scal(const double* __restrict__ scal, int v, float (&out)[NQ]) {
 #pragma unroll
-    for (int l = 0; l < NQ; ++l) out[l] = (float)scal[tslot(l, v)];
+    for (int l = 0; l < NQ; ++l)
+        out[l] = *reinterpret_cast<const float*>(scal + tslot(l, TI_F32 + v - TI_ALPHA));
 }
 
 // r = rh = f_b - O_b f_r, d = 0, zero halos of the vectors; dots (r, r) and (f, f) per lane
@@ -967,6 +971,8 @@ __device__ bool ti_phase(double* scal, const double* red, double tol2_0, double 
             }
         }
     }
+#pragma unroll
+    for (int v = 0; v < 3; ++v) *reinterpret_cast<float*>(s + TI_F32 + v) = (float)s[TI_ALPHA + v];
     return s[TI_ACT] != 0.0;
 }
 
