@@ -679,7 +679,7 @@ ls_status ls_destroy(ls_ctx* c) {
                     c->shf_visc, c->psb2, c->sat_q, c->dbits, c->sht_label, c->sht_fx, c->sht_fy, c->sht_fz,
                     c->shq_P, c->shq_C, c->shq_K, c->shq_V, c->shq_fx, c->shq_fy, c->shq_fz,
                     c->solid_bits, c->solid_bits_b,
-                    c->wlist, c->wcount, c->olist_counts, c->dz_tab, c->kmult, c->dz_sel, c->dz_flips, c->dz_save_frac,
+                    c->wlist, c->wcount, c->mg0_member, c->olist_counts, c->dz_tab, c->kmult, c->dz_sel, c->dz_flips, c->dz_save_frac,
                     c->dz_save_precip, c->dz_save_conc, c->dz_save_label};
     for (void* q : ptrs) rel(q);
     for (void* q : c->l0base) rel(q);
@@ -697,7 +697,7 @@ ls_status ls_destroy(ls_ctx* c) {
     for (auto& gr : c->mg_graphs)
         if (gr.exec) cudaGraphExecDestroy(gr.exec);
     for (auto& lv : c->mg) {
-        void* lp[] = {lv.comp, lv.e, lv.face[0], lv.face[1], lv.face[2], lv.invd, lv.x, lv.b, lv.t};
+        void* lp[] = {lv.comp, lv.member, lv.e, lv.face[0], lv.face[1], lv.face[2], lv.invd, lv.x, lv.b, lv.t};
         for (void* q : lp) rel(q);
         for (void* q : lv.kv) rel(q);
     }

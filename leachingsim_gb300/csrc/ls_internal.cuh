@@ -217,18 +217,15 @@ __device__ __forceinline__ void block_append(bool pred, int value, int* list, un
 // with the terms in the order -i, -j, -k, +k, +j, +i and separate multiply and add, as the
 // per-cell kernels evaluate it. The arrays are padded (l0pad zero elements on both sides) and
 // faces leaving the domain are zero, so no bounds tests are needed: such terms add 0 * (...).
-__device__ __forceinline__ float2 m0_apply_pair(int t, int JK2, int K2, const float* __restrict__ e,
-                                                const float* __restrict__ f0, const float* __restrict__ f1,
-                                                const float* __restrict__ f2, const float* __restrict__ x) {
-    const int r = 2 * t;
+__device__ __forceinline__ float2 m0_pair(int t, int JK2, int K2, const float* __restrict__ e,
+                                          const float* __restrict__ f0, const float* __restrict__ f1,
+                                          const float* __restrict__ f2, float2 xc, float2 xim, float2 xip, float2 xjm,
+                                          float2 xjp, float xkm, float xkp) {
     const float2 ec = reinterpret_cast<const float2*>(e)[t];
     const float2 f0c = reinterpret_cast<const float2*>(f0)[t], f0m = reinterpret_cast<const float2*>(f0)[t - JK2];
     const float2 f1c = reinterpret_cast<const float2*>(f1)[t], f1m = reinterpret_cast<const float2*>(f1)[t - K2];
     const float2 f2c = reinterpret_cast<const float2*>(f2)[t];
-    const float f2m = f2[r - 1];
-    const float2* x2 = reinterpret_cast<const float2*>(x);
-    const float2 xc = x2[t], xim = x2[t - JK2], xip = x2[t + JK2], xjm = x2[t - K2], xjp = x2[t + K2];
-    const float xkm = x[r - 1], xkp = x[r + 2];
+    const float f2m = f2[2 * t - 1];
     float a0 = ec.x * xc.x;
     a0 += f0m.x * (xc.x - xim.x);
     a0 += f1m.x * (xc.x - xjm.x);
@@ -244,6 +241,14 @@ __device__ __forceinline__ float2 m0_apply_pair(int t, int JK2, int K2, const fl
     a1 += f1c.y * (xc.y - xjp.y);
     a1 += f0c.y * (xc.y - xip.y);
     return make_float2(a0, a1);
+}
+// ... of a stored x
+__device__ __forceinline__ float2 m0_apply_pair(int t, int JK2, int K2, const float* __restrict__ e,
+                                                const float* __restrict__ f0, const float* __restrict__ f1,
+                                                const float* __restrict__ f2, const float* __restrict__ x) {
+    const float2* x2 = reinterpret_cast<const float2*>(x);
+    return m0_pair(t, JK2, K2, e, f0, f1, f2, x2[t], x2[t - JK2], x2[t + JK2], x2[t - K2], x2[t + K2], x[2 * t - 1],
+                   x[2 * t + 2]);
 }
 
 // Timed region record.
@@ -305,9 +310,9 @@ struct ls_ctx {
     void* iface[3];     // link coefficients of the +i, +j, +k faces between two unknowns, T
     void* iinvd;        // 1 / (e + sum of the six links), T
     void* inner[5];     // inner PCG vectors x r z p q, T
-    // the finest-level arrays (ie, iface, iinvd, inner, mg0_x, mg0_t) carry l0pad zero
+    // the finest-level arrays (ie, iface, iinvd, inner, mg0_p, mg0_t) carry l0pad zero
     // elements on both sides, so stencil loads need no bounds tests; l0base holds the
-    // allocations (slots: 0 ie, 1-3 iface, 4 iinvd, 5-9 inner, 10 mg0_x, 11 mg0_t)
+    // allocations (slots: 0 ie, 1-3 iface, 4 iinvd, 5-9 inner, 10 mg0_p, 11 mg0_t)
     void* l0base[12];
     size_t l0bytes[12];
     long long l0pad;
@@ -356,11 +361,12 @@ struct ls_ctx {
     int fx_is_shadow;         // fx / fy / fz equal the change-tracking shadows at every voxel
     double flux_consts[2];
 
-    // multigrid: the finest level is the inner system above (vectors mg0_x, mg0_t);
+    // multigrid: the finest level is the inner system above (vectors z, mg0_t);
     // mg[l] are the coarse levels, each owning its arrays
     struct MGLevel {
         ls::Grid g;
         int* comp;          // owning component of the cell (-1 = no unknown)
+        uint8_t* member;    // 1: the cell's component owns its block on the next level
         void* e;            // excess, T
         void* face[3];      // + face links, T
         void* invd;         // 1 / diagonal, T
@@ -371,8 +377,9 @@ struct ls_ctx {
         int esize;          // sizeof(T)
     };
     std::vector<MGLevel> mg;
-    void* mg0_x;
+    void* mg0_p;          // other buffer of the inner PCG's p (FP32, K even)
     void* mg0_t;
+    uint8_t* mg0_member;  // as MGLevel::member, finest level
     int mg_is64;          // -1 = not allocated
     std::vector<ls::MGGraph> mg_graphs;  // captured preconditioner applications
     int mg_graphs_off;    // 1: launch the cycle kernel by kernel (LS_MG_GRAPHS=0)

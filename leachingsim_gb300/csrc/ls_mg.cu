@@ -247,6 +247,21 @@ __global__ void k_mg_dom(Grid f, Grid cg, const int* __restrict__ fcomp, int* __
     }
 }
 
+// 1 for the fine cells that are members of their own block's owner
+__global__ void k_mg_member(Grid f, Grid cg, const int* __restrict__ fcomp, const int* __restrict__ ccomp,
+                            uint8_t* __restrict__ member) {
+    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < f.N; r += (long long)gridDim.x * blockDim.x) {
+        const int id = fcomp[r];
+        bool m = false;
+        if (id >= 0) {
+            int i, j, k;
+            decode(f, r, i, j, k);
+            m = ccomp[lidx(cg, i >> 1, j >> 1, k >> 1)] == id;
+        }
+        member[r] = m ? 1 : 0;
+    }
+}
+
 // is fine cell (i,j,k) a member of its own block's owner?
 __device__ __forceinline__ bool is_member(const Grid& f, const Grid& cg, const int* fcomp, const int* ccomp,
                                           int i, int j, int k) {
@@ -407,48 +422,180 @@ __global__ void __launch_bounds__(kBlock) k_mg_smooth0_pair(int N2, int JK2, int
     }
 }
 
-// Finest-level residual b - M x of kind-2 cells on pairs (FP32, K even, padded arrays), for
-// the restriction: each fine residual is formed once, by a coalesced fine-cell pass.
-__global__ void __launch_bounds__(kBlock) k_mg_resid0_pair(int N2, int JK2, int K2, const int8_t* __restrict__ kind,
-                                                           const float* __restrict__ e, const float* __restrict__ f0,
-                                                           const float* __restrict__ f1, const float* __restrict__ f2,
-                                                           const float* __restrict__ b, const float* __restrict__ x,
-                                                           float* __restrict__ res) {
+// The two sweeps from zero that begin a cycle, in one pass: t = omega invd b is formed again at
+// the neighbours instead of stored by a pass of its own (cells without an unknown hold b = 0).
+// Finest level of 160x256x256: 45 us instead of 2 x 39.
+template <typename T>
+__global__ void __launch_bounds__(kBlock) k_mg_smooth_two(Grid g, const int* __restrict__ comp,
+                                                          const int8_t* __restrict__ kind0, const T* __restrict__ e,
+                                                          const T* __restrict__ f0, const T* __restrict__ f1,
+                                                          const T* __restrict__ f2, const T* __restrict__ invd,
+                                                          const T* __restrict__ b, T* __restrict__ xo) {
     pdl_enter();
+    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
+         r += (long long)gridDim.x * blockDim.x) {
+        if (!(kind0 ? kind0[r] == 2 : comp[r] >= 0)) continue;
+        int i, j, k;
+        decode(g, r, i, j, k);
+        auto t = [&](long long q) { return (T)kOmega * invd[q] * b[q]; };
+        const T xr = t(r);
+        T acc = e[r] * xr;
+        if (i > 0) acc += f0[r - g.JK] * (xr - t(r - g.JK));
+        if (j > 0) acc += f1[r - g.K] * (xr - t(r - g.K));
+        if (k > 0) acc += f2[r - 1] * (xr - t(r - 1));
+        if (k + 1 < g.K) acc += f2[r] * (xr - t(r + 1));
+        if (j + 1 < g.J) acc += f1[r] * (xr - t(r + g.K));
+        if (i + 1 < g.I) acc += f0[r] * (xr - t(r + g.JK));
+        xo[r] = xr + (T)kOmega * invd[r] * (b[r] - acc);
+    }
+}
+
+// ... on pairs of cells of the finest level (FP32, K even, padded arrays)
+__global__ void __launch_bounds__(kBlock) k_mg_smooth0_two_pair(int N2, int JK2, int K2,
+                                                                const int8_t* __restrict__ kind,
+                                                                const float* __restrict__ e,
+                                                                const float* __restrict__ f0,
+                                                                const float* __restrict__ f1,
+                                                                const float* __restrict__ f2,
+                                                                const float* __restrict__ invd,
+                                                                const float* __restrict__ b, float* __restrict__ xo) {
+    pdl_enter();
+    const float om = (float)kOmega;
+    auto two = [&](int t) {
+        const float2 iv = reinterpret_cast<const float2*>(invd)[t], bv = reinterpret_cast<const float2*>(b)[t];
+        return make_float2(om * iv.x * bv.x, om * iv.y * bv.y);
+    };
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < N2; t += gridDim.x * blockDim.x) {
         const char2 kd = reinterpret_cast<const char2*>(kind)[t];
         const bool l0 = kd.x == 2, l1 = kd.y == 2;
         if (!l0 && !l1) continue;
-        const float2 m = m0_apply_pair(t, JK2, K2, e, f0, f1, f2, x);
-        const float2 bv = reinterpret_cast<const float2*>(b)[t];
-        if (l0) res[2 * t] = bv.x - m.x;
-        if (l1) res[2 * t + 1] = bv.y - m.y;
+        const int r = 2 * t;
+        const float2 iv = reinterpret_cast<const float2*>(invd)[t], bv = reinterpret_cast<const float2*>(b)[t];
+        const float2 xc = make_float2(om * iv.x * bv.x, om * iv.y * bv.y);
+        const float2 m = m0_pair(t, JK2, K2, e, f0, f1, f2, xc, two(t - JK2), two(t + JK2), two(t - K2), two(t + K2),
+                                 om * invd[r - 1] * b[r - 1], om * invd[r + 2] * b[r + 2]);
+        if (l0) xo[r] = xc.x + om * iv.x * (bv.x - m.x);
+        if (l1) xo[r + 1] = xc.y + om * iv.y * (bv.y - m.y);
     }
 }
 
-// coarse right-hand side from stored fine residuals: b_c(R) = sum over owned members, in
-// the child order of k_mg_restrict
+// The prolongation and the sweep after it in one pass: x + scale * x_c(block) of the members is
+// formed again at the neighbours instead of stored by a pass of its own.
+// Piecewise-constant prolongation undershoots smooth error; scaling the coarse correction
+// (over-correction) below the K-cycle levels roughly halves the PCG iterations on these
+// pore-space operators (33 instead of 71 on a 96^3 porosity-0.25 field).
+// All of its neighbours' flags and corrections are L1 hits: on the finest level of 160x256x256 57
+// us instead of 25 + 39.
 template <typename T>
-__global__ void k_mg_restrict_gather(Grid f, Grid cg, const int* __restrict__ fcomp, const int* __restrict__ ccomp,
-                                     const T* __restrict__ res, T* __restrict__ cb) {
+__global__ void __launch_bounds__(kBlock) k_mg_smooth_corr(Grid g, Grid cg, const int* __restrict__ comp,
+                                                           const int8_t* __restrict__ kind0,
+                                                           const uint8_t* __restrict__ member,
+                                                           const T* __restrict__ e, const T* __restrict__ f0,
+                                                           const T* __restrict__ f1, const T* __restrict__ f2,
+                                                           const T* __restrict__ invd, const T* __restrict__ b,
+                                                           const T* __restrict__ x, const T* __restrict__ cx, T scale,
+                                                           T* __restrict__ xo) {
     pdl_enter();
-    for (long long R = blockIdx.x * (long long)blockDim.x + threadIdx.x; R < cg.N;
-         R += (long long)gridDim.x * blockDim.x) {
+    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
+         r += (long long)gridDim.x * blockDim.x) {
+        if (!(kind0 ? kind0[r] == 2 : comp[r] >= 0)) continue;
+        int i, j, k;
+        decode(g, r, i, j, k);
+        const long long R = lidx(cg, i >> 1, j >> 1, k >> 1);
+        auto at = [&](long long q, long long Q) {
+            const T v = x[q], w = v + scale * cx[Q];
+            return member[q] ? w : v;
+        };
+        const T xr = at(r, R);
+        T acc = e[r] * xr;
+        if (i > 0) acc += f0[r - g.JK] * (xr - at(r - g.JK, i & 1 ? R : R - cg.JK));
+        if (j > 0) acc += f1[r - g.K] * (xr - at(r - g.K, j & 1 ? R : R - cg.K));
+        if (k > 0) acc += f2[r - 1] * (xr - at(r - 1, k & 1 ? R : R - 1));
+        if (k + 1 < g.K) acc += f2[r] * (xr - at(r + 1, k & 1 ? R + 1 : R));
+        if (j + 1 < g.J) acc += f1[r] * (xr - at(r + g.K, j & 1 ? R + cg.K : R));
+        if (i + 1 < g.I) acc += f0[r] * (xr - at(r + g.JK, i & 1 ? R + cg.JK : R));
+        xo[r] = xr + (T)kOmega * invd[r] * (b[r] - acc);
+    }
+}
+
+// ... on pairs of cells of the finest level (FP32, K even, padded arrays): the two cells of a pair
+// and the pairs beside it over i and j each lie in one block. Neighbours outside the domain (zero
+// links) read the pair's own flags and block, the unpadded arrays end there.
+__global__ void __launch_bounds__(kBlock) k_mg_smooth0_corr_pair(Grid g, Grid cg, FastDiv div_k2,
+                                                                 const int8_t* __restrict__ kind,
+                                                                 const uint8_t* __restrict__ member,
+                                                                 const float* __restrict__ e,
+                                                                 const float* __restrict__ f0,
+                                                                 const float* __restrict__ f1,
+                                                                 const float* __restrict__ f2,
+                                                                 const float* __restrict__ invd,
+                                                                 const float* __restrict__ b,
+                                                                 const float* __restrict__ x,
+                                                                 const float* __restrict__ cx, float scale,
+                                                                 float* __restrict__ xo) {
+    pdl_enter();
+    const int N2 = (int)(g.N / 2), K2 = g.K / 2, JK2 = (int)(g.JK / 2), CK = cg.K, CJK = (int)cg.JK;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < N2; t += gridDim.x * blockDim.x) {
+        const char2 kd = reinterpret_cast<const char2*>(kind)[t];
+        const bool l0 = kd.x == 2, l1 = kd.y == 2;
+        if (!l0 && !l1) continue;
+        const int r = 2 * t;
+        const int row = (int)fdiv(div_k2, (unsigned int)t), kk = t - row * K2;
+        const int i = (int)fdiv(g.div_jk, (unsigned int)r), j = row - i * g.J;
+        const int R = kk + CK * ((j >> 1) + cg.J * (i >> 1));
+        auto two = [&](int q, bool in, int Q) {
+            const float2 v = reinterpret_cast<const float2*>(x)[q];
+            const uchar2 m = reinterpret_cast<const uchar2*>(member)[in ? q : t];
+            const float c = scale * cx[in ? Q : R];
+            return make_float2(m.x ? v.x + c : v.x, m.y ? v.y + c : v.y);
+        };
+        auto one = [&](int q, bool in, int Q) {
+            const float v = x[q], c = scale * cx[in ? Q : R];
+            return member[in ? q : r] ? v + c : v;
+        };
+        const float2 xc = two(t, true, R);
+        const float2 m = m0_pair(t, JK2, K2, e, f0, f1, f2, xc, two(t - JK2, i > 0, i & 1 ? R : R - CJK),
+                                 two(t + JK2, i + 1 < g.I, i & 1 ? R + CJK : R),
+                                 two(t - K2, j > 0, j & 1 ? R : R - CK),
+                                 two(t + K2, j + 1 < g.J, j & 1 ? R + CK : R), one(r - 1, kk > 0, R - 1),
+                                 one(r + 2, kk + 1 < K2, R + 1));
+        const float2 iv = reinterpret_cast<const float2*>(invd)[t], bv = reinterpret_cast<const float2*>(b)[t];
+        if (l0) xo[r] = xc.x + (float)kOmega * iv.x * (bv.x - m.x);
+        if (l1) xo[r + 1] = xc.y + (float)kOmega * iv.y * (bv.y - m.y);
+    }
+}
+
+// Coarse right-hand side of the finest level on pairs (FP32, K even, padded arrays): a thread
+// forms the residuals of its block's four pairs and sums the members' in the child order of
+// k_mg_restrict. The residuals stay in registers: 54 us instead of 38 for a
+// residual pass and 28 for a gather at 160x256x256.
+__global__ void __launch_bounds__(kBlock) k_mg_restrict0_pair(Grid g, Grid cg, const uint8_t* __restrict__ member,
+                                                              const float* __restrict__ e,
+                                                              const float* __restrict__ f0,
+                                                              const float* __restrict__ f1,
+                                                              const float* __restrict__ f2,
+                                                              const float* __restrict__ b,
+                                                              const float* __restrict__ x, float* __restrict__ cb) {
+    pdl_enter();
+    const int K2 = g.K / 2, JK2 = (int)(g.JK / 2);
+    for (int R = blockIdx.x * blockDim.x + threadIdx.x; R < (int)cg.N; R += gridDim.x * blockDim.x) {
         int I, J, K;
         decode(cg, R, I, J, K);
-        const int own = ccomp[R];
-        T acc = (T)0;
-        if (own >= 0) {
-            for (int a = 0; a < 2; ++a)
-                for (int b = 0; b < 2; ++b)
-                    for (int c = 0; c < 2; ++c) {
-                        int i = 2 * I + a, j = 2 * J + b, k = 2 * K + c;
-                        if (i >= f.I || j >= f.J || k >= f.K) continue;
-                        long long fr = lidx(f, i, j, k);
-                        if (fcomp[fr] != own) continue;
-                        acc += res[fr];
-                    }
-        }
+        float acc = 0.f;
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const int i = 2 * I + a, j = 2 * J + c;
+                if (i >= g.I || j >= g.J) continue;
+                const int t = K + K2 * (j + g.J * i);
+                const uchar2 m = reinterpret_cast<const uchar2*>(member)[t];
+                if (!m.x && !m.y) continue;
+                const float2 ax = m0_apply_pair(t, JK2, K2, e, f0, f1, f2, x);
+                const float2 bv = reinterpret_cast<const float2*>(b)[t];
+                if (m.x) acc += bv.x - ax.x;
+                if (m.y) acc += bv.y - ax.y;
+            }
         cb[R] = acc;
     }
 }
@@ -488,30 +635,6 @@ __global__ void k_mg_restrict(Grid f, Grid cg, const int* __restrict__ fcomp, co
     for (long long R = blockIdx.x * (long long)blockDim.x + threadIdx.x; R < cg.N;
          R += (long long)gridDim.x * blockDim.x)
         cb[R] = restrict_cell(f, cg, R, fcomp, ccomp, e, f0, f1, f2, fb, fx);
-}
-
-template <typename T>
-__device__ __forceinline__ void prolong_cell(const Grid& f, const Grid& cg, long long r, const int* __restrict__ fcomp,
-                                             const int* __restrict__ ccomp, const T* __restrict__ cx,
-                                             T* __restrict__ fx, T scale) {
-    const int id = fcomp[r];
-    if (id < 0) return;
-    int i, j, k;
-    decode(f, r, i, j, k);
-    const long long R = lidx(cg, i >> 1, j >> 1, k >> 1);
-    if (ccomp[R] == id) fx[r] += scale * cx[R];
-}
-
-// x_f += kProlongScale * x_c(block) for owned members. Piecewise-constant prolongation
-// undershoots smooth error; scaling the coarse correction (over-correction) roughly halves the
-// PCG iterations on these pore-space operators (33 instead of 71 on a 96^3 porosity-0.25 field).
-template <typename T>
-__global__ void k_mg_prolong(Grid f, Grid cg, const int* __restrict__ fcomp, const int* __restrict__ ccomp,
-                             const T* __restrict__ cx, T* __restrict__ fx, T scale) {
-    pdl_enter();
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < f.N;
-         r += (long long)gridDim.x * blockDim.x)
-        prolong_cell(f, cg, r, fcomp, ccomp, cx, fx, scale);
 }
 
 // ---------------------------------------------------------------------------
@@ -822,12 +945,14 @@ void mg_free(ls_ctx* c) {
         auto& lv = c->mg[m];
         const size_t n = (size_t)lv.g.N, es = (size_t)lv.esize;
         dfree_t(c, &lv.comp, n);
+        dfree_t(c, &lv.member, n);
         void** lp[] = {&lv.e, &lv.face[0], &lv.face[1], &lv.face[2], &lv.invd, &lv.x, &lv.b, &lv.t};
         for (void** q : lp) dfree(c, q, es * n);
         for (void*& q : lv.kv) dfree(c, &q, es * n);
     }
     c->mg.clear();
-    l0_free(c, 10, &c->mg0_x);
+    dfree_t(c, &c->mg0_member, (size_t)c->g.N);
+    l0_free(c, 10, &c->mg0_p);
     l0_free(c, 11, &c->mg0_t);
     c->mg_is64 = -1;
 }
@@ -944,7 +1069,8 @@ static ls_status mg_alloc(ls_ctx* c) {
     c->mg_cluster = fuse_cluster<T>();
     if (!c->comp) LS_TRY(walloc_t(c, &c->comp, (size_t)c->g.N));
     if (!c->cc_flag) LS_TRY(dalloc_t(c, &c->cc_flag, (size_t)4));
-    LS_TRY(l0_alloc(c, 10, sizeof(T), &c->mg0_x));
+    LS_TRY(walloc_t(c, &c->mg0_member, (size_t)c->g.N));
+    if (!is64 && c->g.K % 2 == 0) LS_TRY(l0_alloc(c, 10, sizeof(T), &c->mg0_p));
     LS_TRY(l0_alloc(c, 11, sizeof(T), &c->mg0_t));
     Grid g = c->g;
     g.NP = g.N;
@@ -954,6 +1080,7 @@ static ls_status mg_alloc(ls_ctx* c) {
         lv.g = cg;
         lv.esize = (int)sizeof(T);
         LS_TRY(walloc_t(c, &lv.comp, (size_t)cg.N));
+        LS_TRY(walloc_t(c, &lv.member, (size_t)cg.N));
         void** arrs[] = {&lv.e, &lv.face[0], &lv.face[1], &lv.face[2], &lv.invd, &lv.x, &lv.b, &lv.t};
         for (void** q : arrs) {
             LS_TRY(walloc(c, q, sizeof(T) * (size_t)cg.N));
@@ -1004,6 +1131,8 @@ ls_status mg_setup(ls_ctx* c) {
         auto& cl = c->mg[l];
         const int cgd = grid_for(c, cl.g.N);
         LS_LAUNCH(c, k_mg_dom, cgd, kBlock, 0, fg, cl.g, fcomp, cl.comp);
+        LS_LAUNCH(c, k_mg_member, grid_for(c, fg.N), kBlock, 0, fg, cl.g, fcomp, (const int*)cl.comp,
+                  l == 0 ? c->mg0_member : c->mg[l - 1].member);
         LS_LAUNCH(c, k_mg_coarse_op<T>, cgd, kBlock, 0, fg, cl.g, fcomp, (const int*)cl.comp, fe, ff[0], ff[1],
                   ff[2], (T*)cl.e, (T*)cl.face[0], (T*)cl.face[1], (T*)cl.face[2]);
         LS_LAUNCH(c, k_level_invd<T>, cgd, kBlock, 0, cl.g, (const int*)cl.comp, (const int8_t*)nullptr,
@@ -1028,7 +1157,7 @@ ls_status mg_setup(ls_ctx* c) {
 // Zero every level vector (the smoother and the PCG skip non-member cells, which must hold 0).
 template <typename T>
 ls_status mg_clear(ls_ctx* c) {
-    LS_CUDA(c, cudaMemsetAsync(c->mg0_x, 0, sizeof(T) * (size_t)c->g.N, c->stream));
+    if (c->mg0_p) LS_CUDA(c, cudaMemsetAsync(c->mg0_p, 0, sizeof(T) * (size_t)c->g.N, c->stream));
     LS_CUDA(c, cudaMemsetAsync(c->mg0_t, 0, sizeof(T) * (size_t)c->g.N, c->stream));
     for (auto& lv : c->mg) {
         const size_t b = sizeof(T) * (size_t)lv.g.N;
@@ -1057,7 +1186,7 @@ ls_status mg_apply(ls_ctx* c, const T* r, T* z, const T* dotv2, int* nblocks_out
     };
     std::vector<Lv> lv(L + 1);
     lv[0] = {c->g, c->comp, (const T*)c->ie, (const T*)c->iface[0], (const T*)c->iface[1], (const T*)c->iface[2],
-             (const T*)c->iinvd, (T*)c->mg0_x, nullptr, (T*)c->mg0_t, {}};
+             (const T*)c->iinvd, z, nullptr, (T*)c->mg0_t, {}};
     for (size_t l = 0; l < L; ++l) {
         auto& m = c->mg[l];
         lv[l + 1] = {m.g, m.comp, (const T*)m.e, (const T*)m.face[0], (const T*)m.face[1], (const T*)m.face[2],
@@ -1150,17 +1279,20 @@ ls_status mg_apply(ls_ctx* c, const T* r, T* z, const T* dotv2, int* nblocks_out
             return LS_OK;
         }
         Lv& cl = lv[l + 1];
-        LS_TRY(smooth(l, b, (const T*)nullptr, a.t, nullptr, nullptr, nullptr));
-        LS_TRY(smooth(l, b, (const T*)a.t, a.x, nullptr, nullptr, nullptr));
+        const int gd = grid_for(c, a.g.N);
+        const int N2 = (int)(a.g.N / 2), JK2 = (int)(a.g.JK / 2), K2 = a.g.K / 2;
+        const int8_t* kind0 = l == 0 ? (const int8_t*)c->pkind : (const int8_t*)nullptr;
+        const uint8_t* member = l == 0 ? c->mg0_member : c->mg[l - 1].member;
         if (l == 0 && pair0) {
-            // residual into the free ping-pong buffer, then the per-block sums
-            const int N2 = (int)(a.g.N / 2);
-            LS_LAUNCH_PDL(c, k_mg_resid0_pair, grid_for(c, N2), kBlock, 0, N2, (int)(a.g.JK / 2), a.g.K / 2,
-                      (const int8_t*)c->pkind, (const float*)a.e, (const float*)a.f0, (const float*)a.f1,
-                      (const float*)a.f2, (const float*)b, (const float*)a.x, (float*)a.t);
-            LS_LAUNCH_PDL(c, k_mg_restrict_gather<T>, grid_for(c, cl.g.N), kBlock, 0, a.g, cl.g, a.comp, cl.comp,
-                      (const T*)a.t, cl.b);
+            LS_LAUNCH_PDL(c, k_mg_smooth0_two_pair, grid_for(c, N2), kBlock, 0, N2, JK2, K2, kind0, (const float*)a.e,
+                      (const float*)a.f0, (const float*)a.f1, (const float*)a.f2, (const float*)a.invd,
+                      (const float*)b, (float*)a.x);
+            LS_LAUNCH_PDL(c, k_mg_restrict0_pair, grid_for(c, cl.g.N), kBlock, 0, a.g, cl.g, member, (const float*)a.e,
+                      (const float*)a.f0, (const float*)a.f1, (const float*)a.f2, (const float*)b, (const float*)a.x,
+                      (float*)cl.b);
         } else {
+            LS_LAUNCH_PDL(c, k_mg_smooth_two<T>, gd, kBlock, 0, a.g, a.comp, kind0, a.e, a.f0, a.f1, a.f2, a.invd, b,
+                      a.x);
             LS_LAUNCH_PDL(c, k_mg_restrict<T>, grid_for(c, cl.g.N), kBlock, 0, a.g, cl.g, a.comp, cl.comp, a.e, a.f0,
                       a.f1, a.f2, b, (const T*)a.x, cl.b);
         }
@@ -1184,9 +1316,14 @@ ls_status mg_apply(ls_ctx* c, const T* r, T* z, const T* dotv2, int* nblocks_out
             corr = cl.x;
             scale = (T)kProlongScale;
         }
-        LS_LAUNCH_PDL(c, k_mg_prolong<T>, grid_for(c, a.g.N), kBlock, 0, a.g, cl.g, a.comp, cl.comp, corr, a.x,
-                  scale);
-        LS_TRY(smooth(l, b, (const T*)a.x, a.t, nullptr, nullptr, nullptr));
+        if (l == 0 && pair0)
+            LS_LAUNCH_PDL(c, k_mg_smooth0_corr_pair, grid_for(c, N2), kBlock, 0, a.g, cl.g, make_fastdiv((unsigned)K2),
+                      kind0, member, (const float*)a.e, (const float*)a.f0, (const float*)a.f1, (const float*)a.f2,
+                      (const float*)a.invd, (const float*)b, (const float*)a.x, (const float*)corr, (float)scale,
+                      (float*)a.t);
+        else
+            LS_LAUNCH_PDL(c, k_mg_smooth_corr<T>, gd, kBlock, 0, a.g, cl.g, a.comp, kind0, member, a.e, a.f0, a.f1, a.f2,
+                      a.invd, b, (const T*)a.x, corr, scale, a.t);
         return smooth(l, b, (const T*)a.t, out, dv, dv2, nb);
     };
     return cycle(0, r, z, r, dotv2, nblocks_out);

@@ -672,6 +672,44 @@ __global__ void __launch_bounds__(kBlock) k_cg_apply0_pair(int N2, int JK2, int 
     block_sum_store<1>(acc, partials);
 }
 
+// The direction and the product of one CG iteration in one pass (flexible CG, FP32, K even):
+// po = z + beta p of the unknowns, formed again at the neighbours, and q = M po with the partial
+// (po, q). z and p are read and po is written once, without
+// k_cg_dir's pass, bound by DRAM: 52 us instead of 28 + 36 at 160x256x256.
+__global__ void __launch_bounds__(kBlock) k_cg_dir_apply0_pair(int N2, int JK2, int K2,
+                                                               const int8_t* __restrict__ kind,
+                                                               const double* __restrict__ scal,
+                                                               const float* __restrict__ z,
+                                                               const float* __restrict__ p, float* __restrict__ po,
+                                                               const float* __restrict__ e,
+                                                               const float* __restrict__ w0,
+                                                               const float* __restrict__ w1,
+                                                               const float* __restrict__ w2, float* __restrict__ q,
+                                                               double* __restrict__ partials) {
+    pdl_enter();
+    const float beta = block_scalar<float>([=] {
+        return (float)((scal[SP_PQ] > 0.0) ? -scal[SP_ZQ] / scal[SP_PQ] : 0.0);
+    });
+    auto two = [&](int t) {
+        const float2 zv = reinterpret_cast<const float2*>(z)[t], pv = reinterpret_cast<const float2*>(p)[t];
+        return make_float2(zv.x + beta * pv.x, zv.y + beta * pv.y);
+    };
+    float a = 0.f;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < N2; t += gridDim.x * blockDim.x) {
+        const char2 kd = reinterpret_cast<const char2*>(kind)[t];
+        const bool l0 = kd.x == 2, l1 = kd.y == 2;
+        if (!l0 && !l1) continue;
+        const int r = 2 * t;
+        const float2 pc = two(t);
+        const float2 qv = m0_pair(t, JK2, K2, e, w0, w1, w2, pc, two(t - JK2), two(t + JK2), two(t - K2), two(t + K2),
+                                  z[r - 1] + beta * p[r - 1], z[r + 2] + beta * p[r + 2]);
+        if (l0) { po[r] = pc.x; q[r] = qv.x; a += pc.x * qv.x; }
+        if (l1) { po[r + 1] = pc.y; q[r + 1] = qv.y; a += pc.y * qv.y; }
+    }
+    double acc[1] = {widen(a)};
+    block_sum_store<1>(acc, partials);
+}
+
 // x += a p, r -= a q with a = (r,z)/(p,q) (0 when (p,q) <= 0)
 template <typename T>
 __global__ void k_cg_update(Grid g, const int8_t* __restrict__ kind, const double* __restrict__ scal,
@@ -763,6 +801,8 @@ static ls_status inner_pcg(ls_ctx* c, bool use_mg, double tol, int max_it, int* 
     T* z = (T*)c->inner[2];
     T* p = (T*)c->inner[3];
     T* q = (T*)c->inner[4];
+    T* p_other = (T*)c->mg0_p;
+    const bool pair = std::is_same<T, float>::value && c->g.K % 2 == 0;
     const T* e = (const T*)c->ie;
     const T* w0 = (const T*)c->iface[0];
     const T* w1 = (const T*)c->iface[1];
@@ -808,17 +848,26 @@ static ls_status inner_pcg(ls_ctx* c, bool use_mg, double tol, int max_it, int* 
     for (int it = 0; it < max_it; ++it) {
         {
             Timed tm(c, LS_T_CG_APPLY);
-            if (std::is_same<T, float>::value && g.K % 2 == 0)
+            if (pair && use_mg && it > 0) {
+                LS_LAUNCH_PDL(c, k_cg_dir_apply0_pair, pgrid, kBlock, 0, (int)(g.N / 2), (int)(g.JK / 2), g.K / 2,
+                          (const int8_t*)c->pkind, (const double*)c->scal, (const float*)z, (const float*)p,
+                          (float*)p_other, (const float*)e, (const float*)w0, (const float*)w1, (const float*)w2,
+                          (float*)q, c->partials);
+                std::swap(p, p_other);
+                if (c->timing) c->timer_bytes[LS_T_CG_APPLY] += (double)g.N * 2.0 * sizeof(T);  // z in, p out
+            } else if (pair) {
                 LS_LAUNCH_PDL(c, k_cg_apply0_pair, pgrid, kBlock, 0, (int)(g.N / 2), (int)(g.JK / 2), g.K / 2,
                           (const int8_t*)c->pkind, (const float*)p, (const float*)e, (const float*)w0,
                           (const float*)w1, (const float*)w2, (float*)q, c->partials);
-            else
+            } else {
                 LS_LAUNCH_PDL(c, k_cg_apply<T>, grid, kBlock, 0, g, (const int8_t*)c->pkind, (const T*)p, e, w0, w1,
                           w2, q, c->partials);
+            }
             // p in, excess and three own face links, q out
             if (c->timing) c->timer_bytes[LS_T_CG_APPLY] += (double)g.N * 6.0 * sizeof(T);
         }
-        LS_TRY(finalize_sum(c, (std::is_same<T, float>::value && g.K % 2 == 0) ? pgrid : grid, 1, SP_PQ));
+        if (it > 0) LS_LAUNCH_PDL(c, k_set_scalar, 1, 1, 0, c->scal, SP_RZ, SP_RZN);
+        LS_TRY(finalize_sum(c, pair ? pgrid : grid, 1, SP_PQ));
         LS_LAUNCH_PDL(c, k_cg_update<T>, grid, kBlock, 0, g, (const int8_t*)c->pkind, (const double*)c->scal,
                   (const T*)p, (const T*)q, x, r);
         LS_TRY(precondition(SP_RZN, (const T*)q));
@@ -849,9 +898,9 @@ static ls_status inner_pcg(ls_ctx* c, bool use_mg, double tol, int max_it, int* 
         }
         if (rz != rz) return set_error(c, LS_NONFINITE, "pressure: NaN in inner PCG");
         if (rz <= target || !(pq > 0.0) || rz < 0.0) break;
-        LS_LAUNCH_PDL(c, k_cg_dir<T>, grid, kBlock, 0, g, (const int8_t*)c->pkind, (const double*)c->scal,
-                  (const T*)z, p, use_mg ? 1 : 0);
-        LS_LAUNCH_PDL(c, k_set_scalar, 1, 1, 0, c->scal, SP_RZ, SP_RZN);
+        if (!(pair && use_mg))
+            LS_LAUNCH_PDL(c, k_cg_dir<T>, grid, kBlock, 0, g, (const int8_t*)c->pkind, (const double*)c->scal,
+                      (const T*)z, p, use_mg ? 1 : 0);
     }
     *rel_out = sqrt(std::max(rz, 0.0) / rz0);
     return LS_OK;
