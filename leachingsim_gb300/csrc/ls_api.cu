@@ -658,6 +658,7 @@ ls_status ls_destroy(ls_ctx* c) {
     if (!c) return LS_OK;
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->snap_stream) cudaStreamSynchronize(c->snap_stream);
+    mg_free(c);
     // device arrays of dalloc
     auto rel = [c](void* q) {
         if (!q || in_arena(c, q)) return;  // arrays cut from the arena go with it
@@ -679,7 +680,7 @@ ls_status ls_destroy(ls_ctx* c) {
                     c->shf_visc, c->psb2, c->sat_q, c->dbits, c->sht_label, c->sht_fx, c->sht_fy, c->sht_fz,
                     c->shq_P, c->shq_C, c->shq_K, c->shq_V, c->shq_fx, c->shq_fy, c->shq_fz,
                     c->solid_bits, c->solid_bits_b,
-                    c->wlist, c->wcount, c->mg0_member, c->olist_counts, c->dz_tab, c->kmult, c->dz_sel, c->dz_flips, c->dz_save_frac,
+                    c->wlist, c->wcount, c->olist_counts, c->dz_tab, c->kmult, c->dz_sel, c->dz_flips, c->dz_save_frac,
                     c->dz_save_precip, c->dz_save_conc, c->dz_save_label};
     for (void* q : ptrs) rel(q);
     for (void* q : c->l0base) rel(q);
@@ -693,13 +694,6 @@ ls_status ls_destroy(ls_ctx* c) {
         void* lp[] = {c->lpc_c0, c->lpc_c1, c->lpc_c2, c->lpc_out, c->lpc_isd, c->lpc_anchor};
         for (void* q : lp) rel(q);
         if (c->lpc) ls_lpnet_destroy(c->lpc);
-    }
-    for (auto& gr : c->mg_graphs)
-        if (gr.exec) cudaGraphExecDestroy(gr.exec);
-    for (auto& lv : c->mg) {
-        void* lp[] = {lv.comp, lv.member, lv.e, lv.face[0], lv.face[1], lv.face[2], lv.invd, lv.x, lv.b, lv.t};
-        for (void* q : lp) rel(q);
-        for (void* q : lv.kv) rel(q);
     }
     if (c->h_scal) cudaFreeHost(c->h_scal);
     if (c->h_int) cudaFreeHost(c->h_int);

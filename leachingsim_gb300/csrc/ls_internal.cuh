@@ -365,21 +365,22 @@ struct ls_ctx {
     // mg[l] are the coarse levels, each owning its arrays
     struct MGLevel {
         ls::Grid g;
+        // the arrays but comp carry the zero pads of level_pad cells on both sides
         int* comp;          // owning component of the cell (-1 = no unknown)
-        uint8_t* member;    // 1: the cell's component owns its block on the next level
+        uint8_t* flags;     // kCellLive: an unknown, kCellMember: its component owns its block on the next level
         void* e;            // excess, T
         void* face[3];      // + face links, T
         void* invd;         // 1 / diagonal, T
         void* x;            // T
         void* b;            // T
         void* t;            // T
-        void* kv[7];        // K-cycle vectors on this level (rr, za, zb, pd, q0, q1, e), T, or null
+        void* kv[6];        // K-cycle vectors on this level (za, zb, pd, q0, q1, e), T, or null
         int esize;          // sizeof(T)
     };
     std::vector<MGLevel> mg;
     void* mg0_p;          // other buffer of the inner PCG's p (FP32, K even)
     void* mg0_t;
-    uint8_t* mg0_member;  // as MGLevel::member, finest level
+    uint8_t* mg0_flags;   // as MGLevel::flags, finest level
     int mg_is64;          // -1 = not allocated
     std::vector<ls::MGGraph> mg_graphs;  // captured preconditioner applications
     int mg_graphs_off;    // 1: launch the cycle kernel by kernel (LS_MG_GRAPHS=0)

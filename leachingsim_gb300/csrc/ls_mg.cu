@@ -76,6 +76,38 @@ __device__ __forceinline__ T m_apply(const Grid& g, long long r, int i, int j, i
     return acc;
 }
 
+// The same on arrays with zero pads of a plane on both sides (level_pad): a link out of the box is
+// a stored 0 and its other end is read from the pad or from the next row, so the index needs no
+// decoding and all reads are under way together. With the bounds as branches each face waited
+// for the one before: on the 4.0M cells of the first coarse level of 338x338x283 a sweep took 60
+// us, now 31, and the sweep with the correction 104, now 36. at(q) is x of cell q.
+template <typename T, typename F>
+__device__ __forceinline__ T m_cell(int r, int JK, int K, const T* __restrict__ e, const T* __restrict__ f0,
+                                    const T* __restrict__ f1, const T* __restrict__ f2, T xr, F at) {
+    const T er = e[r], l0m = f0[r - JK], l1m = f1[r - K], l2m = f2[r - 1], l2 = f2[r], l1 = f1[r], l0 = f0[r];
+    const T xim = at(r - JK), xjm = at(r - K), xkm = at(r - 1), xkp = at(r + 1), xjp = at(r + K), xip = at(r + JK);
+    T acc = er * xr;
+    acc += l0m * (xr - xim);
+    acc += l1m * (xr - xjm);
+    acc += l2m * (xr - xkm);
+    acc += l2 * (xr - xkp);
+    acc += l1 * (xr - xjp);
+    acc += l0 * (xr - xip);
+    return acc;
+}
+
+// Resident blocks per SM of the passes that hold more than 32 registers and sum nothing, whose
+// grid is that many blocks per SM: with grid_for's 8 a second, partly filled wave followed (the
+// finest sweep with the correction at 338x338x283: 186 us, now 163). 4, 5 or 6: the step with
+// acid there takes 81.1, 80.8 or 81.1 ms. The passes that leave partial sums keep grid_for's
+// grid, which is part of the order of their sums.
+constexpr int kPassBlocks = 5;
+static int pass_grid(const ls_ctx* c, long long n) { return std::min(grid_for(c, n), c->num_sms * kPassBlocks); }
+
+constexpr uint8_t kCellMember = 1, kCellLive = 2;
+
+static size_t level_pad(const Grid& g) { return ((size_t)g.JK + 31) / 32 * 32; }
+
 // 1 / (e + sum of the six links) of live cells, 1 elsewhere
 template <typename T>
 __global__ void k_level_invd(Grid g, const int* __restrict__ comp, const int8_t* __restrict__ kind,
@@ -247,18 +279,17 @@ __global__ void k_mg_dom(Grid f, Grid cg, const int* __restrict__ fcomp, int* __
     }
 }
 
-// 1 for the fine cells that are members of their own block's owner
-__global__ void k_mg_member(Grid f, Grid cg, const int* __restrict__ fcomp, const int* __restrict__ ccomp,
-                            uint8_t* __restrict__ member) {
+__global__ void k_mg_flags(Grid f, Grid cg, const int* __restrict__ fcomp, const int* __restrict__ ccomp,
+                           uint8_t* __restrict__ flags) {
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < f.N; r += (long long)gridDim.x * blockDim.x) {
         const int id = fcomp[r];
-        bool m = false;
+        int out = 0;
         if (id >= 0) {
             int i, j, k;
             decode(f, r, i, j, k);
-            m = ccomp[lidx(cg, i >> 1, j >> 1, k >> 1)] == id;
+            out = kCellLive | (ccomp[lidx(cg, i >> 1, j >> 1, k >> 1)] == id ? kCellMember : 0);
         }
-        member[r] = m ? 1 : 0;
+        flags[r] = (uint8_t)out;
     }
 }
 
@@ -330,42 +361,25 @@ __global__ void k_mg_coarse_op(Grid f, Grid cg, const int* __restrict__ fcomp, c
 // ---------------------------------------------------------------------------
 // V-cycle kernels
 
-// One damped-Jacobi update of cell r
+// x_out = x + omega invd (b - M x), a damped-Jacobi sweep. With dotv, the per-block partial of
+// (dotv, x_out) is stored (the (r, z) of the PCG).
+// Cells that are not unknowns keep 0 in every level vector: the buffers are cleared when
+// allocated and nothing writes them there, so the smoother skips them.
 template <typename T>
-__device__ __forceinline__ T smooth_cell(const Grid& g, long long r, const T* __restrict__ e,
-                                         const T* __restrict__ f0, const T* __restrict__ f1,
-                                         const T* __restrict__ f2, const T* __restrict__ invd,
-                                         const T* __restrict__ b, const T* __restrict__ x) {
-    const T bv = b[r];
-    if (x) {
-        int i, j, k;
-        decode(g, r, i, j, k);
-        const T res = bv - m_apply(g, r, i, j, k, e, f0, f1, f2, x);
-        return x[r] + (T)kOmega * invd[r] * res;
-    }
-    return (T)kOmega * invd[r] * bv;
-}
-
-// x_out = x + omega invd (b - M x); x == nullptr means x = 0. With dotv, the per-block
-// partial of (dotv, x_out) is stored (the (r, z) of the PCG).
-// Cells that are not members keep 0 in every level vector: the buffers are cleared when
-// allocated and nothing writes them there, so the smoother skips them (membership from the
-// 1-byte kind on the finest level, the component id on coarse levels).
-template <typename T>
-__global__ void __launch_bounds__(kBlock) k_mg_smooth(Grid g, const int* __restrict__ comp,
-                                                      const int8_t* __restrict__ kind0, const T* __restrict__ e,
-                                                      const T* __restrict__ f0, const T* __restrict__ f1,
-                                                      const T* __restrict__ f2, const T* __restrict__ invd,
-                                                      const T* __restrict__ b, const T* __restrict__ x,
-                                                      T* __restrict__ xo, const T* __restrict__ dotv,
-                                                      const T* __restrict__ dotv2, double* __restrict__ partials) {
+__global__ void __launch_bounds__(kBlock) k_mg_smooth(int N, int JK, int K, const uint8_t* __restrict__ flags,
+                                                      const T* __restrict__ e, const T* __restrict__ f0,
+                                                      const T* __restrict__ f1, const T* __restrict__ f2,
+                                                      const T* __restrict__ invd, const T* __restrict__ b,
+                                                      const T* __restrict__ x, T* __restrict__ xo,
+                                                      const T* __restrict__ dotv, const T* __restrict__ dotv2,
+                                                      double* __restrict__ partials) {
     pdl_enter();
     T acc = (T)0, acc2 = (T)0;
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
-         r += (long long)gridDim.x * blockDim.x) {
-        const bool live = kind0 ? kind0[r] == 2 : comp[r] >= 0;
-        if (!live) continue;
-        const T out = smooth_cell(g, r, e, f0, f1, f2, invd, b, x);
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < N; r += gridDim.x * blockDim.x) {
+        if (!flags[r]) continue;
+        const T xr = x[r], bv = b[r], iv = invd[r];
+        const T res = bv - m_cell(r, JK, K, e, f0, f1, f2, xr, [=](int q) { return x[q]; });
+        const T out = xr + (T)kOmega * iv * res;
         xo[r] = out;
         if (dotv) acc += dotv[r] * out;
         if (dotv2) acc2 += dotv2[r] * out;
@@ -393,18 +407,12 @@ __global__ void __launch_bounds__(kBlock) k_mg_smooth0_pair(int N2, int JK2, int
         const char2 kd = reinterpret_cast<const char2*>(kind)[t];
         const bool l0 = kd.x == 2, l1 = kd.y == 2;
         if (!l0 && !l1) continue;
+        const float2 m = m0_apply_pair(t, JK2, K2, e, f0, f1, f2, x);
+        const float2 xv = reinterpret_cast<const float2*>(x)[t];
         const float2 bv = reinterpret_cast<const float2*>(b)[t];
         const float2 iv = reinterpret_cast<const float2*>(invd)[t];
-        float o0, o1;
-        if (x) {
-            const float2 m = m0_apply_pair(t, JK2, K2, e, f0, f1, f2, x);
-            const float2 xv = reinterpret_cast<const float2*>(x)[t];
-            o0 = xv.x + (float)kOmega * iv.x * (bv.x - m.x);
-            o1 = xv.y + (float)kOmega * iv.y * (bv.y - m.y);
-        } else {
-            o0 = (float)kOmega * iv.x * bv.x;
-            o1 = (float)kOmega * iv.y * bv.y;
-        }
+        const float o0 = xv.x + (float)kOmega * iv.x * (bv.x - m.x);
+        const float o1 = xv.y + (float)kOmega * iv.y * (bv.y - m.y);
         if (l0) xo[2 * t] = o0;
         if (l1) xo[2 * t + 1] = o1;
         if (dotv) {
@@ -426,27 +434,17 @@ __global__ void __launch_bounds__(kBlock) k_mg_smooth0_pair(int N2, int JK2, int
 // the neighbours instead of stored by a pass of its own (cells without an unknown hold b = 0).
 // Finest level of 160x256x256: 45 us instead of 2 x 39.
 template <typename T>
-__global__ void __launch_bounds__(kBlock) k_mg_smooth_two(Grid g, const int* __restrict__ comp,
-                                                          const int8_t* __restrict__ kind0, const T* __restrict__ e,
-                                                          const T* __restrict__ f0, const T* __restrict__ f1,
-                                                          const T* __restrict__ f2, const T* __restrict__ invd,
-                                                          const T* __restrict__ b, T* __restrict__ xo) {
+__global__ void __launch_bounds__(kBlock) k_mg_smooth_two(int N, int JK, int K, const uint8_t* __restrict__ flags,
+                                                          const T* __restrict__ e, const T* __restrict__ f0,
+                                                          const T* __restrict__ f1, const T* __restrict__ f2,
+                                                          const T* __restrict__ invd, const T* __restrict__ b,
+                                                          T* __restrict__ xo) {
     pdl_enter();
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
-         r += (long long)gridDim.x * blockDim.x) {
-        if (!(kind0 ? kind0[r] == 2 : comp[r] >= 0)) continue;
-        int i, j, k;
-        decode(g, r, i, j, k);
-        auto t = [&](long long q) { return (T)kOmega * invd[q] * b[q]; };
-        const T xr = t(r);
-        T acc = e[r] * xr;
-        if (i > 0) acc += f0[r - g.JK] * (xr - t(r - g.JK));
-        if (j > 0) acc += f1[r - g.K] * (xr - t(r - g.K));
-        if (k > 0) acc += f2[r - 1] * (xr - t(r - 1));
-        if (k + 1 < g.K) acc += f2[r] * (xr - t(r + 1));
-        if (j + 1 < g.J) acc += f1[r] * (xr - t(r + g.K));
-        if (i + 1 < g.I) acc += f0[r] * (xr - t(r + g.JK));
-        xo[r] = xr + (T)kOmega * invd[r] * (b[r] - acc);
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < N; r += gridDim.x * blockDim.x) {
+        if (!flags[r]) continue;
+        const T bv = b[r], iv = invd[r], xr = (T)kOmega * iv * bv;
+        const T acc = m_cell(r, JK, K, e, f0, f1, f2, xr, [=](int q) { return (T)kOmega * invd[q] * b[q]; });
+        xo[r] = xr + (T)kOmega * iv * (bv - acc);
     }
 }
 
@@ -485,45 +483,46 @@ __global__ void __launch_bounds__(kBlock) k_mg_smooth0_two_pair(int N2, int JK2,
 // (over-correction) below the K-cycle levels roughly halves the PCG iterations on these
 // pore-space operators (33 instead of 71 on a 96^3 porosity-0.25 field).
 // All of its neighbours' flags and corrections are L1 hits: on the finest level of 160x256x256 57
-// us instead of 25 + 39.
+// us instead of 25 + 39. A link out of the box reads a flag and a correction from the zero pads.
 template <typename T>
-__global__ void __launch_bounds__(kBlock) k_mg_smooth_corr(Grid g, Grid cg, const int* __restrict__ comp,
-                                                           const int8_t* __restrict__ kind0,
-                                                           const uint8_t* __restrict__ member,
+__global__ void __launch_bounds__(kBlock, kPassBlocks) k_mg_smooth_corr(Grid g, Grid cg, const uint8_t* __restrict__ flags,
                                                            const T* __restrict__ e, const T* __restrict__ f0,
                                                            const T* __restrict__ f1, const T* __restrict__ f2,
                                                            const T* __restrict__ invd, const T* __restrict__ b,
                                                            const T* __restrict__ x, const T* __restrict__ cx, T scale,
                                                            T* __restrict__ xo) {
     pdl_enter();
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
-         r += (long long)gridDim.x * blockDim.x) {
-        if (!(kind0 ? kind0[r] == 2 : comp[r] >= 0)) continue;
+    const int JK = (int)g.JK, K = g.K, CJK = (int)cg.JK, CK = cg.K;
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < (int)g.N; r += gridDim.x * blockDim.x) {
+        if (!flags[r]) continue;
         int i, j, k;
         decode(g, r, i, j, k);
-        const long long R = lidx(cg, i >> 1, j >> 1, k >> 1);
-        auto at = [&](long long q, long long Q) {
+        const int R = (k >> 1) + CK * ((j >> 1) + cg.J * (i >> 1));
+        auto at = [=](int q, int Q) {
             const T v = x[q], w = v + scale * cx[Q];
-            return member[q] ? w : v;
+            return flags[q] & kCellMember ? w : v;
         };
-        const T xr = at(r, R);
-        T acc = e[r] * xr;
-        if (i > 0) acc += f0[r - g.JK] * (xr - at(r - g.JK, i & 1 ? R : R - cg.JK));
-        if (j > 0) acc += f1[r - g.K] * (xr - at(r - g.K, j & 1 ? R : R - cg.K));
-        if (k > 0) acc += f2[r - 1] * (xr - at(r - 1, k & 1 ? R : R - 1));
-        if (k + 1 < g.K) acc += f2[r] * (xr - at(r + 1, k & 1 ? R + 1 : R));
-        if (j + 1 < g.J) acc += f1[r] * (xr - at(r + g.K, j & 1 ? R + cg.K : R));
-        if (i + 1 < g.I) acc += f0[r] * (xr - at(r + g.JK, i & 1 ? R + cg.JK : R));
-        xo[r] = xr + (T)kOmega * invd[r] * (b[r] - acc);
+        const T xr = at(r, R), bv = b[r], iv = invd[r];
+        const T er = e[r], l0m = f0[r - JK], l1m = f1[r - K], l2m = f2[r - 1], l2 = f2[r], l1 = f1[r], l0 = f0[r];
+        const T xim = at(r - JK, i & 1 ? R : R - CJK), xip = at(r + JK, i & 1 ? R + CJK : R);
+        const T xjm = at(r - K, j & 1 ? R : R - CK), xjp = at(r + K, j & 1 ? R + CK : R);
+        const T xkm = at(r - 1, k & 1 ? R : R - 1), xkp = at(r + 1, k & 1 ? R + 1 : R);
+        T acc = er * xr;
+        acc += l0m * (xr - xim);
+        acc += l1m * (xr - xjm);
+        acc += l2m * (xr - xkm);
+        acc += l2 * (xr - xkp);
+        acc += l1 * (xr - xjp);
+        acc += l0 * (xr - xip);
+        xo[r] = xr + (T)kOmega * iv * (bv - acc);
     }
 }
 
 // ... on pairs of cells of the finest level (FP32, K even, padded arrays): the two cells of a pair
-// and the pairs beside it over i and j each lie in one block. Neighbours outside the domain (zero
-// links) read the pair's own flags and block, the unpadded arrays end there.
-__global__ void __launch_bounds__(kBlock) k_mg_smooth0_corr_pair(Grid g, Grid cg, FastDiv div_k2,
+// and the pairs beside it over i and j each lie in one block.
+__global__ void __launch_bounds__(kBlock, kPassBlocks) k_mg_smooth0_corr_pair(Grid g, Grid cg, FastDiv div_k2,
                                                                  const int8_t* __restrict__ kind,
-                                                                 const uint8_t* __restrict__ member,
+                                                                 const uint8_t* __restrict__ flags,
                                                                  const float* __restrict__ e,
                                                                  const float* __restrict__ f0,
                                                                  const float* __restrict__ f1,
@@ -543,22 +542,20 @@ __global__ void __launch_bounds__(kBlock) k_mg_smooth0_corr_pair(Grid g, Grid cg
         const int row = (int)fdiv(div_k2, (unsigned int)t), kk = t - row * K2;
         const int i = (int)fdiv(g.div_jk, (unsigned int)r), j = row - i * g.J;
         const int R = kk + CK * ((j >> 1) + cg.J * (i >> 1));
-        auto two = [&](int q, bool in, int Q) {
+        auto two = [=](int q, int Q) {
             const float2 v = reinterpret_cast<const float2*>(x)[q];
-            const uchar2 m = reinterpret_cast<const uchar2*>(member)[in ? q : t];
-            const float c = scale * cx[in ? Q : R];
-            return make_float2(m.x ? v.x + c : v.x, m.y ? v.y + c : v.y);
+            const uchar2 m = reinterpret_cast<const uchar2*>(flags)[q];
+            const float c = scale * cx[Q];
+            return make_float2(m.x & kCellMember ? v.x + c : v.x, m.y & kCellMember ? v.y + c : v.y);
         };
-        auto one = [&](int q, bool in, int Q) {
-            const float v = x[q], c = scale * cx[in ? Q : R];
-            return member[in ? q : r] ? v + c : v;
+        auto one = [=](int q, int Q) {
+            const float v = x[q], c = scale * cx[Q];
+            return flags[q] & kCellMember ? v + c : v;
         };
-        const float2 xc = two(t, true, R);
-        const float2 m = m0_pair(t, JK2, K2, e, f0, f1, f2, xc, two(t - JK2, i > 0, i & 1 ? R : R - CJK),
-                                 two(t + JK2, i + 1 < g.I, i & 1 ? R + CJK : R),
-                                 two(t - K2, j > 0, j & 1 ? R : R - CK),
-                                 two(t + K2, j + 1 < g.J, j & 1 ? R + CK : R), one(r - 1, kk > 0, R - 1),
-                                 one(r + 2, kk + 1 < K2, R + 1));
+        const float2 xc = two(t, R);
+        const float2 m = m0_pair(t, JK2, K2, e, f0, f1, f2, xc, two(t - JK2, i & 1 ? R : R - CJK),
+                                 two(t + JK2, i & 1 ? R + CJK : R), two(t - K2, j & 1 ? R : R - CK),
+                                 two(t + K2, j & 1 ? R + CK : R), one(r - 1, R - 1), one(r + 2, R + 1));
         const float2 iv = reinterpret_cast<const float2*>(invd)[t], bv = reinterpret_cast<const float2*>(b)[t];
         if (l0) xo[r] = xc.x + (float)kOmega * iv.x * (bv.x - m.x);
         if (l1) xo[r + 1] = xc.y + (float)kOmega * iv.y * (bv.y - m.y);
@@ -569,7 +566,7 @@ __global__ void __launch_bounds__(kBlock) k_mg_smooth0_corr_pair(Grid g, Grid cg
 // forms the residuals of its block's four pairs and sums the members' in the child order of
 // k_mg_restrict. The residuals stay in registers: 54 us instead of 38 for a
 // residual pass and 28 for a gather at 160x256x256.
-__global__ void __launch_bounds__(kBlock) k_mg_restrict0_pair(Grid g, Grid cg, const uint8_t* __restrict__ member,
+__global__ void __launch_bounds__(kBlock, kPassBlocks) k_mg_restrict0_pair(Grid g, Grid cg, const uint8_t* __restrict__ flags,
                                                               const float* __restrict__ e,
                                                               const float* __restrict__ f0,
                                                               const float* __restrict__ f1,
@@ -589,52 +586,59 @@ __global__ void __launch_bounds__(kBlock) k_mg_restrict0_pair(Grid g, Grid cg, c
                 const int i = 2 * I + a, j = 2 * J + c;
                 if (i >= g.I || j >= g.J) continue;
                 const int t = K + K2 * (j + g.J * i);
-                const uchar2 m = reinterpret_cast<const uchar2*>(member)[t];
-                if (!m.x && !m.y) continue;
+                const uchar2 fl = reinterpret_cast<const uchar2*>(flags)[t];
+                const bool m0 = fl.x & kCellMember, m1 = fl.y & kCellMember;
+                if (!m0 && !m1) continue;
                 const float2 ax = m0_apply_pair(t, JK2, K2, e, f0, f1, f2, x);
                 const float2 bv = reinterpret_cast<const float2*>(b)[t];
-                if (m.x) acc += bv.x - ax.x;
-                if (m.y) acc += bv.y - ax.y;
+                if (m0) acc += bv.x - ax.x;
+                if (m1) acc += bv.y - ax.y;
             }
         cb[R] = acc;
     }
 }
 
-// b_c(R) = sum over the owned members of (b - M x)
+// Coarse right-hand side: b_c(R) = sum over the owned members of (b - M x), the children in the
+// order of their indices. Two threads per coarse cell, one for each k of its children, so that a
+// warp reads its rows without gaps; the even one adds up both's residuals.
 template <typename T>
-__device__ __forceinline__ T restrict_cell(const Grid& f, const Grid& cg, long long R, const int* __restrict__ fcomp,
-                                           const int* __restrict__ ccomp, const T* __restrict__ e,
-                                           const T* __restrict__ f0, const T* __restrict__ f1,
-                                           const T* __restrict__ f2, const T* __restrict__ fb,
-                                           const T* __restrict__ fx) {
-    int I, J, K;
-    decode(cg, R, I, J, K);
-    const int own = ccomp[R];
-    T acc = (T)0;
-    if (own >= 0) {
-        for (int a = 0; a < 2; ++a)
-            for (int b = 0; b < 2; ++b)
-                for (int c = 0; c < 2; ++c) {
-                    int i = 2 * I + a, j = 2 * J + b, k = 2 * K + c;
-                    if (i >= f.I || j >= f.J || k >= f.K) continue;
-                    long long fr = lidx(f, i, j, k);
-                    if (fcomp[fr] != own) continue;
-                    acc += fb[fr] - m_apply(f, fr, i, j, k, e, f0, f1, f2, fx);
-                }
-    }
-    return acc;
-}
-
-// coarse right-hand side: b_c(R) = sum over owned members of (b - M x)
-template <typename T>
-__global__ void k_mg_restrict(Grid f, Grid cg, const int* __restrict__ fcomp, const int* __restrict__ ccomp,
-                              const T* __restrict__ e, const T* __restrict__ f0, const T* __restrict__ f1,
-                              const T* __restrict__ f2, const T* __restrict__ fb, const T* __restrict__ fx,
-                              T* __restrict__ cb) {
+__global__ void __launch_bounds__(kBlock, kPassBlocks) k_mg_restrict(Grid f, Grid cg, const uint8_t* __restrict__ flags,
+                                                        const T* __restrict__ e, const T* __restrict__ f0,
+                                                        const T* __restrict__ f1, const T* __restrict__ f2,
+                                                        const T* __restrict__ fb, const T* __restrict__ fx,
+                                                        T* __restrict__ cb) {
     pdl_enter();
-    for (long long R = blockIdx.x * (long long)blockDim.x + threadIdx.x; R < cg.N;
-         R += (long long)gridDim.x * blockDim.x)
-        cb[R] = restrict_cell(f, cg, R, fcomp, ccomp, e, f0, f1, f2, fb, fx);
+    const int JK = (int)f.JK, K = f.K, n = 2 * (int)cg.N;
+    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < (n + 31) / 32 * 32; u += gridDim.x * blockDim.x) {
+        int I, J, KC;
+        decode(cg, min(u, n - 1) >> 1, I, J, KC);
+        const int k = 2 * KC + (u & 1);
+        int at[4], m[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int i = 2 * I + (q >> 1), j = 2 * J + (q & 1);
+            const bool in = i < f.I && j < f.J && k < K;
+            at[q] = (in ? k : 2 * KC) + K * ((in ? j : 2 * J) + f.J * (in ? i : 2 * I));
+            m[q] = flags[at[q]] & (in ? kCellMember : 0);
+        }
+        T v[4] = {(T)0, (T)0, (T)0, (T)0};
+        if (m[0] | m[1] | m[2] | m[3]) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const T xr = fx[at[q]], bv = fb[at[q]];
+                v[q] = bv - m_cell(at[q], JK, K, e, f0, f1, f2, xr, [=](int s) { return fx[s]; });
+            }
+        }
+        T acc = (T)0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const T w = __shfl_xor_sync(0xffffffffu, v[q], 1);
+            const int mw = __shfl_xor_sync(0xffffffffu, m[q], 1);
+            if (m[q]) acc += v[q];
+            if (mw) acc += w;
+        }
+        if (!(u & 1) && u < n) cb[u >> 1] = acc;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -643,24 +647,30 @@ __global__ void k_mg_restrict(Grid f, Grid cg, const int* __restrict__ fcomp, co
 // instead of one cycle. The scalars of each level's FCG live on the device (slots kKSlot0 +
 // 5 (level - 1) + {pq0, prr0, zq0, pq1, prr1}), so no host synchronisation is needed.
 
-// q = M pd and the partial dots (pd, q), (pd, rr) over member cells
-template <typename T>
-__global__ void __launch_bounds__(kBlock) k_kc_apply(Grid g, const int* __restrict__ comp, const T* __restrict__ e,
+// q = M pd and the partial dots (pd, q), (pd, rr). SECOND: the second direction,
+// pd1 = z - ((z, q0) / (pd0, q0)) pd0, is formed here, and again at the neighbours, instead of by a
+// pass of its own.
+template <typename T, bool SECOND>
+__global__ void __launch_bounds__(kBlock) k_kc_apply(int N, int JK, int K, const uint8_t* __restrict__ flags,
+                                                     const double* __restrict__ s, const T* __restrict__ e,
                                                      const T* __restrict__ f0, const T* __restrict__ f1,
-                                                     const T* __restrict__ f2, const T* __restrict__ pd,
-                                                     const T* __restrict__ rr, T* __restrict__ q,
+                                                     const T* __restrict__ f2, const T* __restrict__ z,
+                                                     const T* __restrict__ pd0, const T* __restrict__ rr,
+                                                     T* __restrict__ pd1, T* __restrict__ q,
                                                      double* __restrict__ partials) {
     pdl_enter();
+    T b = (T)0;
+    if (SECOND) b = block_scalar<T>([=] { return (T)((s[0] > 0.0) ? -s[2] / s[0] : 0.0); });
+    auto dir = [=](int v) { return SECOND ? z[v] + b * pd0[v] : pd0[v]; };
     T a0 = (T)0, a1 = (T)0;
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
-         r += (long long)gridDim.x * blockDim.x) {
-        if (comp[r] < 0) continue;
-        int i, j, k;
-        decode(g, r, i, j, k);
-        const T qv = m_apply(g, r, i, j, k, e, f0, f1, f2, pd);
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < N; r += gridDim.x * blockDim.x) {
+        if (!flags[r]) continue;
+        const T p = dir(r), rv = rr[r];
+        const T qv = m_cell(r, JK, K, e, f0, f1, f2, p, dir);
+        if (SECOND) pd1[r] = p;
         q[r] = qv;
-        a0 += pd[r] * qv;
-        a1 += pd[r] * rr[r];
+        a0 += p * qv;
+        a1 += p * rv;
     }
     double a[2] = {widen(a0), widen(a1)};
     block_sum_store<2>(a, partials);
@@ -668,39 +678,26 @@ __global__ void __launch_bounds__(kBlock) k_kc_apply(Grid g, const int* __restri
 
 // first iteration: e = alpha pd, rr -= alpha q with alpha = (pd, rr) / (pd, q)
 template <typename T>
-__global__ void k_kc_first(Grid g, const int* __restrict__ comp, const double* __restrict__ s,
+__global__ void k_kc_first(int N, const uint8_t* __restrict__ flags, const double* __restrict__ s,
                            const T* __restrict__ pd, const T* __restrict__ q, T* __restrict__ e,
                            T* __restrict__ rr) {
     pdl_enter();
     const T a = block_scalar<T>([=] { return (T)((s[0] > 0.0) ? s[1] / s[0] : 0.0); });
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
-         r += (long long)gridDim.x * blockDim.x) {
-        if (comp[r] < 0) continue;
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < N; r += gridDim.x * blockDim.x) {
+        if (!flags[r]) continue;
         e[r] = a * pd[r];
         rr[r] -= a * q[r];
     }
 }
 
-// second direction: pd1 = z - ((z, q0) / (pd0, q0)) pd0
-template <typename T>
-__global__ void k_kc_dir(Grid g, const int* __restrict__ comp, const double* __restrict__ s,
-                         const T* __restrict__ z, const T* __restrict__ pd0, T* __restrict__ pd1) {
-    pdl_enter();
-    const T b = block_scalar<T>([=] { return (T)((s[0] > 0.0) ? -s[2] / s[0] : 0.0); });
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
-         r += (long long)gridDim.x * blockDim.x)
-        if (comp[r] >= 0) pd1[r] = z[r] + b * pd0[r];
-}
-
 // second iteration: e += alpha1 pd1, alpha1 = (pd1, rr) / (pd1, q1)
 template <typename T>
-__global__ void k_kc_second(Grid g, const int* __restrict__ comp, const double* __restrict__ s,
+__global__ void k_kc_second(int N, const uint8_t* __restrict__ flags, const double* __restrict__ s,
                             const T* __restrict__ pd1, T* __restrict__ e) {
     pdl_enter();
     const T a = block_scalar<T>([=] { return (T)((s[3] > 0.0) ? s[4] / s[3] : 0.0); });
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
-         r += (long long)gridDim.x * blockDim.x)
-        if (comp[r] >= 0) e[r] += a * pd1[r];
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < N; r += gridDim.x * blockDim.x)
+        if (flags[r]) e[r] += a * pd1[r];
 }
 
 // coarsest level: a fixed number of damped Jacobi sweeps from zero by one CTA
@@ -939,19 +936,35 @@ void mg_graphs_clear(ls_ctx* c) {
     c->mg_graphs.clear();
 }
 
+static ls_status level_alloc(ls_ctx* c, const Grid& g, size_t esize, void** out) {
+    const size_t pad = level_pad(g), bytes = esize * ((size_t)g.N + 2 * pad);
+    void* base = nullptr;
+    LS_TRY(walloc(c, &base, bytes));
+    *out = (char*)base + esize * pad;
+    LS_CUDA(c, cudaMemsetAsync(base, 0, bytes, c->stream));
+    return LS_OK;
+}
+
+static void level_free(ls_ctx* c, const Grid& g, size_t esize, void** p) {
+    if (!*p) return;
+    const size_t pad = level_pad(g);
+    void* base = (char*)*p - esize * pad;
+    dfree(c, &base, esize * ((size_t)g.N + 2 * pad));
+    *p = nullptr;
+}
+
 void mg_free(ls_ctx* c) {
     mg_graphs_clear(c);
     for (size_t m = 0; m < c->mg.size(); ++m) {
         auto& lv = c->mg[m];
-        const size_t n = (size_t)lv.g.N, es = (size_t)lv.esize;
-        dfree_t(c, &lv.comp, n);
-        dfree_t(c, &lv.member, n);
+        dfree_t(c, &lv.comp, (size_t)lv.g.N);
+        level_free(c, lv.g, 1, (void**)&lv.flags);
         void** lp[] = {&lv.e, &lv.face[0], &lv.face[1], &lv.face[2], &lv.invd, &lv.x, &lv.b, &lv.t};
-        for (void** q : lp) dfree(c, q, es * n);
-        for (void*& q : lv.kv) dfree(c, &q, es * n);
+        for (void** q : lp) level_free(c, lv.g, (size_t)lv.esize, q);
+        for (void*& q : lv.kv) level_free(c, lv.g, (size_t)lv.esize, &q);
     }
     c->mg.clear();
-    dfree_t(c, &c->mg0_member, (size_t)c->g.N);
+    level_free(c, c->g, 1, (void**)&c->mg0_flags);
     l0_free(c, 10, &c->mg0_p);
     l0_free(c, 11, &c->mg0_t);
     c->mg_is64 = -1;
@@ -1069,33 +1082,27 @@ static ls_status mg_alloc(ls_ctx* c) {
     c->mg_cluster = fuse_cluster<T>();
     if (!c->comp) LS_TRY(walloc_t(c, &c->comp, (size_t)c->g.N));
     if (!c->cc_flag) LS_TRY(dalloc_t(c, &c->cc_flag, (size_t)4));
-    LS_TRY(walloc_t(c, &c->mg0_member, (size_t)c->g.N));
+    LS_TRY(level_alloc(c, c->g, 1, (void**)&c->mg0_flags));
     if (!is64 && c->g.K % 2 == 0) LS_TRY(l0_alloc(c, 10, sizeof(T), &c->mg0_p));
     LS_TRY(l0_alloc(c, 11, sizeof(T), &c->mg0_t));
     Grid g = c->g;
     g.NP = g.N;
     while ((c->mg.empty() || g.N > kCoarsestCells) && (g.I > 1 || g.J > 1 || g.K > 1)) {
         Grid cg = coarse_of(g);
-        ls_ctx::MGLevel lv = {};
+        c->mg.push_back({});
+        ls_ctx::MGLevel& lv = c->mg.back();
         lv.g = cg;
         lv.esize = (int)sizeof(T);
         LS_TRY(walloc_t(c, &lv.comp, (size_t)cg.N));
-        LS_TRY(walloc_t(c, &lv.member, (size_t)cg.N));
+        LS_TRY(level_alloc(c, cg, 1, (void**)&lv.flags));
         void** arrs[] = {&lv.e, &lv.face[0], &lv.face[1], &lv.face[2], &lv.invd, &lv.x, &lv.b, &lv.t};
-        for (void** q : arrs) {
-            LS_TRY(walloc(c, q, sizeof(T) * (size_t)cg.N));
-            LS_CUDA(c, cudaMemsetAsync(*q, 0, sizeof(T) * (size_t)cg.N, c->stream));
-        }
-        c->mg.push_back(lv);
+        for (void** q : arrs) LS_TRY(level_alloc(c, cg, sizeof(T), q));
         g = cg;
     }
     // K-cycle vectors on the levels 1..kKLevels that have a coarser level below them
     for (size_t m = 1; m <= (size_t)kKLevels && m < c->mg.size(); ++m) {
         auto& lv = c->mg[m - 1];
-        for (void*& q : lv.kv) {
-            LS_TRY(walloc(c, &q, sizeof(T) * (size_t)lv.g.N));
-            LS_CUDA(c, cudaMemsetAsync(q, 0, sizeof(T) * (size_t)lv.g.N, c->stream));
-        }
+        for (void*& q : lv.kv) LS_TRY(level_alloc(c, lv.g, sizeof(T), &q));
     }
     c->mg_is64 = is64;
     return LS_OK;
@@ -1131,8 +1138,8 @@ ls_status mg_setup(ls_ctx* c) {
         auto& cl = c->mg[l];
         const int cgd = grid_for(c, cl.g.N);
         LS_LAUNCH(c, k_mg_dom, cgd, kBlock, 0, fg, cl.g, fcomp, cl.comp);
-        LS_LAUNCH(c, k_mg_member, grid_for(c, fg.N), kBlock, 0, fg, cl.g, fcomp, (const int*)cl.comp,
-                  l == 0 ? c->mg0_member : c->mg[l - 1].member);
+        LS_LAUNCH(c, k_mg_flags, grid_for(c, fg.N), kBlock, 0, fg, cl.g, fcomp, (const int*)cl.comp,
+                  l == 0 ? c->mg0_flags : c->mg[l - 1].flags);
         LS_LAUNCH(c, k_mg_coarse_op<T>, cgd, kBlock, 0, fg, cl.g, fcomp, (const int*)cl.comp, fe, ff[0], ff[1],
                   ff[2], (T*)cl.e, (T*)cl.face[0], (T*)cl.face[1], (T*)cl.face[2]);
         LS_LAUNCH(c, k_level_invd<T>, cgd, kBlock, 0, cl.g, (const int*)cl.comp, (const int8_t*)nullptr,
@@ -1180,18 +1187,19 @@ ls_status mg_apply(ls_ctx* c, const T* r, T* z, const T* dotv2, int* nblocks_out
     struct Lv {
         Grid g;
         const int* comp;
+        const uint8_t* flags;
         const T *e, *f0, *f1, *f2, *invd;
         T *x, *b, *t;
-        T* kv[7];
+        T* kv[6];
     };
     std::vector<Lv> lv(L + 1);
-    lv[0] = {c->g, c->comp, (const T*)c->ie, (const T*)c->iface[0], (const T*)c->iface[1], (const T*)c->iface[2],
+    lv[0] = {c->g, c->comp, c->mg0_flags, (const T*)c->ie, (const T*)c->iface[0], (const T*)c->iface[1], (const T*)c->iface[2],
              (const T*)c->iinvd, z, nullptr, (T*)c->mg0_t, {}};
     for (size_t l = 0; l < L; ++l) {
         auto& m = c->mg[l];
-        lv[l + 1] = {m.g, m.comp, (const T*)m.e, (const T*)m.face[0], (const T*)m.face[1], (const T*)m.face[2],
+        lv[l + 1] = {m.g, m.comp, m.flags, (const T*)m.e, (const T*)m.face[0], (const T*)m.face[1], (const T*)m.face[2],
                      (const T*)m.invd, (T*)m.x, (T*)m.b, (T*)m.t, {}};
-        for (int q = 0; q < 7; ++q) lv[l + 1].kv[q] = (T*)m.kv[q];
+        for (int q = 0; q < 6; ++q) lv[l + 1].kv[q] = (T*)m.kv[q];
     }
     // one damped-Jacobi sweep on level l (paired finest-level kernel for FP32 and even K)
     const bool pair0 = std::is_same<T, float>::value && (c->g.K % 2 == 0);
@@ -1210,36 +1218,34 @@ ls_status mg_apply(ls_ctx* c, const T* r, T* z, const T* dotv2, int* nblocks_out
             return LS_OK;
         }
         const int gd = grid_for(c, a.g.N);
-        LS_LAUNCH_PDL(c, k_mg_smooth<T>, gd, kBlock, 0, a.g, a.comp,
-                  l == 0 ? (const int8_t*)c->pkind : (const int8_t*)nullptr, a.e, a.f0, a.f1, a.f2, a.invd, b, x,
-                  xo, dv, dv2, partials);
+        LS_LAUNCH_PDL(c, k_mg_smooth<T>, gd, kBlock, 0, (int)a.g.N, (int)a.g.JK, a.g.K, a.flags, a.e, a.f0, a.f1, a.f2,
+                  a.invd, b, x, xo, dv, dv2, partials);
         if (nb) *nb = gd;
         return LS_OK;
     };
     // cycle(l, b, out): out = B_l b; with dv non-null the final sweep leaves the partial dots
     // (dv, out), (dv2, out) and their block count in *nb. Level l's x and t are its scratch.
     std::function<ls_status(size_t, const T*, T*, const T*, const T*, int*)> cycle;
-    // kfcg(m): two FCG iterations on level m for M_m e = b_m (m's b), result in kv[6]
+    // kfcg(m): two FCG iterations on level m for M_m e = b_m (m's b, left as the residual of the
+    // first), result in kv[5]
     auto kfcg = [&](size_t m) -> ls_status {
         Lv& a = lv[m];
-        T *rr = a.kv[0], *za = a.kv[1], *zb = a.kv[2], *pd = a.kv[3], *q0 = a.kv[4], *q1 = a.kv[5], *e = a.kv[6];
+        T *rr = a.b, *za = a.kv[0], *zb = a.kv[1], *pd = a.kv[2], *q0 = a.kv[3], *q1 = a.kv[4], *e = a.kv[5];
         const int slot = kKSlot0 + 5 * ((int)m - 1);
         const double* s = c->scal + slot;
-        const int gd = grid_for(c, a.g.N);
-        LS_CUDA(c, cudaMemcpyAsync(rr, a.b, sizeof(T) * (size_t)a.g.N, cudaMemcpyDeviceToDevice, c->stream));
+        const int gd = grid_for(c, a.g.N), N = (int)a.g.N, JK = (int)a.g.JK, K = a.g.K;
         LS_TRY(cycle(m, (const T*)rr, za, nullptr, nullptr, nullptr));
-        LS_LAUNCH_PDL(c, k_kc_apply<T>, gd, kBlock, 0, a.g, a.comp, a.e, a.f0, a.f1, a.f2, (const T*)za,
-                  (const T*)rr, q0, c->partials);
+        LS_LAUNCH_PDL(c, (k_kc_apply<T, false>), gd, kBlock, 0, N, JK, K, a.flags, s, a.e, a.f0, a.f1, a.f2,
+                  (const T*)nullptr, (const T*)za, (const T*)rr, (T*)nullptr, q0, c->partials);
         LS_TRY(finalize_sum(c, gd, 2, slot));  // (za, q0), (za, rr)
-        LS_LAUNCH_PDL(c, k_kc_first<T>, gd, kBlock, 0, a.g, a.comp, s, (const T*)za, (const T*)q0, e, rr);
+        LS_LAUNCH_PDL(c, k_kc_first<T>, gd, kBlock, 0, N, a.flags, s, (const T*)za, (const T*)q0, e, rr);
         int nb = 0;
         LS_TRY(cycle(m, (const T*)rr, zb, (const T*)q0, nullptr, &nb));
         LS_TRY(finalize_sum(c, nb, 2, slot + 2));  // (zb, q0)
-        LS_LAUNCH_PDL(c, k_kc_dir<T>, gd, kBlock, 0, a.g, a.comp, s, (const T*)zb, (const T*)za, pd);
-        LS_LAUNCH_PDL(c, k_kc_apply<T>, gd, kBlock, 0, a.g, a.comp, a.e, a.f0, a.f1, a.f2, (const T*)pd,
-                  (const T*)rr, q1, c->partials);
+        LS_LAUNCH_PDL(c, (k_kc_apply<T, true>), gd, kBlock, 0, N, JK, K, a.flags, s, a.e, a.f0, a.f1, a.f2,
+                  (const T*)zb, (const T*)za, (const T*)rr, pd, q1, c->partials);
         LS_TRY(finalize_sum(c, gd, 2, slot + 3));  // (pd, q1), (pd, rr)
-        LS_LAUNCH_PDL(c, k_kc_second<T>, gd, kBlock, 0, a.g, a.comp, s, (const T*)pd, e);
+        LS_LAUNCH_PDL(c, k_kc_second<T>, gd, kBlock, 0, N, a.flags, s, (const T*)pd, e);
         return LS_OK;
     };
     // the levels from `fuse` down run as one launch each time they are visited (k_mg_fused)
@@ -1265,7 +1271,7 @@ ls_status mg_apply(ls_ctx* c, const T* r, T* z, const T* dotv2, int* nblocks_out
                 f.invd = a.invd;
                 f.x = a.x;
                 f.b = a.b;
-                f.ev = a.kv[6];
+                f.ev = a.kv[5];
                 if (l + q <= (size_t)kKLevels && l + q < L) fa.nk = q + 1;
             }
             if (fuse_plan(fa, c->mg_cluster, &fuse_smem)) fuse = l;
@@ -1281,31 +1287,30 @@ ls_status mg_apply(ls_ctx* c, const T* r, T* z, const T* dotv2, int* nblocks_out
         Lv& cl = lv[l + 1];
         const int gd = grid_for(c, a.g.N);
         const int N2 = (int)(a.g.N / 2), JK2 = (int)(a.g.JK / 2), K2 = a.g.K / 2;
-        const int8_t* kind0 = l == 0 ? (const int8_t*)c->pkind : (const int8_t*)nullptr;
-        const uint8_t* member = l == 0 ? c->mg0_member : c->mg[l - 1].member;
         if (l == 0 && pair0) {
-            LS_LAUNCH_PDL(c, k_mg_smooth0_two_pair, grid_for(c, N2), kBlock, 0, N2, JK2, K2, kind0, (const float*)a.e,
+            LS_LAUNCH_PDL(c, k_mg_smooth0_two_pair, grid_for(c, N2), kBlock, 0, N2, JK2, K2,
+                      (const int8_t*)c->pkind, (const float*)a.e,
                       (const float*)a.f0, (const float*)a.f1, (const float*)a.f2, (const float*)a.invd,
                       (const float*)b, (float*)a.x);
-            LS_LAUNCH_PDL(c, k_mg_restrict0_pair, grid_for(c, cl.g.N), kBlock, 0, a.g, cl.g, member, (const float*)a.e,
+            LS_LAUNCH_PDL(c, k_mg_restrict0_pair, pass_grid(c, cl.g.N), kBlock, 0, a.g, cl.g, a.flags, (const float*)a.e,
                       (const float*)a.f0, (const float*)a.f1, (const float*)a.f2, (const float*)b, (const float*)a.x,
                       (float*)cl.b);
         } else {
-            LS_LAUNCH_PDL(c, k_mg_smooth_two<T>, gd, kBlock, 0, a.g, a.comp, kind0, a.e, a.f0, a.f1, a.f2, a.invd, b,
-                      a.x);
-            LS_LAUNCH_PDL(c, k_mg_restrict<T>, grid_for(c, cl.g.N), kBlock, 0, a.g, cl.g, a.comp, cl.comp, a.e, a.f0,
-                      a.f1, a.f2, b, (const T*)a.x, cl.b);
+            LS_LAUNCH_PDL(c, k_mg_smooth_two<T>, gd, kBlock, 0, (int)a.g.N, (int)a.g.JK, a.g.K, a.flags, a.e, a.f0, a.f1,
+                      a.f2, a.invd, b, a.x);
+            LS_LAUNCH_PDL(c, k_mg_restrict<T>, pass_grid(c, 2 * cl.g.N), kBlock, 0, a.g, cl.g, a.flags, a.e, a.f0, a.f1,
+                      a.f2, b, (const T*)a.x, cl.b);
         }
         const T* corr;
         T scale;
         if (l + 1 >= fuse) {
             LS_TRY(fuse_launch<T>(c, fa, fuse_smem));
             const bool kc = l + 1 <= (size_t)kKLevels && l + 1 < L;
-            corr = kc ? cl.kv[6] : cl.x;
+            corr = kc ? cl.kv[5] : cl.x;
             scale = kc ? (T)1 : (T)kProlongScale;
         } else if (l + 1 <= (size_t)kKLevels && l + 1 < L) {
             LS_TRY(kfcg(l + 1));
-            corr = cl.kv[6];
+            corr = cl.kv[5];
             scale = (T)1;  // the FCG steps carry the optimal scaling
         } else if (learned && l + 1 == (size_t)kLearnedLevel) {
             LS_TRY(lpc_solve(c, cl.g, cl.comp, (const float*)cl.b, (float*)cl.x));
@@ -1317,13 +1322,13 @@ ls_status mg_apply(ls_ctx* c, const T* r, T* z, const T* dotv2, int* nblocks_out
             scale = (T)kProlongScale;
         }
         if (l == 0 && pair0)
-            LS_LAUNCH_PDL(c, k_mg_smooth0_corr_pair, grid_for(c, N2), kBlock, 0, a.g, cl.g, make_fastdiv((unsigned)K2),
-                      kind0, member, (const float*)a.e, (const float*)a.f0, (const float*)a.f1, (const float*)a.f2,
+            LS_LAUNCH_PDL(c, k_mg_smooth0_corr_pair, pass_grid(c, N2), kBlock, 0, a.g, cl.g, make_fastdiv((unsigned)K2),
+                      (const int8_t*)c->pkind, a.flags, (const float*)a.e, (const float*)a.f0, (const float*)a.f1, (const float*)a.f2,
                       (const float*)a.invd, (const float*)b, (const float*)a.x, (const float*)corr, (float)scale,
                       (float*)a.t);
         else
-            LS_LAUNCH_PDL(c, k_mg_smooth_corr<T>, gd, kBlock, 0, a.g, cl.g, a.comp, kind0, member, a.e, a.f0, a.f1, a.f2,
-                      a.invd, b, (const T*)a.x, corr, scale, a.t);
+            LS_LAUNCH_PDL(c, k_mg_smooth_corr<T>, pass_grid(c, a.g.N), kBlock, 0, a.g, cl.g, a.flags, a.e, a.f0, a.f1, a.f2, a.invd, b,
+                      (const T*)a.x, corr, scale, a.t);
         return smooth(l, b, (const T*)a.t, out, dv, dv2, nb);
     };
     return cycle(0, r, z, r, dotv2, nblocks_out);
