@@ -76,26 +76,6 @@ __device__ __forceinline__ T m_apply(const Grid& g, long long r, int i, int j, i
     return acc;
 }
 
-// The same on arrays with zero pads of a plane on both sides (level_pad): a link out of the box is
-// a stored 0 and its other end is read from the pad or from the next row, so the index needs no
-// decoding and all reads are under way together. With the bounds as branches each face waited
-// for the one before: on the 4.0M cells of the first coarse level of 338x338x283 a sweep took 60
-// us, now 31, and the sweep with the correction 104, now 36. at(q) is x of cell q.
-template <typename T, typename F>
-__device__ __forceinline__ T m_cell(int r, int JK, int K, const T* __restrict__ e, const T* __restrict__ f0,
-                                    const T* __restrict__ f1, const T* __restrict__ f2, T xr, F at) {
-    const T er = e[r], l0m = f0[r - JK], l1m = f1[r - K], l2m = f2[r - 1], l2 = f2[r], l1 = f1[r], l0 = f0[r];
-    const T xim = at(r - JK), xjm = at(r - K), xkm = at(r - 1), xkp = at(r + 1), xjp = at(r + K), xip = at(r + JK);
-    T acc = er * xr;
-    acc += l0m * (xr - xim);
-    acc += l1m * (xr - xjm);
-    acc += l2m * (xr - xkm);
-    acc += l2 * (xr - xkp);
-    acc += l1 * (xr - xjp);
-    acc += l0 * (xr - xip);
-    return acc;
-}
-
 // Resident blocks per SM of the passes that hold more than 32 registers and sum nothing, whose
 // grid is that many blocks per SM: with grid_for's 8 a second, partly filled wave followed (the
 // finest sweep with the correction at 338x338x283: 186 us, now 163). 4, 5 or 6: the step with
@@ -1083,7 +1063,7 @@ static ls_status mg_alloc(ls_ctx* c) {
     if (!c->comp) LS_TRY(walloc_t(c, &c->comp, (size_t)c->g.N));
     if (!c->cc_flag) LS_TRY(dalloc_t(c, &c->cc_flag, (size_t)4));
     LS_TRY(level_alloc(c, c->g, 1, (void**)&c->mg0_flags));
-    if (!is64 && c->g.K % 2 == 0) LS_TRY(l0_alloc(c, 10, sizeof(T), &c->mg0_p));
+    LS_TRY(l0_alloc(c, 10, sizeof(T), &c->mg0_p));
     LS_TRY(l0_alloc(c, 11, sizeof(T), &c->mg0_t));
     Grid g = c->g;
     g.NP = g.N;
@@ -1164,7 +1144,7 @@ ls_status mg_setup(ls_ctx* c) {
 // Zero every level vector (the smoother and the PCG skip non-member cells, which must hold 0).
 template <typename T>
 ls_status mg_clear(ls_ctx* c) {
-    if (c->mg0_p) LS_CUDA(c, cudaMemsetAsync(c->mg0_p, 0, sizeof(T) * (size_t)c->g.N, c->stream));
+    LS_CUDA(c, cudaMemsetAsync(c->mg0_p, 0, sizeof(T) * (size_t)c->g.N, c->stream));
     LS_CUDA(c, cudaMemsetAsync(c->mg0_t, 0, sizeof(T) * (size_t)c->g.N, c->stream));
     for (auto& lv : c->mg) {
         const size_t b = sizeof(T) * (size_t)lv.g.N;

@@ -607,45 +607,31 @@ __global__ void k_press_accumulate(Grid g, const int8_t* __restrict__ kind,
 // ---------------------------------------------------------------------------
 // inner PCG on sigma*M (excess + Laplacian form)
 
-template <typename T>
-__device__ __forceinline__ T inner_apply_row(const Grid& g, long long r, int i, int j, int k,
-                                             const T* __restrict__ v, const T* __restrict__ e,
-                                             const T* __restrict__ w0, const T* __restrict__ w1,
-                                             const T* __restrict__ w2) {
-    const T vr = v[r];
-    T acc = e[r] * vr;
-    if (i > 0) acc += w0[r - g.JK] * (vr - v[r - g.JK]);
-    if (j > 0) acc += w1[r - g.K] * (vr - v[r - g.K]);
-    if (k > 0) acc += w2[r - 1] * (vr - v[r - 1]);
-    if (k + 1 < g.K) acc += w2[r] * (vr - v[r + 1]);
-    if (j + 1 < g.J) acc += w1[r] * (vr - v[r + g.K]);
-    if (i + 1 < g.I) acc += w0[r] * (vr - v[r + g.JK]);
-    return acc;
-}
-
 // The inner vectors are zero on voxels that are not inner unknowns (kind != 2) and no
 // kernel writes them there (the buffers are cleared when allocated), so the inner PCG
 // kernels skip those voxels: ~3/4 of the box in a porosity-0.25 medium.
 
-// q = M p, partial (p, q)
-template <typename T>
-__global__ void __launch_bounds__(kBlock) k_cg_apply(Grid g, const int8_t* __restrict__ kind,
-                                                     const T* __restrict__ p,
-                                                     const T* __restrict__ e,
-                                                     const T* __restrict__ w0,
-                                                     const T* __restrict__ w1,
-                                                     const T* __restrict__ w2, T* __restrict__ q,
-                                                     double* __restrict__ partials) {
+// q = M p, partial (p, q). DIR (flexible CG): the direction z + beta p is formed here, and
+// again at the neighbours, and stored in po, instead of by k_cg_dir's pass.
+template <typename T, bool DIR>
+__global__ void __launch_bounds__(kBlock) k_cg_apply(int N, int JK, int K, const int8_t* __restrict__ kind,
+                                                     const double* __restrict__ scal, const T* __restrict__ z,
+                                                     const T* __restrict__ p, const T* __restrict__ e,
+                                                     const T* __restrict__ w0, const T* __restrict__ w1,
+                                                     const T* __restrict__ w2, T* __restrict__ po,
+                                                     T* __restrict__ q, double* __restrict__ partials) {
     pdl_enter();
+    T beta = (T)0;
+    if (DIR) beta = block_scalar<T>([=] { return (T)((scal[SP_PQ] > 0.0) ? -scal[SP_ZQ] / scal[SP_PQ] : 0.0); });
+    auto dir = [=](int v) { return DIR ? z[v] + beta * p[v] : p[v]; };
     T a = (T)0;  // per-thread partial in the inner precision
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
-         r += (long long)gridDim.x * blockDim.x) {
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < N; r += gridDim.x * blockDim.x) {
         if (kind[r] != 2) continue;
-        int i, j, k;
-        decode(g, r, i, j, k);
-        T qv = inner_apply_row(g, r, i, j, k, p, e, w0, w1, w2);
+        const T pv = dir(r);
+        const T qv = m_cell(r, JK, K, e, w0, w1, w2, pv, dir);
+        if (DIR) po[r] = pv;
         q[r] = qv;
-        a += p[r] * qv;
+        a += pv * qv;
     }
     double acc[1] = {widen(a)};
     block_sum_store<1>(acc, partials);
@@ -674,8 +660,8 @@ __global__ void __launch_bounds__(kBlock) k_cg_apply0_pair(int N2, int JK2, int 
 
 // The direction and the product of one CG iteration in one pass (flexible CG, FP32, K even):
 // po = z + beta p of the unknowns, formed again at the neighbours, and q = M po with the partial
-// (po, q). z and p are read and po is written once, without
-// k_cg_dir's pass, bound by DRAM: 52 us instead of 28 + 36 at 160x256x256.
+// (po, q). z and p are read and po is written once, bound by DRAM, without a pass that forms p: 52
+// us instead of 28 + 36 at 160x256x256.
 __global__ void __launch_bounds__(kBlock) k_cg_dir_apply0_pair(int N2, int JK2, int K2,
                                                                const int8_t* __restrict__ kind,
                                                                const double* __restrict__ scal,
@@ -712,13 +698,13 @@ __global__ void __launch_bounds__(kBlock) k_cg_dir_apply0_pair(int N2, int JK2, 
 
 // x += a p, r -= a q with a = (r,z)/(p,q) (0 when (p,q) <= 0)
 template <typename T>
-__global__ void k_cg_update(Grid g, const int8_t* __restrict__ kind, const double* __restrict__ scal,
+__global__ void k_cg_update(Grid g, const int8_t* __restrict__ kind, const double* __restrict__ scal, int rz,
                             const T* __restrict__ p, const T* __restrict__ q, T* __restrict__ x,
                             T* __restrict__ r_) {
     pdl_enter();
     const T a = block_scalar<T>([=] {
         const double pq = scal[SP_PQ];
-        return (T)((pq > 0.0) ? scal[SP_RZ] / pq : 0.0);
+        return (T)((pq > 0.0) ? scal[rz] / pq : 0.0);
     });
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
          r += (long long)gridDim.x * blockDim.x) {
@@ -746,15 +732,13 @@ __global__ void __launch_bounds__(kBlock) k_cg_jacobi(Grid g, const T* __restric
     block_sum_store<1>(acc, partials);
 }
 
-// p = z + b p with b = (r,z)_new / (r,z)_old (fixed preconditioner) or, for the flexible CG
-// that the K-cycle needs, b = -(z_new, q) / (p, q) (Notay's FCG(1))
+// p = z + b p with b = (r,z)_new / (r,z)_old (fixed preconditioner; the flexible CG that the
+// K-cycle needs, Notay's FCG(1) with b = -(z_new, q) / (p, q), forms p in its product)
 template <typename T>
 __global__ void k_cg_dir(Grid g, const int8_t* __restrict__ kind, const double* __restrict__ scal,
-                         const T* __restrict__ z, T* __restrict__ p, int flexible) {
+                         const T* __restrict__ z, T* __restrict__ p) {
     pdl_enter();
-    const T beta = block_scalar<T>([=] {
-        return (T)(flexible ? ((scal[SP_PQ] > 0.0) ? -scal[SP_ZQ] / scal[SP_PQ] : 0.0) : scal[SP_RZN] / scal[SP_RZ]);
-    });
+    const T beta = block_scalar<T>([=] { return (T)(scal[SP_RZN] / scal[SP_RZ]); });
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
          r += (long long)gridDim.x * blockDim.x)
         if (kind[r] == 2) p[r] = z[r] + beta * p[r];
@@ -848,28 +832,33 @@ static ls_status inner_pcg(ls_ctx* c, bool use_mg, double tol, int max_it, int* 
     for (int it = 0; it < max_it; ++it) {
         {
             Timed tm(c, LS_T_CG_APPLY);
-            if (pair && use_mg && it > 0) {
+            const bool dir = use_mg && it > 0;
+            if (pair && dir) {
                 LS_LAUNCH_PDL(c, k_cg_dir_apply0_pair, pgrid, kBlock, 0, (int)(g.N / 2), (int)(g.JK / 2), g.K / 2,
                           (const int8_t*)c->pkind, (const double*)c->scal, (const float*)z, (const float*)p,
                           (float*)p_other, (const float*)e, (const float*)w0, (const float*)w1, (const float*)w2,
                           (float*)q, c->partials);
-                std::swap(p, p_other);
-                if (c->timing) c->timer_bytes[LS_T_CG_APPLY] += (double)g.N * 2.0 * sizeof(T);  // z in, p out
             } else if (pair) {
                 LS_LAUNCH_PDL(c, k_cg_apply0_pair, pgrid, kBlock, 0, (int)(g.N / 2), (int)(g.JK / 2), g.K / 2,
                           (const int8_t*)c->pkind, (const float*)p, (const float*)e, (const float*)w0,
                           (const float*)w1, (const float*)w2, (float*)q, c->partials);
+            } else if (dir) {
+                LS_LAUNCH_PDL(c, (k_cg_apply<T, true>), grid, kBlock, 0, (int)g.N, (int)g.JK, g.K,
+                          (const int8_t*)c->pkind, (const double*)c->scal, (const T*)z, (const T*)p, e, w0, w1, w2,
+                          p_other, q, c->partials);
             } else {
-                LS_LAUNCH_PDL(c, k_cg_apply<T>, grid, kBlock, 0, g, (const int8_t*)c->pkind, (const T*)p, e, w0, w1,
-                          w2, q, c->partials);
+                LS_LAUNCH_PDL(c, (k_cg_apply<T, false>), grid, kBlock, 0, (int)g.N, (int)g.JK, g.K,
+                          (const int8_t*)c->pkind, (const double*)c->scal, (const T*)nullptr, (const T*)p, e, w0, w1,
+                          w2, (T*)nullptr, q, c->partials);
             }
-            // p in, excess and three own face links, q out
-            if (c->timing) c->timer_bytes[LS_T_CG_APPLY] += (double)g.N * 6.0 * sizeof(T);
+            if (dir) std::swap(p, p_other);
+            // p in, excess and three own face links, q out; z in and p out with the direction
+            if (c->timing) c->timer_bytes[LS_T_CG_APPLY] += (double)g.N * (dir ? 8.0 : 6.0) * sizeof(T);
         }
-        if (it > 0) LS_LAUNCH_PDL(c, k_set_scalar, 1, 1, 0, c->scal, SP_RZ, SP_RZN);
         LS_TRY(finalize_sum(c, pair ? pgrid : grid, 1, SP_PQ));
+        // the flexible CG's direction does not need the last (r, z), which stays in SP_RZN
         LS_LAUNCH_PDL(c, k_cg_update<T>, grid, kBlock, 0, g, (const int8_t*)c->pkind, (const double*)c->scal,
-                  (const T*)p, (const T*)q, x, r);
+                  use_mg && it > 0 ? (int)SP_RZN : (int)SP_RZ, (const T*)p, (const T*)q, x, r);
         LS_TRY(precondition(SP_RZN, (const T*)q));
         *its = it + 1;
         double sc[3];
@@ -898,9 +887,11 @@ static ls_status inner_pcg(ls_ctx* c, bool use_mg, double tol, int max_it, int* 
         }
         if (rz != rz) return set_error(c, LS_NONFINITE, "pressure: NaN in inner PCG");
         if (rz <= target || !(pq > 0.0) || rz < 0.0) break;
-        if (!(pair && use_mg))
+        if (!use_mg) {
             LS_LAUNCH_PDL(c, k_cg_dir<T>, grid, kBlock, 0, g, (const int8_t*)c->pkind, (const double*)c->scal,
-                      (const T*)z, p, use_mg ? 1 : 0);
+                      (const T*)z, p);
+            LS_LAUNCH_PDL(c, k_set_scalar, 1, 1, 0, c->scal, SP_RZ, SP_RZN);
+        }
     }
     *rel_out = sqrt(std::max(rz, 0.0) / rz0);
     return LS_OK;
