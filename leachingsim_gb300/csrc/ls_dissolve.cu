@@ -313,19 +313,17 @@ __global__ void __launch_bounds__(kBlock) k_dz_grow(Grid g, int* __restrict__ M,
 }
 
 // S as a list (any order), its members marked 0
-__global__ void __launch_bounds__(kBlock) k_dz_collect(Grid g, int* __restrict__ M, int* __restrict__ list,
+__global__ void __launch_bounds__(kBlock) k_dz_collect(Grid g, int* __restrict__ M, int per, int* __restrict__ list,
                                                        unsigned int* __restrict__ count) {
-    // block-uniform trip count (block_append is called by every thread of the block)
-    for (long long b0 = (long long)blockIdx.x * blockDim.x; b0 < g.N; b0 += (long long)gridDim.x * blockDim.x) {
-        const long long r = b0 + threadIdx.x;
-        bool in = false;
-        if (r < g.N) {
+    scan_blocks(g.N, per, [=](long long v0) {
+        const unsigned int in = ballot_words(v0, per, g.N, [=](int r) {
             const int m = M[r];
-            in = (m == 0 || m == -3 || m == -4);
-            if (in) M[r] = 0;
-        }
-        block_append(in, (int)r, list, count);
-    }
+            const bool is = (m == 0 || m == -3 || m == -4);
+            if (is) M[r] = 0;
+            return is;
+        });
+        append_words(in, v0, per, list, count);
+    });
 }
 
 // wavefront levels of the listed voxels: histogram, then the list sorted by level
@@ -578,7 +576,8 @@ static ls_status dissolve_t(ls_ctx* c, double dt, int* leached_out, ls_substep_i
             LS_TRY(dalloc(c, &c->dz_save_label, (size_t)n_active * c->label_bytes));
             c->dz_sel_cap = n_active;
         }
-        LS_LAUNCH(c, k_dz_collect, grid, kBlock, 0, g, M, c->dz_sel, c->wcount);
+        const int per = scan_words(c->num_sms, g.N);
+        LS_LAUNCH(c, k_dz_collect, scan_grid(c->num_sms, g.N, per), kBlock, 0, g, M, per, c->dz_sel, c->wcount);
         unsigned int nsel_u = 0;
         LS_TRY(read_device(c, c->wcount, &nsel_u, sizeof(unsigned int)));
         const int nsel = (int)nsel_u;

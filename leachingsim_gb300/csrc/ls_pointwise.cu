@@ -88,28 +88,26 @@ __global__ void __launch_bounds__(kBlock) k_props_scan(Grid g, const L* __restri
                                                        const double* __restrict__ precip,
                                                        const float* __restrict__ frac, L* __restrict__ sl,
                                                        double* __restrict__ ss, double* __restrict__ sp,
-                                                       float* __restrict__ sf, int force,
+                                                       float* __restrict__ sf, int force, int per,
                                                        int* __restrict__ list, unsigned int* __restrict__ count) {
-    // block-uniform trip count (block_append is called by every thread of the block)
-    for (int b0 = blockIdx.x * blockDim.x; b0 < (int)g.N; b0 += gridDim.x * blockDim.x) {
-        const int r = b0 + (int)threadIdx.x;
-        bool d = false;
-        if (r < (int)g.N) {
+    scan_blocks(g.N, per, [=](long long v0) {
+        const unsigned int dirty = ballot_words(v0, per, g.N, [=](int r) {
             const L lab = label[r];
             const long long sb = __double_as_longlong(sat[r]);
             const long long pb = __double_as_longlong(precip[r]);
             const unsigned int fb = __float_as_uint(frac[r]);
-            d = force || lab != sl[r] || sb != __double_as_longlong(ss[r]) || pb != __double_as_longlong(sp[r]) ||
-                fb != __float_as_uint(sf[r]);
+            const bool d = force || lab != sl[r] || sb != __double_as_longlong(ss[r]) ||
+                           pb != __double_as_longlong(sp[r]) || fb != __float_as_uint(sf[r]);
             if (d) {
                 sl[r] = lab;
                 ss[r] = __longlong_as_double(sb);
                 sp[r] = __longlong_as_double(pb);
                 sf[r] = __uint_as_float(fb);
             }
-        }
-        block_append(d, r, list, count);
-    }
+            return d;
+        });
+        append_words(dirty, v0, per, list, count);
+    });
 }
 
 // Pass 2: the properties of the listed voxels (dense: every lane has work).
@@ -177,15 +175,16 @@ ls_status props_run(ls_ctx* c) {
     const int force = c->props_force;
     c->props_force = 0;
     LS_TRY(wlist_reset(c));
+    const int per = scan_words(c->num_sms, c->g.N), sgrid = scan_grid(c->num_sms, c->g.N, per);
     if (c->label_bytes == 1) {
-        LS_LAUNCH(c, k_props_scan<uint8_t>, grid, kBlock, 0, c->g, (const uint8_t*)c->label, c->sat, c->precip,
-                  c->frac, (uint8_t*)c->sh_label, c->sh_sat, c->sh_precip, c->sh_frac, force, c->wlist, c->wcount);
+        LS_LAUNCH(c, k_props_scan<uint8_t>, sgrid, kBlock, 0, c->g, (const uint8_t*)c->label, c->sat, c->precip,
+                  c->frac, (uint8_t*)c->sh_label, c->sh_sat, c->sh_precip, c->sh_frac, force, per, c->wlist, c->wcount);
         LS_LAUNCH(c, k_props<uint8_t>, grid, kBlock, 0, pc, (const uint8_t*)c->label, c->sat, c->precip,
                   c->frac, (const float*)c->kmult, c->kr, c->pc, c->perm, c->visc, (const int*)c->wlist,
                   (const unsigned int*)c->wcount);
     } else {
-        LS_LAUNCH(c, k_props_scan<uint16_t>, grid, kBlock, 0, c->g, (const uint16_t*)c->label, c->sat, c->precip,
-                  c->frac, (uint16_t*)c->sh_label, c->sh_sat, c->sh_precip, c->sh_frac, force, c->wlist,
+        LS_LAUNCH(c, k_props_scan<uint16_t>, sgrid, kBlock, 0, c->g, (const uint16_t*)c->label, c->sat, c->precip,
+                  c->frac, (uint16_t*)c->sh_label, c->sh_sat, c->sh_precip, c->sh_frac, force, per, c->wlist,
                   c->wcount);
         LS_LAUNCH(c, k_props<uint16_t>, grid, kBlock, 0, pc, (const uint16_t*)c->label, c->sat, c->precip,
                   c->frac, (const float*)c->kmult, c->kr, c->pc, c->perm, c->visc, (const int*)c->wlist,
@@ -252,32 +251,26 @@ __global__ void __launch_bounds__(kBlock) k_flux_scan(Grid g, const unsigned int
                                                       double* __restrict__ fx, double* __restrict__ fy,
                                                       double* __restrict__ fz, const double* __restrict__ sfx,
                                                       const double* __restrict__ sfy,
-                                                      const double* __restrict__ sfz, int* __restrict__ list,
-                                                      unsigned int* __restrict__ count) {
+                                                      const double* __restrict__ sfz, int per,
+                                                      int* __restrict__ list, unsigned int* __restrict__ count) {
     const int lane = (int)(threadIdx.x & 31u);
-    // block-uniform trip count (block_append is called by every thread of the block)
-    for (long long b0 = (long long)blockIdx.x * blockDim.x; b0 < g.N; b0 += (long long)gridDim.x * blockDim.x) {
-        const long long r0 = b0 + (threadIdx.x & ~31u);
-        const long long r = r0 + lane;
-        const unsigned int own = dwin(bits, nw, r0) | dwin(bits + nw, nw, r0);
-        const unsigned int km = dwin(bits, nw, r0 - 1), kp = dwin(bits, nw, r0 + 1);
-        const unsigned int jm = dwin(bits, nw, r0 - g.K), jp = dwin(bits, nw, r0 + g.K);
-        const unsigned int im = dwin(bits, nw, r0 - g.JK), ip = dwin(bits, nw, r0 + g.JK);
-        bool d = false;
-        if (r < g.N) {
-            int i, j, k;
-            decode(g, r, i, j, k);
-            d = dbit(own, lane) || (i > 0 && dbit(im, lane)) || (i + 1 < g.I && dbit(ip, lane)) ||
-                (j > 0 && dbit(jm, lane)) || (j + 1 < g.J && dbit(jp, lane)) || (k > 0 && dbit(km, lane)) ||
-                (k + 1 < g.K && dbit(kp, lane));
-            if (!d && sfx) {  // null: the fluxes already equal the shadows
-                fx[r] = sfx[r];
-                fy[r] = sfy[r];
-                fz[r] = sfz[r];
+    scan_blocks(g.N, per, [=](long long v0) {
+        const long long s = v0 + 32 * lane;
+        unsigned int need = 0u;
+        if (lane < per && s < g.N)
+            need = stencil_word<true>(g, bits, nw, s, bits[s >> 5] | bits[nw + (s >> 5)]);
+        if (sfx)  // null: the fluxes already equal the shadows
+            for (int q = 0; q < per; ++q) {
+                const long long r = v0 + 32 * q + lane;
+                const unsigned int m = __shfl_sync(0xffffffffu, need, q);
+                if (r < g.N && !((m >> lane) & 1u)) {
+                    fx[r] = sfx[r];
+                    fy[r] = sfy[r];
+                    fz[r] = sfz[r];
+                }
             }
-        }
-        block_append(d, (int)r, list, count);
-    }
+        append_words(need, v0, per, list, count);
+    });
 }
 
 // Pass 3: calculateFlux at the listed voxels.
@@ -339,10 +332,12 @@ ls_status flux_run(ls_ctx* c) {
               c->shq_K, c->shq_V, c->dbits, c->dwords, force);
     // unchanged voxels get their last computed flux back, unless the fluxes still hold it
     const bool restore = !c->fx_is_shadow || force;
-    LS_LAUNCH(c, k_flux_scan, grid, kBlock, 0, c->g, (const unsigned int*)c->dbits, c->dwords, c->fx, c->fy, c->fz,
+    const int per = scan_words(c->num_sms, c->g.N);
+    LS_LAUNCH(c, k_flux_scan, scan_grid(c->num_sms, c->g.N, per), kBlock, 0, c->g, (const unsigned int*)c->dbits,
+              c->dwords, c->fx, c->fy, c->fz,
               restore ? (const double*)c->shq_fx : (const double*)nullptr,
               restore ? (const double*)c->shq_fy : (const double*)nullptr,
-              restore ? (const double*)c->shq_fz : (const double*)nullptr, c->wlist, c->wcount);
+              restore ? (const double*)c->shq_fz : (const double*)nullptr, per, c->wlist, c->wcount);
     LS_LAUNCH(c, k_flux, grid, kBlock, 0, c->g, make_dxdiv(c->p.dx), c->p.max_cap_grad, c->P, c->pc,
               c->perm, c->visc, c->fx, c->fy, c->fz, c->shq_fx, c->shq_fy, c->shq_fz, (const int*)c->wlist,
               (const unsigned int*)c->wcount);
@@ -485,15 +480,14 @@ __global__ void __launch_bounds__(kBlock) k_sat_rate_list(Grid g, DxDiv dd, doub
 }
 
 __global__ void __launch_bounds__(kBlock) k_active_list_sat(Grid g, const uint8_t* __restrict__ l8,
-                                                            const uint16_t* __restrict__ l16,
+                                                            const uint16_t* __restrict__ l16, int per,
                                                             int* __restrict__ list, unsigned int* __restrict__ count) {
-    // block-uniform trip count (block_append is called by every thread of the block)
-    for (long long b0 = (long long)blockIdx.x * blockDim.x; b0 < g.N; b0 += (long long)gridDim.x * blockDim.x) {
-        const long long r = b0 + threadIdx.x;
-        bool act = false;
-        if (r < g.N) act = !sat_inactive(l8 ? (int)l8[r] : (int)l16[r]);
-        block_append(act, (int)r, list, count);
-    }
+    scan_blocks(g.N, per, [=](long long v0) {
+        const unsigned int act = ballot_words(v0, per, g.N, [=](int r) {
+            return !sat_inactive(l8 ? (int)l8[r] : (int)l16[r]);
+        });
+        append_words(act, v0, per, list, count);
+    });
 }
 
 template <typename L>
@@ -533,9 +527,11 @@ ls_status saturation_run(ls_ctx* c, double dt, ls_substep_info* info) {
     if (!c->sat_q) LS_TRY(walloc_t(c, &c->sat_q, (size_t)c->g.N));
     // the active voxels (any order: the pass writes per voxel and takes a maximum)
     LS_TRY(wlist_reset(c));
-    LS_LAUNCH(c, k_active_list_sat, grid, kBlock, 0, c->g,
+    const int per = scan_words(c->num_sms, c->g.N);
+    LS_LAUNCH(c, k_active_list_sat, scan_grid(c->num_sms, c->g.N, per), kBlock, 0, c->g,
               c->label_bytes == 1 ? (const uint8_t*)c->label : (const uint8_t*)nullptr,
-              c->label_bytes == 2 ? (const uint16_t*)c->label : (const uint16_t*)nullptr, c->wlist, c->wcount);
+              c->label_bytes == 2 ? (const uint16_t*)c->label : (const uint16_t*)nullptr, per, c->wlist,
+              c->wcount);
     if (c->label_bytes == 1)
         LS_LAUNCH(c, k_sat_rate_list<uint8_t>, grid, kBlock, 0, c->g, dx, evap, (const uint8_t*)c->label,
                   c->fx, c->fy, c->fz, (const int*)c->wlist, (const unsigned int*)c->wcount, c->sat_q, c->partials);

@@ -108,24 +108,15 @@ __global__ void __launch_bounds__(kBlock) k_faces_dirty(Grid g, const L* __restr
 
 // Pass 2: voxels holding a face (their +i, +j, +k faces) with a dirty voxel on either side.
 __global__ void __launch_bounds__(kBlock) k_faces_scan(Grid g, const unsigned int* __restrict__ bits,
-                                                       long long nw, int* __restrict__ list,
+                                                       long long nw, int per, int* __restrict__ list,
                                                        unsigned int* __restrict__ count) {
     const int lane = (int)(threadIdx.x & 31u);
-    // block-uniform trip count (block_append is called by every thread of the block)
-    for (long long b0 = (long long)blockIdx.x * blockDim.x; b0 < g.N; b0 += (long long)gridDim.x * blockDim.x) {
-        const long long r0 = b0 + (threadIdx.x & ~31u);
-        const long long r = r0 + lane;
-        const unsigned int own = dwin(bits, nw, r0), kp = dwin(bits, nw, r0 + 1),
-                           jp = dwin(bits, nw, r0 + g.K), ip = dwin(bits, nw, r0 + g.JK);
-        bool need = false;
-        if (r < g.N) {
-            int i, j, k;
-            decode(g, r, i, j, k);
-            need = dbit(own, lane) || (i + 1 < g.I && dbit(ip, lane)) || (j + 1 < g.J && dbit(jp, lane)) ||
-                   (k + 1 < g.K && dbit(kp, lane));
-        }
-        block_append(need, (int)r, list, count);
-    }
+    scan_blocks(g.N, per, [=](long long v0) {
+        const long long s = v0 + 32 * lane;
+        unsigned int need = 0u;
+        if (lane < per && s < g.N) need = stencil_word<false>(g, bits, nw, s, bits[s >> 5]);
+        append_words(need, v0, per, list, count);
+    });
 }
 
 // Pass 3: face coefficients of the +i, +j, +k faces of the listed voxels. A face is used
@@ -223,28 +214,18 @@ __device__ __forceinline__ void press_row_eval(const Grid& g, const PressConst& 
 // rows; rows with a dirty voxel in that stencil (face change bits) and all Air rows are listed.
 __global__ void __launch_bounds__(kBlock) k_rows_scan(Grid g, const unsigned int* __restrict__ bits, long long nw,
                                                       const uint8_t* __restrict__ label8,
-                                                      const uint16_t* __restrict__ label16, int force,
+                                                      const uint16_t* __restrict__ label16, int force, int per,
                                                       int* __restrict__ list, unsigned int* __restrict__ count) {
     const int lane = (int)(threadIdx.x & 31u);
-    // block-uniform trip count (block_append is called by every thread of the block)
-    for (long long b0 = (long long)blockIdx.x * blockDim.x; b0 < g.N; b0 += (long long)gridDim.x * blockDim.x) {
-        const long long r0 = b0 + (threadIdx.x & ~31u);
-        const long long r = r0 + lane;
-        const unsigned int own = dwin(bits, nw, r0);
-        const unsigned int km = dwin(bits, nw, r0 - 1), kp = dwin(bits, nw, r0 + 1);
-        const unsigned int jm = dwin(bits, nw, r0 - g.K), jp = dwin(bits, nw, r0 + g.K);
-        const unsigned int im = dwin(bits, nw, r0 - g.JK), ip = dwin(bits, nw, r0 + g.JK);
-        bool d = false;
-        if (r < g.N) {
-            int i, j, k;
-            decode(g, r, i, j, k);
-            const int t = label8 ? (int)label8[r] : (int)label16[r];
-            d = force || t == kAir || dbit(own, lane) || (i > 0 && dbit(im, lane)) ||
-                (i + 1 < g.I && dbit(ip, lane)) || (j > 0 && dbit(jm, lane)) || (j + 1 < g.J && dbit(jp, lane)) ||
-                (k > 0 && dbit(km, lane)) || (k + 1 < g.K && dbit(kp, lane));
-        }
-        block_append(d, (int)r, list, count);
-    }
+    scan_blocks(g.N, per, [=](long long v0) {
+        const long long s = v0 + 32 * lane;
+        unsigned int need = ballot_words(v0, per, g.N, [=](int r) {
+            return (label8 ? (int)label8[r] : (int)label16[r]) == kAir;
+        });
+        if (lane < per && s < g.N)
+            need |= force ? word_tail(g.N, s) : stencil_word<true>(g, bits, nw, s, bits[s >> 5]);
+        append_words(need, v0, per, list, count);
+    });
 }
 
 // Rows pass 2: the listed rows, their (b/diag)^2 for the norm of the relative residual test
@@ -953,7 +934,8 @@ ls_status pressure_setup_run(ls_ctx* c, double t) {
         else
             LS_LAUNCH(c, k_faces_dirty<uint16_t>, grid, kBlock, 0, g, (const uint16_t*)c->label, c->perm, c->visc,
                       (uint16_t*)c->shf_label, c->shf_perm, c->shf_visc, c->dbits, faces_force);
-        LS_LAUNCH(c, k_faces_scan, grid, kBlock, 0, g, (const unsigned int*)c->dbits, c->dwords, c->wlist,
+        const int per = scan_words(c->num_sms, g.N), sgrid = scan_grid(c->num_sms, g.N, per);
+        LS_LAUNCH(c, k_faces_scan, sgrid, kBlock, 0, g, (const unsigned int*)c->dbits, c->dwords, per, c->wlist,
                   c->wcount);
         if (c->label_bytes == 1)
             LS_LAUNCH(c, k_press_faces<uint8_t>, grid, kBlock, 0, g, (const uint8_t*)c->label, c->perm,
@@ -965,9 +947,9 @@ ls_status pressure_setup_run(ls_ctx* c, double t) {
                       (const unsigned int*)c->wcount);
         // rows: the same change bits (labels, faces), plus every Air row (boundary pressure)
         LS_CUDA(c, cudaMemsetAsync(c->wcount, 0, sizeof(unsigned int), c->stream));
-        LS_LAUNCH(c, k_rows_scan, grid, kBlock, 0, g, (const unsigned int*)c->dbits, c->dwords,
+        LS_LAUNCH(c, k_rows_scan, sgrid, kBlock, 0, g, (const unsigned int*)c->dbits, c->dwords,
                   c->label_bytes == 1 ? (const uint8_t*)c->label : (const uint8_t*)nullptr,
-                  c->label_bytes == 2 ? (const uint16_t*)c->label : (const uint16_t*)nullptr, rows_force, c->wlist,
+                  c->label_bytes == 2 ? (const uint16_t*)c->label : (const uint16_t*)nullptr, rows_force, per, c->wlist,
                   c->wcount);
     }  // lean: the work list still holds every voxel
     if (c->label_bytes == 1)

@@ -328,26 +328,15 @@ __global__ void __launch_bounds__(kBlock) k_t_dirty(Grid g, const L* __restrict_
 // forms the right-hand sides of every row (old value over dt, or the old value on identity
 // rows) and the partial norms in a fixed order.
 __global__ void __launch_bounds__(kBlock) k_t_scan(Grid g, const unsigned int* __restrict__ bits, long long nw,
-                                                   int* __restrict__ list, unsigned int* __restrict__ count) {
+                                                   int per, int* __restrict__ list,
+                                                   unsigned int* __restrict__ count) {
     const int lane = (int)(threadIdx.x & 31u);
-    // block-uniform trip count (block_append is called by every thread of the block)
-    for (long long b0 = (long long)blockIdx.x * blockDim.x; b0 < g.N; b0 += (long long)gridDim.x * blockDim.x) {
-        const long long r0 = b0 + (threadIdx.x & ~31u);
-        const long long r = r0 + lane;
-        const unsigned int own = dwin(bits, nw, r0);
-        const unsigned int km = dwin(bits, nw, r0 - 1), kp = dwin(bits, nw, r0 + 1);
-        const unsigned int jm = dwin(bits, nw, r0 - g.K), jp = dwin(bits, nw, r0 + g.K);
-        const unsigned int im = dwin(bits, nw, r0 - g.JK), ip = dwin(bits, nw, r0 + g.JK);
-        bool d = false;
-        if (r < g.N) {
-            int i, j, k;
-            decode(g, r, i, j, k);
-            d = dbit(own, lane) || (i > 0 && dbit(im, lane)) || (i + 1 < g.I && dbit(ip, lane)) ||
-                (j > 0 && dbit(jm, lane)) || (j + 1 < g.J && dbit(jp, lane)) || (k > 0 && dbit(km, lane)) ||
-                (k + 1 < g.K && dbit(kp, lane));
-        }
-        block_append(d, (int)r, list, count);
-    }
+    scan_blocks(g.N, per, [=](long long v0) {
+        const long long s = v0 + 32 * lane;
+        unsigned int need = 0u;
+        if (lane < per && s < g.N) need = stencil_word<true>(g, bits, nw, s, bits[s >> 5]);
+        append_words(need, v0, per, list, count);
+    });
 }
 
 template <typename L>
@@ -1214,7 +1203,9 @@ static ls_status mixed_solve(ls_ctx* c, const Rows<L>& rows, int nrhs, const dou
         LS_TRY(wlist_reset(c));
         LS_LAUNCH(c, k_t_dirty<L>, grid, kBlock, 0, g, rows.label, rows.fx, rows.fy, rows.fz,
                   (L*)c->sht_label, c->sht_fx, c->sht_fy, c->sht_fz, c->dbits, force);
-        LS_LAUNCH(c, k_t_scan, grid, kBlock, 0, g, (const unsigned int*)c->dbits, c->dwords, c->wlist, c->wcount);
+        const int per = scan_words(c->num_sms, g.N);
+        LS_LAUNCH(c, k_t_scan, scan_grid(c->num_sms, g.N, per), kBlock, 0, g, (const unsigned int*)c->dbits, c->dwords,
+                  per, c->wlist, c->wcount);
         LS_LAUNCH(c, k_t_rows<L>, grid, kBlock, 0, rows, tb, (const int*)c->wlist, (const unsigned int*)c->wcount);
         LS_LAUNCH(c, k_t_rhs, grid, kBlock, 0, g, rows.tc.inv_dt, rows.tc.in_val[0], rows.tc.in_val[1], tb, nrhs,
                   f0, f1, (const double*)x0, (const double*)x1, c->partials);
