@@ -117,22 +117,6 @@ __global__ void k_dz_scatter(Grid g, const L* __restrict__ label, const float* _
     }
 }
 
-// a / b, correctly rounded, for several a and one b > 0, from y = 1 / b correctly rounded: with
-// the quotient within an ulp, one residual correction rounds it correctly (Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev.
-// 34(1), 1990); a y is within two ulps, so two corrections. Five FP64 operations instead of a
-// division's dozen or so. For operands whose quotient and residuals stay normal (div_ok).
-__device__ __forceinline__ double div_by(double a, double b, double y) {
-    double q = a * y;
-    q = __fma_rn(__fma_rn(-q, b, a), y, q);
-    return __fma_rn(__fma_rn(-q, b, a), y, q);
-}
-__device__ __noinline__ double div_any(double a, double b) { return a / b; }
-__device__ __forceinline__ bool div_ok(double v, int lo, int hi) {  // zero, or 2^lo <= |v| < 2^hi
-    const unsigned int h = (unsigned int)__double2hiint(v) & 0x7fffffffu;
-    return h - ((unsigned int)(1023 + lo) << 20) < ((unsigned int)(hi - lo) << 20) || (h | (unsigned int)__double2loint(v)) == 0u;
-}
-
 // One voxel of one sub-step (the body of src/Simulation.cpp:475-603). A level's time is the
 // chain of one update, so its memory reads go out together: the six neighbours' labels and acid
 // beside the voxel's own state, whatever the labels turn out to be (indices outside the domain

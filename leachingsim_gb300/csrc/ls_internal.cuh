@@ -172,6 +172,22 @@ __device__ __forceinline__ double drcp_nr(double d) {
     return __fma_rn(y, __fma_rn(-d, y, 1.0), y);
 }
 
+// a / b, correctly rounded, for several a and one b > 0, from y = 1 / b correctly rounded: with
+// the quotient within an ulp, one residual correction rounds it correctly (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev.
+// 34(1), 1990); a y is within two ulps, so two corrections. Five FP64 operations instead of a
+// division's dozen or so. For operands whose quotient and residuals stay normal (div_ok).
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+    double q = a * y;
+    q = __fma_rn(__fma_rn(-q, b, a), y, q);
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+static __device__ __noinline__ double div_any(double a, double b) { return a / b; }
+__device__ __forceinline__ bool div_ok(double v, int lo, int hi) {  // zero, or 2^lo <= |v| < 2^hi
+    const unsigned int h = (unsigned int)__double2hiint(v) & 0x7fffffffu;
+    return h - ((unsigned int)(1023 + lo) << 20) < ((unsigned int)(hi - lo) << 20) || (h | (unsigned int)__double2loint(v)) == 0u;
+}
+
 // Dirty bits of the change-tracked kernels: one bit per voxel, word w holds voxels 32w ..
 // 32w+31. The change tests run warp-aligned (a warp covers voxels r0 .. r0+31, r0 a multiple
 // of 32) and store one ballot word per warp; the scans read windows of 32 neighbours' bits.
