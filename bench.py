@@ -209,7 +209,8 @@ def roofline(ctx, shape, nsteps):
     read or written once: 12 for z = O_r p, v = p - O_b z (p, z, rhat in twice or once; z, v
     out; 14 on the first iteration, which also stores p = r), 18 for s = r - alpha v,
     z = O_r s, t = s - O_b z); one right-hand side is live in this workload (the acid field is
-    zero)."""
+    zero). The launches of a batch beyond the last iteration return at once: their time counts,
+    their bytes do not."""
     peaks_path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     peaks = json.load(open(peaks_path)) if os.path.exists(peaks_path) else None
     ms, cnt = ctx.timing_get("kry_apply")

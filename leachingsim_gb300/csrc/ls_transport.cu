@@ -1139,7 +1139,6 @@ static ls_status inner_solve(ls_ctx* c, const TBuf& tb, const int lane_q[NQ], co
                 else
                     LS_LAUNCH_PDL(c, (k_rb_v<NQ, false>), dgrid, kBlock, 0, rb, iv, (const double*)c->scal,
                                   c->partials);
-                if (c->timing) c->timer_bytes[LS_T_KRY_APPLY] += v_bytes + (it == 0 ? 2.0 * NQ * g.N : 0.0);
             }
             LS_LAUNCH_PDL(c, (k_ti_fin<PH_V, NQ>), 1, ti_fin_threads(ti_values(PH_V, NQ)), 0, (const double*)c->partials, dgrid,
                           c->scal, 0.0, 0.0);
@@ -1147,7 +1146,6 @@ static ls_status inner_solve(ls_ctx* c, const TBuf& tb, const int lane_q[NQ], co
                 Timed tm(c, LS_T_KRY_APPLY);
                 LS_LAUNCH_PDL(c, k_rb_zs<NQ>, grid, kBlock, 0, rb, iv, (const double*)c->scal);
                 LS_LAUNCH_PDL(c, k_rb_t<NQ>, dgrid, kBlock, 0, rb, iv, (const double*)c->scal, c->partials);
-                if (c->timing) c->timer_bytes[LS_T_KRY_APPLY] += st_bytes;
             }
             LS_LAUNCH_PDL(c, (k_ti_fin<PH_ST, NQ>), 1, ti_fin_threads(ti_values(PH_ST, NQ)), 0, (const double*)c->partials, dgrid,
                           c->scal, 0.0, 0.0);
@@ -1172,6 +1170,11 @@ static ls_status inner_solve(ls_ctx* c, const TBuf& tb, const int lane_q[NQ], co
     if (g.K % 2 == 0) LS_LAUNCH_PDL(c, (k_rb_accum<NQ, true>), grid, kBlock, 0, rb, iv, xl[0], xl[1]);
     else LS_LAUNCH_PDL(c, (k_rb_accum<NQ, false>), grid, kBlock, 0, rb, iv, xl[0], xl[1]);
     for (int l = 0; l < NQ; ++l) its[l] = (int)sc[TI_STRIDE * l + TI_ITS];
+    // the launches of a batch beyond the last iteration return at once and move nothing
+    if (c->timing) {
+        const int live = NQ > 1 ? std::max(its[0], its[NQ - 1]) : its[0];
+        c->timer_bytes[LS_T_KRY_APPLY] += live * (v_bytes + st_bytes) + (live > 0 ? 2.0 * NQ * g.N : 0.0);
+    }
     return LS_OK;
 }
 
