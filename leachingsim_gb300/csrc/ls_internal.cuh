@@ -497,7 +497,7 @@ struct ls_ctx {
         int esize;          // sizeof(T)
     };
     std::vector<MGLevel> mg;
-    void* mg0_p;          // other buffer of the inner PCG's p
+    void* mg0_p;          // other buffer of the inner PCG's p (FP32)
     void* mg0_t;
     uint8_t* mg0_flags;   // as MGLevel::flags, finest level
     int mg_is64;          // -1 = not allocated

@@ -428,6 +428,44 @@ __global__ void __launch_bounds__(kBlock) k_mg_smooth_two(int N, int JK, int K, 
     }
 }
 
+// In FP64 the values formed again cost more than the pass that they save (FP64 issue bounds these
+// passes: cold FP64 solve of 338x338x283 219 ms, 188 with the three passes below and k_cg_dir), so
+// there the first sweep, the correction and the second direction are passes of their own.
+template <typename T>
+constexpr bool form_again() { return sizeof(T) == 4; }
+
+// t = omega invd b, the first sweep from zero
+template <typename T>
+__global__ void k_mg_first(int N, const uint8_t* __restrict__ flags, const T* __restrict__ invd,
+                           const T* __restrict__ b, T* __restrict__ t) {
+    pdl_enter();
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < N; r += gridDim.x * blockDim.x)
+        if (flags[r]) t[r] = (T)kOmega * invd[r] * b[r];
+}
+
+// x += scale * x_c(block) of the members
+template <typename T>
+__global__ void k_mg_correct(Grid g, Grid cg, const uint8_t* __restrict__ flags, const T* __restrict__ cx,
+                             T* __restrict__ x, T scale) {
+    pdl_enter();
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < (int)g.N; r += gridDim.x * blockDim.x) {
+        if (!(flags[r] & kCellMember)) continue;
+        int i, j, k;
+        decode(g, r, i, j, k);
+        x[r] += scale * cx[(k >> 1) + cg.K * ((j >> 1) + cg.J * (i >> 1))];
+    }
+}
+
+// pd1 = z - ((z, q0) / (pd0, q0)) pd0
+template <typename T>
+__global__ void k_kc_dir(int N, const uint8_t* __restrict__ flags, const double* __restrict__ s,
+                         const T* __restrict__ z, const T* __restrict__ pd0, T* __restrict__ pd1) {
+    pdl_enter();
+    const T b = block_scalar<T>([=] { return (T)((s[0] > 0.0) ? -s[2] / s[0] : 0.0); });
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < N; r += gridDim.x * blockDim.x)
+        if (flags[r]) pd1[r] = z[r] + b * pd0[r];
+}
+
 // ... on pairs of cells of the finest level (FP32, K even, padded arrays)
 __global__ void __launch_bounds__(kBlock) k_mg_smooth0_two_pair(int N2, int JK2, int K2,
                                                                 const int8_t* __restrict__ kind,
@@ -1063,7 +1101,7 @@ static ls_status mg_alloc(ls_ctx* c) {
     if (!c->comp) LS_TRY(walloc_t(c, &c->comp, (size_t)c->g.N));
     if (!c->cc_flag) LS_TRY(dalloc_t(c, &c->cc_flag, (size_t)4));
     LS_TRY(level_alloc(c, c->g, 1, (void**)&c->mg0_flags));
-    LS_TRY(l0_alloc(c, 10, sizeof(T), &c->mg0_p));
+    if (form_again<T>()) LS_TRY(l0_alloc(c, 10, sizeof(T), &c->mg0_p));
     LS_TRY(l0_alloc(c, 11, sizeof(T), &c->mg0_t));
     Grid g = c->g;
     g.NP = g.N;
@@ -1144,7 +1182,7 @@ ls_status mg_setup(ls_ctx* c) {
 // Zero every level vector (the smoother and the PCG skip non-member cells, which must hold 0).
 template <typename T>
 ls_status mg_clear(ls_ctx* c) {
-    LS_CUDA(c, cudaMemsetAsync(c->mg0_p, 0, sizeof(T) * (size_t)c->g.N, c->stream));
+    if (c->mg0_p) LS_CUDA(c, cudaMemsetAsync(c->mg0_p, 0, sizeof(T) * (size_t)c->g.N, c->stream));
     LS_CUDA(c, cudaMemsetAsync(c->mg0_t, 0, sizeof(T) * (size_t)c->g.N, c->stream));
     for (auto& lv : c->mg) {
         const size_t b = sizeof(T) * (size_t)lv.g.N;
@@ -1222,8 +1260,14 @@ ls_status mg_apply(ls_ctx* c, const T* r, T* z, const T* dotv2, int* nblocks_out
         int nb = 0;
         LS_TRY(cycle(m, (const T*)rr, zb, (const T*)q0, nullptr, &nb));
         LS_TRY(finalize_sum(c, nb, 2, slot + 2));  // (zb, q0)
-        LS_LAUNCH_PDL(c, (k_kc_apply<T, true>), gd, kBlock, 0, N, JK, K, a.flags, s, a.e, a.f0, a.f1, a.f2,
-                  (const T*)zb, (const T*)za, (const T*)rr, pd, q1, c->partials);
+        if (form_again<T>()) {
+            LS_LAUNCH_PDL(c, (k_kc_apply<T, true>), gd, kBlock, 0, N, JK, K, a.flags, s, a.e, a.f0, a.f1, a.f2,
+                      (const T*)zb, (const T*)za, (const T*)rr, pd, q1, c->partials);
+        } else {
+            LS_LAUNCH_PDL(c, k_kc_dir<T>, gd, kBlock, 0, N, a.flags, s, (const T*)zb, (const T*)za, pd);
+            LS_LAUNCH_PDL(c, (k_kc_apply<T, false>), gd, kBlock, 0, N, JK, K, a.flags, s, a.e, a.f0, a.f1, a.f2,
+                      (const T*)nullptr, (const T*)pd, (const T*)rr, (T*)nullptr, q1, c->partials);
+        }
         LS_TRY(finalize_sum(c, gd, 2, slot + 3));  // (pd, q1), (pd, rr)
         LS_LAUNCH_PDL(c, k_kc_second<T>, gd, kBlock, 0, N, a.flags, s, (const T*)pd, e);
         return LS_OK;
@@ -1276,8 +1320,13 @@ ls_status mg_apply(ls_ctx* c, const T* r, T* z, const T* dotv2, int* nblocks_out
                       (const float*)a.f0, (const float*)a.f1, (const float*)a.f2, (const float*)b, (const float*)a.x,
                       (float*)cl.b);
         } else {
-            LS_LAUNCH_PDL(c, k_mg_smooth_two<T>, gd, kBlock, 0, (int)a.g.N, (int)a.g.JK, a.g.K, a.flags, a.e, a.f0, a.f1,
-                      a.f2, a.invd, b, a.x);
+            if (form_again<T>()) {
+                LS_LAUNCH_PDL(c, k_mg_smooth_two<T>, gd, kBlock, 0, (int)a.g.N, (int)a.g.JK, a.g.K, a.flags, a.e, a.f0,
+                          a.f1, a.f2, a.invd, b, a.x);
+            } else {
+                LS_LAUNCH_PDL(c, k_mg_first<T>, gd, kBlock, 0, (int)a.g.N, a.flags, a.invd, b, a.t);
+                LS_TRY(smooth(l, b, (const T*)a.t, a.x, nullptr, nullptr, nullptr));
+            }
             LS_LAUNCH_PDL(c, k_mg_restrict<T>, pass_grid(c, 2 * cl.g.N), kBlock, 0, a.g, cl.g, a.flags, a.e, a.f0, a.f1,
                       a.f2, b, (const T*)a.x, cl.b);
         }
@@ -1306,9 +1355,13 @@ ls_status mg_apply(ls_ctx* c, const T* r, T* z, const T* dotv2, int* nblocks_out
                       (const int8_t*)c->pkind, a.flags, (const float*)a.e, (const float*)a.f0, (const float*)a.f1, (const float*)a.f2,
                       (const float*)a.invd, (const float*)b, (const float*)a.x, (const float*)corr, (float)scale,
                       (float*)a.t);
-        else
+        else if (form_again<T>())
             LS_LAUNCH_PDL(c, k_mg_smooth_corr<T>, pass_grid(c, a.g.N), kBlock, 0, a.g, cl.g, a.flags, a.e, a.f0, a.f1, a.f2, a.invd, b,
                       (const T*)a.x, corr, scale, a.t);
+        else {
+            LS_LAUNCH_PDL(c, k_mg_correct<T>, gd, kBlock, 0, a.g, cl.g, a.flags, corr, a.x, scale);
+            LS_TRY(smooth(l, b, (const T*)a.x, a.t, nullptr, nullptr, nullptr));
+        }
         return smooth(l, b, (const T*)a.t, out, dv, dv2, nb);
     };
     return cycle(0, r, z, r, dotv2, nblocks_out);

@@ -608,8 +608,9 @@ __global__ void k_press_accumulate(Grid g, const int8_t* __restrict__ kind,
 // kernel writes them there (the buffers are cleared when allocated), so the inner PCG
 // kernels skip those voxels: ~3/4 of the box in a porosity-0.25 medium.
 
-// q = M p, partial (p, q). DIR (flexible CG): the direction z + beta p is formed here, and
-// again at the neighbours, and stored in po, instead of by k_cg_dir's pass.
+// q = M p, partial (p, q). DIR (flexible CG, FP32): the direction z + beta p is formed here, and
+// again at the neighbours, and stored in po, instead of by k_cg_dir's pass (which FP64 keeps: its
+// issue slots bound the product).
 template <typename T, bool DIR>
 __global__ void __launch_bounds__(kBlock) k_cg_apply(int N, int JK, int K, const int8_t* __restrict__ kind,
                                                      const double* __restrict__ scal, const T* __restrict__ z,
@@ -729,13 +730,15 @@ __global__ void __launch_bounds__(kBlock) k_cg_jacobi(Grid g, const T* __restric
     block_sum_store<1>(acc, partials);
 }
 
-// p = z + b p with b = (r,z)_new / (r,z)_old (fixed preconditioner; the flexible CG that the
-// K-cycle needs, Notay's FCG(1) with b = -(z_new, q) / (p, q), forms p in its product)
+// p = z + b p with b = (r,z)_new / (r,z)_old (fixed preconditioner) or, for the flexible CG
+// that the K-cycle needs, b = -(z_new, q) / (p, q) (Notay's FCG(1))
 template <typename T>
 __global__ void k_cg_dir(Grid g, const int8_t* __restrict__ kind, const double* __restrict__ scal,
-                         const T* __restrict__ z, T* __restrict__ p) {
+                         const T* __restrict__ z, T* __restrict__ p, int flexible) {
     pdl_enter();
-    const T beta = block_scalar<T>([=] { return (T)(scal[SP_RZN] / scal[SP_RZ]); });
+    const T beta = block_scalar<T>([=] {
+        return (T)(flexible ? ((scal[SP_PQ] > 0.0) ? -scal[SP_ZQ] / scal[SP_PQ] : 0.0) : scal[SP_RZN] / scal[SP_RZ]);
+    });
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
          r += (long long)gridDim.x * blockDim.x)
         if (kind[r] == 2) p[r] = z[r] + beta * p[r];
@@ -829,7 +832,7 @@ static ls_status inner_pcg(ls_ctx* c, bool use_mg, double tol, int max_it, int* 
     for (int it = 0; it < max_it; ++it) {
         {
             Timed tm(c, LS_T_CG_APPLY);
-            const bool dir = use_mg && it > 0;
+            const bool dir = use_mg && it > 0 && sizeof(T) == 4;
             if (pair && dir) {
                 LS_LAUNCH_PDL(c, k_cg_dir_apply0_pair, pgrid, kBlock, 0, (int)(g.N / 2), (int)(g.JK / 2), g.K / 2,
                           (const int8_t*)c->pkind, (const double*)c->scal, (const float*)z, (const float*)p,
@@ -886,8 +889,11 @@ static ls_status inner_pcg(ls_ctx* c, bool use_mg, double tol, int max_it, int* 
         if (rz <= target || !(pq > 0.0) || rz < 0.0) break;
         if (!use_mg) {
             LS_LAUNCH_PDL(c, k_cg_dir<T>, grid, kBlock, 0, g, (const int8_t*)c->pkind, (const double*)c->scal,
-                      (const T*)z, p);
+                      (const T*)z, p, 0);
             LS_LAUNCH_PDL(c, k_set_scalar, 1, 1, 0, c->scal, SP_RZ, SP_RZN);
+        } else if (sizeof(T) == 8) {
+            LS_LAUNCH_PDL(c, k_cg_dir<T>, grid, kBlock, 0, g, (const int8_t*)c->pkind, (const double*)c->scal,
+                      (const T*)z, p, 1);
         }
     }
     *rel_out = sqrt(std::max(rz, 0.0) / rz0);
