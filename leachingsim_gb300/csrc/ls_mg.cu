@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(kBlock, kPassBlocks) k_mg_smooth0_corr_pair(Gr
 
 // Coarse right-hand side of the finest level on pairs (FP32, K even, padded arrays): a thread
 // forms the residuals of its block's four pairs and sums the members' in the child order of
-// k_mg_restrict. The residuals stay in registers: 54 us instead of 38 for a
+// k_mg_restrict. The residuals stay in registers: 41 us instead of 38 for a
 // residual pass and 28 for a gather at 160x256x256.
 __global__ void __launch_bounds__(kBlock, kPassBlocks) k_mg_restrict0_pair(Grid g, Grid cg, const uint8_t* __restrict__ flags,
                                                               const float* __restrict__ e,
