@@ -858,11 +858,19 @@ __global__ void __launch_bounds__(kBlock) k_rb_pending(RBGrid g, TIVec iv, const
 }
 
 // both halves of the correction into the FP64 solution: x_b += d, x_r += f_r - O_r d (EVEN: the
-// pairs of voxels are 16-byte aligned)
+// pairs of voxels are 16-byte aligned). A lane whose system FP32 does not hold (a norm that
+// overflowed before the first update, or one that underflowed to 0) keeps its solution.
 template <int NQ, bool EVEN>
-__global__ void __launch_bounds__(kBlock) k_rb_accum(RBGrid g, TIVec iv, double* __restrict__ x0,
-                                                     double* __restrict__ x1) {
+__global__ void __launch_bounds__(kBlock) k_rb_accum(RBGrid g, TIVec iv, const double* __restrict__ scal,
+                                                     double* __restrict__ x0, double* __restrict__ x1) {
     pdl_enter();
+    bool add[NQ];
+#pragma unroll
+    for (int l = 0; l < NQ; ++l) {
+        const long long reason = __double_as_longlong(scal[tslot(l, TI_REASON)]);
+        const bool started = __double_as_longlong(scal[tslot(l, TI_ITS)]) != 0;
+        add[l] = (started || reason != __double_as_longlong(-4.0)) && dpos(scal[tslot(l, TI_RR0)]);
+    }
     const int n = (int)(g.H / (4 / NQ));
     const SrcVec<NQ> src{iv.d};
     const SrcRhs<NQ> red{iv.rhs[0] + g.H, iv.rhs[1] + g.H};
@@ -881,6 +889,7 @@ __global__ void __launch_bounds__(kBlock) k_rb_accum(RBGrid g, TIVec iv, double*
             const int k0 = 2 * (k2 + m / NQ);
             const float dr = f.v[m] - y.v[m];
             const double e0 = widen(par ? dr : d.v[m]), e1 = widen(par ? d.v[m] : dr);  // at k0, k0 + 1
+            if (!add[m % NQ]) continue;
             if (EVEN) {
                 if (k0 < g.K) {
                     D2* q = reinterpret_cast<D2*>(x + base + k0);
@@ -1167,8 +1176,8 @@ static ls_status inner_solve(ls_ctx* c, const TBuf& tb, const int lane_q[NQ], co
     }
     LS_LAUNCH_PDL(c, k_rb_pending<NQ>, grid, kBlock, 0, rb, iv, (const double*)c->scal);
     double* const xl[2] = {x[lane_q[0]], NQ > 1 ? x[lane_q[1]] : (double*)nullptr};
-    if (g.K % 2 == 0) LS_LAUNCH_PDL(c, (k_rb_accum<NQ, true>), grid, kBlock, 0, rb, iv, xl[0], xl[1]);
-    else LS_LAUNCH_PDL(c, (k_rb_accum<NQ, false>), grid, kBlock, 0, rb, iv, xl[0], xl[1]);
+    if (g.K % 2 == 0) LS_LAUNCH_PDL(c, (k_rb_accum<NQ, true>), grid, kBlock, 0, rb, iv, (const double*)c->scal, xl[0], xl[1]);
+    else LS_LAUNCH_PDL(c, (k_rb_accum<NQ, false>), grid, kBlock, 0, rb, iv, (const double*)c->scal, xl[0], xl[1]);
     for (int l = 0; l < NQ; ++l) its[l] = (int)sc[TI_STRIDE * l + TI_ITS];
     // the launches of a batch beyond the last iteration return at once and move nothing
     if (c->timing) {
