@@ -183,9 +183,10 @@ __device__ __forceinline__ double div_by(double a, double b, double y) {
     return __fma_rn(__fma_rn(-q, b, a), y, q);
 }
 static __device__ __noinline__ double div_any(double a, double b) { return a / b; }
-__device__ __forceinline__ bool div_ok(double v, int lo, int hi) {  // zero, or 2^lo <= |v| < 2^hi
-    const unsigned int h = (unsigned int)__double2hiint(v) & 0x7fffffffu;
-    return h - ((unsigned int)(1023 + lo) << 20) < ((unsigned int)(hi - lo) << 20) || (h | (unsigned int)__double2loint(v)) == 0u;
+// +0, or 2^lo <= |v| < 2^hi (not -0: div_by's corrections add +0 to it, and the quotient's sign is lost)
+__device__ __forceinline__ bool div_ok(double v, int lo, int hi) {
+    const unsigned int w = (unsigned int)__double2hiint(v), h = w & 0x7fffffffu;
+    return h - ((unsigned int)(1023 + lo) << 20) < ((unsigned int)(hi - lo) << 20) || (w | (unsigned int)__double2loint(v)) == 0u;
 }
 
 // Dirty bits of the change-tracked kernels: one bit per voxel, word w holds voxels 32w ..
