@@ -208,35 +208,65 @@ struct Rows {
 // past a row's end are virtual: zero links, zero values). The neighbours of an element at h are
 // the other colour's elements at h -+ J K2p (i), h -+ K2p (j), and along k at h ("near") and at
 // h + 1 (odd k) or h - 1 (even k) ("far").
+// I, J, K are the layout's extents and i, j, k its coordinates: those of the grid (axis 2), or,
+// where rows along k are so short that the rounding makes the arrays larger, the grid's (i, k, j)
+// (axis 1) or (j, k, i) (axis 0).
 struct RBGrid {
     int I, J, K, K2p, JK2;
+    int axis;        // of the grid, along which the layout's rows run
+    int si, sj, sk;  // strides of i, j and k in the voxel arrays
     long long H;
     FastDiv div4, div2, div_j;  // by K2p / 4, K2p / 2 and J
 };
 
+// of the grid's voxel (i, j, k)
 __host__ __device__ __forceinline__ int rb_index(const RBGrid& g, int i, int j, int k, int& colour) {
     colour = (i + j + k) & 1;
-    return (k >> 1) + g.K2p * (j + g.J * i);
+    const int li = g.axis == 0 ? j : i, lj = g.axis == 2 ? j : k, lk = g.axis == 2 ? k : g.axis == 1 ? j : i;
+    return (lk >> 1) + g.K2p * (lj + g.J * li);
 }
 
-static RBGrid make_rb(const Grid& g) {
+static RBGrid make_rb_axis(const Grid& g, int axis) {
+    const int n[3] = {g.I, g.J, g.K}, stride[3] = {(int)g.JK, g.K, 1};
+    const int ai = axis == 0 ? 1 : 0, aj = axis == 2 ? 1 : 2;
     RBGrid r;
-    r.I = g.I;
-    r.J = g.J;
-    r.K = g.K;
-    r.K2p = (((g.K + 1) / 2 + 3) / 4) * 4;
-    r.JK2 = g.J * r.K2p;
-    r.H = (long long)g.I * r.JK2;
+    r.axis = axis;
+    r.I = n[ai];
+    r.J = n[aj];
+    r.K = n[axis];
+    r.si = stride[ai];
+    r.sj = stride[aj];
+    r.sk = stride[axis];
+    r.K2p = (((r.K + 1) / 2 + 3) / 4) * 4;
+    r.JK2 = r.J * r.K2p;
+    r.H = (long long)r.I * r.JK2;
     r.div4 = make_fastdiv((unsigned int)(r.K2p / 4));
     r.div2 = make_fastdiv((unsigned int)(r.K2p / 2));
-    r.div_j = make_fastdiv((unsigned int)g.J);
+    r.div_j = make_fastdiv((unsigned int)r.J);
     return r;
+}
+
+// Rows along k, whose chunks are neighbours in the voxel arrays too, unless the virtual elements
+// make more than 3/8 of the real ones (K of 2-5, 9-11, 17): the links, residuals and vectors of the
+// solve, 64 bytes a voxel with none, would take more than the 88 that a layout of whole rows takes.
+// Then the axis whose vectors, with the plane of zeros at either end, are the smallest. Two
+// species to 1e-10, rows along k against rows along j: 2000x2000x2 6.9 and 3.2 ms, 2000x2000x5 8.8
+// and 8.0, 1700x1700x9 12.2 and 10.4, 1500x1500x11 10.3 and 9.9, 1200x1200x17 9.96 and 9.76 (whole
+// rows: 7.5, 16.5, 21.0, 20.1, 19.9).
+static RBGrid make_rb(const Grid& g) {
+    RBGrid best = make_rb_axis(g, 2);
+    if (16 * best.H <= 11 * g.N) return best;
+    for (int axis = 1; axis >= 0; --axis) {
+        const RBGrid r = make_rb_axis(g, axis);
+        if (r.H + 2 * r.JK2 < best.H + 2 * best.JK2) best = r;
+    }
+    return best;
 }
 
 struct TBuf {
     double* c[7];
     double* b[2];
-    float* o[6];  // FP32 scaled links, black then red (H each): -i, -j, near, far, +j, +i
+    float* o[6];  // FP32 scaled links, black then red (H each): -i, -j, near, far, +j, +i of the layout
     double* inv;
     int8_t* kind;
     RBGrid rb;
@@ -247,13 +277,18 @@ __device__ __forceinline__ void store_links(const TBuf& tb, int i, int j, int k,
     int colour;
     const int h = rb_index(tb.rb, i, j, k, colour);
     const long long at = colour * tb.rb.H + h;
-    const bool odd = k & 1;
-    tb.o[0][at] = d2f_rz(off[1]) * inv32;
-    tb.o[1][at] = d2f_rz(off[3]) * inv32;
-    tb.o[2][at] = d2f_rz(odd ? off[5] : off[4]) * inv32;
-    tb.o[3][at] = d2f_rz(odd ? off[4] : off[5]) * inv32;
-    tb.o[4][at] = d2f_rz(off[2]) * inv32;
-    tb.o[5][at] = d2f_rz(off[0]) * inv32;
+    auto put = [&](double ip, double im, double jp, double jm, double kp, double km, int lk) {
+        const bool odd = lk & 1;
+        tb.o[0][at] = d2f_rz(im) * inv32;
+        tb.o[1][at] = d2f_rz(jm) * inv32;
+        tb.o[2][at] = d2f_rz(odd ? km : kp) * inv32;
+        tb.o[3][at] = d2f_rz(odd ? kp : km) * inv32;
+        tb.o[4][at] = d2f_rz(jp) * inv32;
+        tb.o[5][at] = d2f_rz(ip) * inv32;
+    };
+    if (tb.rb.axis == 2) put(off[0], off[1], off[2], off[3], off[4], off[5], k);
+    else if (tb.rb.axis == 1) put(off[0], off[1], off[4], off[5], off[2], off[3], j);
+    else put(off[2], off[3], off[4], off[5], off[0], off[1], i);
 }
 
 template <typename L, bool EXPL>
@@ -453,6 +488,8 @@ __global__ void __launch_bounds__(kBlock) k_t_resid(Grid g, TBuf tb, const doubl
         ld_rows<V>(tb.inv, r, inv);
         int colour;
         const int h = rb_index(tb.rb, i, j, k, colour);
+        // rows k and k + 1 (k even) differ in colour only, unless k is not the layout's row axis
+        const int h1 = tb.rb.axis == 2 ? h : h + tb.rb.K2p;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             if (!(MASK >> q & 1)) continue;
@@ -479,8 +516,8 @@ __global__ void __launch_bounds__(kBlock) k_t_resid(Grid g, TBuf tb, const doubl
                 a = __fma_rn(-c[1][e], xip[e], a);
                 const double rv = a * inv[e];
                 // the inner right-hand side in FP32 rounded toward zero on the integer pipe (its
-                // rounding is the inner solve's business); rows k and k + 1 differ in colour only
-                const long long at = (e ? colour ^ 1 : colour) * tb.rb.H + h;
+                // rounding is the inner solve's business)
+                const long long at = (e ? colour ^ 1 : colour) * tb.rb.H + (e ? h1 : h);
                 (q ? r1 : r0)[at] = d2f_rz(rv);
                 acc[q] = __fma_rn(rv, rv, acc[q]);
                 nan[q] += disnan(rv) ? 1 : 0;
@@ -860,8 +897,8 @@ __global__ void __launch_bounds__(kBlock) k_rb_pending(RBGrid g, TIVec iv, const
     }
 }
 
-// both halves of the correction into the FP64 solution: x_b += d, x_r += f_r - O_r d (EVEN: the
-// pairs of voxels are 16-byte aligned). A lane whose system FP32 does not hold (a norm that
+// both halves of the correction into the FP64 solution: x_b += d, x_r += f_r - O_r d (EVEN: rows
+// along k whose pairs of voxels are 16-byte aligned). A lane whose system FP32 does not hold (a norm that
 // overflowed before the first update, or one that underflowed to 0) keeps its solution.
 template <int NQ, bool EVEN>
 __global__ void __launch_bounds__(kBlock) k_rb_accum(RBGrid g, TIVec iv, const double* __restrict__ scal,
@@ -882,10 +919,10 @@ __global__ void __launch_bounds__(kBlock) k_rb_accum(RBGrid g, TIVec iv, const d
         Chunk<NQ> d;
         const Chunk<NQ> y = rb_links<NQ, 1>(g, iv, ch, src, d);
         const Chunk<NQ> f = red.chunk(h);
-        const int ch4 = (int)fdiv(NQ == 1 ? g.div4 : g.div2, (unsigned int)ch);
-        const int row = ch4, k2 = h - row * g.K2p, i = (int)fdiv(g.div_j, (unsigned int)row);
-        const int par = (row - i * g.J + i) & 1;  // black at k = 2 k2 + par, red at 2 k2 + 1 - par
-        const long long base = (long long)row * g.K;
+        const int row = (int)fdiv(NQ == 1 ? g.div4 : g.div2, (unsigned int)ch), i = (int)fdiv(g.div_j, (unsigned int)row);
+        const int k2 = h - row * g.K2p, j = row - i * g.J;
+        const int par = (i + j) & 1;  // black at k = 2 k2 + par, red at 2 k2 + 1 - par
+        const long long base = (long long)i * g.si + (long long)j * g.sj;
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
             double* x = (m % NQ) ? x1 : x0;
@@ -902,8 +939,8 @@ __global__ void __launch_bounds__(kBlock) k_rb_accum(RBGrid g, TIVec iv, const d
                     *q = w;
                 }
             } else {
-                if (k0 < g.K) x[base + k0] += e0;
-                if (k0 + 1 < g.K) x[base + k0 + 1] += e1;
+                if (k0 < g.K) x[base + k0 * g.sk] += e0;
+                if (k0 + 1 < g.K) x[base + (k0 + 1) * g.sk] += e1;
             }
         }
     }
@@ -1179,7 +1216,7 @@ static ls_status inner_solve(ls_ctx* c, const TBuf& tb, const int lane_q[NQ], co
     }
     LS_LAUNCH_PDL(c, k_rb_pending<NQ>, grid, kBlock, 0, rb, iv, (const double*)c->scal);
     double* const xl[2] = {x[lane_q[0]], NQ > 1 ? x[lane_q[1]] : (double*)nullptr};
-    if (g.K % 2 == 0) LS_LAUNCH_PDL(c, (k_rb_accum<NQ, true>), grid, kBlock, 0, rb, iv, (const double*)c->scal, xl[0], xl[1]);
+    if (rb.axis == 2 && g.K % 2 == 0) LS_LAUNCH_PDL(c, (k_rb_accum<NQ, true>), grid, kBlock, 0, rb, iv, (const double*)c->scal, xl[0], xl[1]);
     else LS_LAUNCH_PDL(c, (k_rb_accum<NQ, false>), grid, kBlock, 0, rb, iv, (const double*)c->scal, xl[0], xl[1]);
     for (int l = 0; l < NQ; ++l) its[l] = (int)sc[TI_STRIDE * l + TI_ITS];
     // the launches of a batch beyond the last iteration return at once and move nothing
