@@ -539,6 +539,8 @@ ls_status ls_create(ls_ctx** out, int I, int J, int K, int label_bytes, const ls
         c->mg_graphs_off = (gv && gv[0] == '0') ? 1 : 0;
         const char* tv = getenv("LS_MG_TAIL_CELLS");
         c->mg_tail_cells = tv ? std::max(0ll, atoll(tv)) : -1;
+        const char* cv = getenv("LS_MG_CLUSTER");
+        c->mg_cluster_max = cv ? atoi(cv) : 16;
         const char* pv = getenv("LS_PDL");
         c->pdl = (pv && pv[0] == '0') ? 0 : 1;
     }

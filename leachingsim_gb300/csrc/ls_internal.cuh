@@ -506,6 +506,7 @@ struct ls_ctx {
     int mg_graphs_off;    // 1: launch the cycle kernel by kernel (LS_MG_GRAPHS=0)
     long long mg_tail_cells;  // coarse levels up to this many cells run fused (LS_MG_TAIL_CELLS; 0: off, -1: default)
     int mg_cluster;           // blocks of the fused kernel's cluster (0: not available)
+    int mg_cluster_max;       // the most that it may take (LS_MG_CLUSTER)
     int pdl;                  // programmatic dependent launch in the multigrid cycle (LS_PDL; 0: off)
     int* comp;            // fine-level strong-component ids (-1 = not an inner unknown)
     uint8_t* start_anchor; // per component root: anchored to fixed values (supplied starts)

@@ -1072,16 +1072,17 @@ static ls_status fuse_launch(ls_ctx* c, const FuseArgs<T>& fa, size_t smem) {
     return e == cudaSuccess ? LS_OK : check_cuda(c, e, "k_mg_fused");
 }
 
-// The cluster of k_mg_fused: 16 blocks where the device can hold such a cluster, else 8, else
-// none (0: the level kernels).
+// The cluster of k_mg_fused: 16 blocks where the device can hold such a cluster (and max_blocks
+// allows it), else 8, else none (0: the level kernels).
 template <typename T>
-static int fuse_cluster() {
+static int fuse_cluster(int max_blocks) {
     if (cudaFuncSetAttribute(k_mg_fused<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
         cudaFuncSetAttribute(k_mg_fused<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFuseSmem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     for (int blocks = 16; blocks >= 8; blocks /= 2) {
+        if (blocks > max_blocks) continue;
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute at[2];
         fuse_config(cfg, at, blocks, kFuseSmem, 0);
@@ -1097,7 +1098,7 @@ static ls_status mg_alloc(ls_ctx* c) {
     const int is64 = sizeof(T) == 8;
     if (c->mg_is64 == is64) return LS_OK;
     mg_free(c);
-    c->mg_cluster = fuse_cluster<T>();
+    c->mg_cluster = fuse_cluster<T>(c->mg_cluster_max);
     if (!c->comp) LS_TRY(walloc_t(c, &c->comp, (size_t)c->g.N));
     if (!c->cc_flag) LS_TRY(dalloc_t(c, &c->cc_flag, (size_t)4));
     LS_TRY(level_alloc(c, c->g, 1, (void**)&c->mg0_flags));
