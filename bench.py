@@ -201,7 +201,7 @@ def run_steps(ctx, t0, n0, count, dt):
     return t, n, infos
 
 
-def roofline(ctx, shape, nsteps):
+def roofline(ctx, shape, infos):
     """Roofline of the dominant kernel class, the transport operator applications of the
     inner BiCGStab on the red-black reduced system (two half sweeps each: k_rb_z + k_rb_v and
     k_rb_zs + k_rb_t). The library accumulates their algorithmic bytes per application: N x (six
@@ -209,13 +209,15 @@ def roofline(ctx, shape, nsteps):
     read or written once: 12 for z = O_r p, v = p - O_b z (p, z, rhat in twice or once; z, v
     out; 14 on the first iteration, which also stores p = r), 18 for s = r - alpha v,
     z = O_r s, t = s - O_b z); one right-hand side is live in this workload (the acid field is
-    zero). The launches of a batch beyond the last iteration return at once: their time counts,
-    their bytes do not."""
+    zero). The launches of a batch beyond the last iteration return at once and move nothing: every
+    figure per launch is per application of an iteration that ran (two each, from the steps'
+    infos), with all of the class's time; `launched` counts the idle ones too."""
     peaks_path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     peaks = json.load(open(peaks_path)) if os.path.exists(peaks_path) else None
     ms, cnt = ctx.timing_get("kry_apply")
     nbytes = ctx.timing_bytes("kry_apply")
-    if cnt == 0 or ms <= 0:
+    live = 2 * sum(max(i["conc"]["iterations"], i["acid"]["iterations"]) for i in infos)
+    if live == 0 or ms <= 0:
         return None
     achieved = nbytes / (ms / 1e3) / 1e9
     peak, src = (peaks["hbm_gbs"], "measured") if peaks else (6800.0, "fallback")
@@ -227,8 +229,8 @@ def roofline(ctx, shape, nsteps):
     return {"bound": "hbm", "kernel": "transport operator apply (k_rb_z + k_rb_v, k_rb_zs + k_rb_t)",
             "achieved": round(achieved, 1), "peak": peak, "peak_source": src, "unit": "GB/s",
             "frac": round(achieved / peak, 4), "traffic": round(traffic),
-            "bytes_per_launch": round(nbytes / cnt), "bytes_per_voxel": round(nbytes / cnt / vox, 2),
-            "launches": cnt, "us_per_launch": round(ms * 1e3 / cnt, 2)}
+            "bytes_per_launch": round(nbytes / live), "bytes_per_voxel": round(nbytes / live / vox, 2),
+            "launches": live, "launched": cnt, "us_per_launch": round(ms * 1e3 / live, 2)}
 
 
 def true_rel_residual(ctx):
@@ -383,7 +385,7 @@ def gpu_arm(args, ws, rank, local):
     classes = {k: ctx.timing_get(k) for k in ("props", "press_setup", "press_inner", "press_outer",
                                               "flux", "saturation", "transport", "precip",
                                               "dissolve", "snapshot", "kry_apply", "cg_apply")}
-    roof = roofline(ctx, shape, args.steps)
+    roof = roofline(ctx, shape, infos)
     ctx.timing(False)
     mem = ctx.device_bytes()
     # the CPU baseline leg at the full grid, from this state (rank 0 of a 1-GPU run)
