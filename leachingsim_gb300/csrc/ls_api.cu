@@ -692,6 +692,8 @@ ls_status ls_destroy(ls_ctx* c) {
     for (float* q : c->trhs) rel(q);
     rel(c->ti);
     rel(c->start_anchor);
+    rel(c->t_hard);
+    for (double* q : c->t_keep) rel(q);
     {
         void* lp[] = {c->lpc_c0, c->lpc_c1, c->lpc_c2, c->lpc_out, c->lpc_isd, c->lpc_anchor};
         for (void* q : lp) rel(q);

@@ -533,7 +533,9 @@ struct ls_ctx {
     float* ti;            // FP32 inner vectors r rh p v s t d z of one colour, padded, float or float2
     long long ti_half;    // elements of one colour (virtual ones included)
     long long ti_pad, ti_stride;  // zero elements around each vector; floats per vector
-    int8_t* tkind;        // 1 identity row, 2 coupled row
+    int8_t* tkind;        // 1 identity row, 2 coupled row, 3 inflow row; 4 added: a hard row
+    int* t_hard;          // number of hard rows (change-tracked rows)
+    double* t_keep[2];    // first solution of a solve with hard rows, per right-hand side (null until one comes)
 
     // dissolution
     int* dz_list;         // active mineral voxels sorted by wavefront (or by dependency level)

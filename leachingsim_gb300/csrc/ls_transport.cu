@@ -268,32 +268,48 @@ struct TBuf {
     double* b[2];
     float* o[6];  // FP32 scaled links, black then red (H each): -i, -j, near, far, +j, +i of the layout
     double* inv;
-    int8_t* kind;
+    int8_t* kind;  // trans_row's, kHardRow added on hard rows
     RBGrid rb;
 };
 
-// the FP32 links of row (i, j, k) from its FP64 off-diagonals (+i,-i,+j,-j,+k,-k)
-__device__ __forceinline__ void store_links(const TBuf& tb, int i, int j, int k, const double off[6], float inv32) {
+// A hard row: its links outweigh its diagonal by more than kHardSum (much more inflow than outflow; a
+// flow without sources has at most as much). Systems with one keep their first solution and turn
+// to the whole system when the reduced one fails (mixed_solve).
+constexpr int kHardRow = 4;
+constexpr float kHardSum = 16.f;
+__device__ __forceinline__ int row_kind(int k) { return k & (kHardRow - 1); }
+
+// the FP32 links of row (i, j, k) from its FP64 off-diagonals (+i,-i,+j,-j,+k,-k); whether they
+// make a hard row
+__device__ __forceinline__ bool store_links(const TBuf& tb, int i, int j, int k, const double off[6], float inv32) {
     int colour;
     const int h = rb_index(tb.rb, i, j, k, colour);
     const long long at = colour * tb.rb.H + h;
-    auto put = [&](double ip, double im, double jp, double jm, double kp, double km, int lk) {
+    float o[6], sum = 0.f;
+#pragma unroll
+    for (int d = 0; d < 6; ++d) {
+        o[d] = d2f_rz(off[d]) * inv32;
+        sum += fabsf(o[d]);
+    }
+    auto put = [&](float ip, float im, float jp, float jm, float kp, float km, int lk) {
         const bool odd = lk & 1;
-        tb.o[0][at] = d2f_rz(im) * inv32;
-        tb.o[1][at] = d2f_rz(jm) * inv32;
-        tb.o[2][at] = d2f_rz(odd ? km : kp) * inv32;
-        tb.o[3][at] = d2f_rz(odd ? kp : km) * inv32;
-        tb.o[4][at] = d2f_rz(jp) * inv32;
-        tb.o[5][at] = d2f_rz(ip) * inv32;
+        tb.o[0][at] = im;
+        tb.o[1][at] = jm;
+        tb.o[2][at] = odd ? km : kp;
+        tb.o[3][at] = odd ? kp : km;
+        tb.o[4][at] = jp;
+        tb.o[5][at] = ip;
     };
-    if (tb.rb.axis == 2) put(off[0], off[1], off[2], off[3], off[4], off[5], k);
-    else if (tb.rb.axis == 1) put(off[0], off[1], off[4], off[5], off[2], off[3], j);
-    else put(off[2], off[3], off[4], off[5], off[0], off[1], i);
+    if (tb.rb.axis == 2) put(o[0], o[1], o[2], o[3], o[4], o[5], k);
+    else if (tb.rb.axis == 1) put(o[0], o[1], o[4], o[5], o[2], o[3], j);
+    else put(o[2], o[3], o[4], o[5], o[0], o[1], i);
+    return sum > kHardSum;
 }
 
 template <typename L, bool EXPL>
 __global__ void __launch_bounds__(kBlock) k_t_setup(Rows<L> op, TBuf tb, int nrhs, const double* f0,
-                                                    const double* f1, double* __restrict__ partials) {
+                                                    const double* f1, int* __restrict__ hard,
+                                                    double* __restrict__ partials) {
     double acc[2] = {0.0, 0.0};
     const Grid& g = op.g;
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
@@ -313,8 +329,9 @@ __global__ void __launch_bounds__(kBlock) k_t_setup(Rows<L> op, TBuf tb, int nrh
         tb.inv[r] = inv;
 #pragma unroll
         for (int d = 0; d < 6; ++d) tb.c[1 + d][r] = off[d];
-        store_links(tb, i, j, k, off, inv32);
-        tb.kind[r] = (int8_t)kind;
+        const bool hr = store_links(tb, i, j, k, off, inv32);
+        if (hr) atomicAdd(hard, 1);
+        tb.kind[r] = (int8_t)(kind + (hr ? kHardRow : 0));
         for (int q = 0; q < nrhs; ++q) {
             tb.b[q][r] = rhs[q];
             double bt = rhs[q] * inv;
@@ -375,8 +392,8 @@ __global__ void __launch_bounds__(kBlock) k_t_scan(Grid g, const unsigned int* _
 }
 
 template <typename L>
-__global__ void __launch_bounds__(kBlock) k_t_rows(Rows<L> op, TBuf tb, const int* __restrict__ list,
-                                                   const unsigned int* __restrict__ count) {
+__global__ void __launch_bounds__(kBlock) k_t_rows(Rows<L> op, TBuf tb, int force, const int* __restrict__ list,
+                                                   const unsigned int* __restrict__ count, int* __restrict__ hard) {
     const Grid& g = op.g;
     const int n = (int)*count;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
@@ -392,8 +409,10 @@ __global__ void __launch_bounds__(kBlock) k_t_rows(Rows<L> op, TBuf tb, const in
         tb.inv[r] = inv;
 #pragma unroll
         for (int d = 0; d < 6; ++d) tb.c[1 + d][r] = off[d];
-        store_links(tb, i, j, k, off, inv32);
-        tb.kind[r] = (int8_t)kind;
+        // the number of hard rows follows the marks (force: it starts from 0, the old marks mean nothing)
+        const bool hr = store_links(tb, i, j, k, off, inv32), was = !force && (tb.kind[r] & kHardRow);
+        if (hr != was) atomicAdd(hard, hr ? 1 : -1);
+        tb.kind[r] = (int8_t)(kind + (hr ? kHardRow : 0));
     }
 }
 
@@ -407,11 +426,12 @@ __device__ __forceinline__ double plus_zero(double v) {
 __global__ void __launch_bounds__(kBlock) k_t_rhs(Grid g, double inv_dt, double in0, double in1, TBuf tb,
                                                   int nrhs, const double* f0, const double* f1,
                                                   const double* __restrict__ x0, const double* __restrict__ x1,
+                                                  const int* __restrict__ hard, double* __restrict__ hard_out,
                                                   double* __restrict__ partials) {
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
     unsigned int nz[2] = {0u, 0u};
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < (int)g.N; r += gridDim.x * blockDim.x) {
-        const int kind = tb.kind[r];
+        const int kind = row_kind(tb.kind[r]);
         const double inv = tb.inv[r];
         for (int q = 0; q < nrhs; ++q) {
             const double fv = (q ? f1 : f0)[r];
@@ -431,16 +451,22 @@ __global__ void __launch_bounds__(kBlock) k_t_rhs(Grid g, double inv_dt, double 
     }
     acc[2] = (double)nz[0];
     acc[3] = (double)nz[1];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *hard_out = (double)*hard;  // read with the sums
     block_sum_store<4>(acc, partials);
 }
 
-__global__ void k_set_ones(double* v) { v[threadIdx.x] = 1.0; }
+// after k_t_setup, which counts no nonzero rows
+__global__ void k_t_counts(const int* __restrict__ hard, double* __restrict__ v) {
+    v[0] = v[1] = 1.0;
+    v[2] = (double)*hard;
+}
 
 // identity rows take their value
 __global__ void k_t_xid(Grid g, TBuf tb, double* x0, double* x1, int nrhs) {
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < g.N;
          r += (long long)gridDim.x * blockDim.x) {
-        if (tb.kind[r] != 1 && tb.kind[r] != 3) continue;
+        const int kind = row_kind(tb.kind[r]);
+        if (kind != 1 && kind != 3) continue;
         x0[r] = tb.b[0][r];
         if (nrhs > 1) x1[r] = tb.b[1][r];
     }
@@ -662,17 +688,17 @@ struct SrcRhs {
     }
 };
 
-// sum over the six links of the elements of colour COLOUR in chunk ch, times the other colour's
+// sum over the six links of the elements of a colour in chunk ch, times the other colour's
 // values; near = the other colour's chunk at the same place
-template <int NQ, int COLOUR, typename SRC>
-__device__ __forceinline__ Chunk<NQ> rb_links(const RBGrid& g, const TIVec& iv, int ch, const SRC& src,
+template <int NQ, typename SRC>
+__device__ __forceinline__ Chunk<NQ> rb_links(const RBGrid& g, const TIVec& iv, int colour, int ch, const SRC& src,
                                               Chunk<NQ>& near) {
     constexpr int W = 4 / NQ;
     const int h = ch * W;
     const int row = (int)fdiv(NQ == 1 ? g.div4 : g.div2, (unsigned int)ch);
     const int i = (int)fdiv(g.div_j, (unsigned int)row);
-    const bool odd = ((row - i * g.J + i) & 1) != COLOUR;  // odd k: the far neighbour is at h + 1
-    const long long base = COLOUR * g.H;
+    const bool odd = ((row - i * g.J + i) & 1) != colour;  // odd k: the far neighbour is at h + 1
+    const long long base = colour * g.H;
     float l[6][W];
 #pragma unroll
     for (int d = 0; d < 6; ++d) ld_link<NQ>(iv.o[d] + base, h, l[d]);
@@ -732,7 +758,7 @@ __global__ void __launch_bounds__(kBlock) k_rb_init(RBGrid g, int pad, TIVec iv,
         const int h = ch * (4 / NQ);
         const Chunk<NQ> fb = black.chunk(h);
         Chunk<NQ> fr;
-        const Chunk<NQ> y = rb_links<NQ, 0>(g, iv, ch, red, fr);
+        const Chunk<NQ> y = rb_links<NQ>(g, iv, 0, ch, red, fr);
         Chunk<NQ> r;
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
@@ -766,7 +792,7 @@ __global__ void __launch_bounds__(kBlock) k_rb_z(RBGrid g, TIVec iv, const float
     const SrcVec<NQ> src{x};
     for (int ch = blockIdx.x * blockDim.x + threadIdx.x; ch < n; ch += gridDim.x * blockDim.x) {
         Chunk<NQ> near;
-        st_chunk<NQ>(iv.z, ch * (4 / NQ), rb_links<NQ, 1>(g, iv, ch, src, near));
+        st_chunk<NQ>(iv.z, ch * (4 / NQ), rb_links<NQ>(g, iv, 1, ch, src, near));
     }
 }
 
@@ -785,7 +811,7 @@ __global__ void __launch_bounds__(kBlock) k_rb_v(RBGrid g, TIVec iv, const doubl
         const int h = ch * (4 / NQ);
         const Chunk<NQ> p = ld_chunk<NQ>(FIRST ? iv.r : iv.p, h), rh = ld_chunk<NQ>(iv.rh, h);
         Chunk<NQ> near;
-        Chunk<NQ> y = rb_links<NQ, 0>(g, iv, ch, src, near);
+        Chunk<NQ> y = rb_links<NQ>(g, iv, 0, ch, src, near);
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
             y.v[m] = p.v[m] - y.v[m];
@@ -809,7 +835,7 @@ __global__ void __launch_bounds__(kBlock) k_rb_zs(RBGrid g, TIVec iv, const doub
     for (int l = 0; l < NQ; ++l) src.na[l] = -src.na[l];
     for (int ch = blockIdx.x * blockDim.x + threadIdx.x; ch < n; ch += gridDim.x * blockDim.x) {
         Chunk<NQ> near;
-        st_chunk<NQ>(iv.z, ch * (4 / NQ), rb_links<NQ, 1>(g, iv, ch, src, near));
+        st_chunk<NQ>(iv.z, ch * (4 / NQ), rb_links<NQ>(g, iv, 1, ch, src, near));
     }
 }
 
@@ -830,7 +856,7 @@ __global__ void __launch_bounds__(kBlock) k_rb_t(RBGrid g, TIVec iv, const doubl
         const int h = ch * (4 / NQ);
         const Chunk<NQ> r = ld_chunk<NQ>(iv.r, h), v = ld_chunk<NQ>(iv.v, h), rh = ld_chunk<NQ>(iv.rh, h);
         Chunk<NQ> near;
-        Chunk<NQ> t = rb_links<NQ, 0>(g, iv, ch, src, near);
+        Chunk<NQ> t = rb_links<NQ>(g, iv, 0, ch, src, near);
         Chunk<NQ> s;
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
@@ -917,7 +943,7 @@ __global__ void __launch_bounds__(kBlock) k_rb_accum(RBGrid g, TIVec iv, const d
     for (int ch = blockIdx.x * blockDim.x + threadIdx.x; ch < n; ch += gridDim.x * blockDim.x) {
         const int h = ch * (4 / NQ);
         Chunk<NQ> d;
-        const Chunk<NQ> y = rb_links<NQ, 1>(g, iv, ch, src, d);
+        const Chunk<NQ> y = rb_links<NQ>(g, iv, 1, ch, src, d);
         const Chunk<NQ> f = red.chunk(h);
         const int row = (int)fdiv(NQ == 1 ? g.div4 : g.div2, (unsigned int)ch), i = (int)fdiv(g.div_j, (unsigned int)row);
         const int k2 = h - row * g.K2p, j = row - i * g.J;
@@ -944,6 +970,111 @@ __global__ void __launch_bounds__(kBlock) k_rb_accum(RBGrid g, TIVec iv, const d
             }
         }
     }
+}
+
+// The whole system (one right-hand side): the same iteration on vectors of both colours, black
+// from element 0 and red from element cs, with v = p + O p and t = s + O s, both colours' links in
+// one pass, twice the iterations. Where rows' links outweigh their diagonal (sum |O| > 1) the two
+// forms differ: with many such rows the reduced one holds longer (33x35x37, sums up to 50: 28
+// iterations, this one diverges); with a few extreme ones among ordinary rows (2e6 in four of 84) it
+// fails, its right-hand side and products taking up FP32's rounding times the sums, and this one
+// takes 39.
+__global__ void __launch_bounds__(kBlock) k_rw_init(RBGrid g, int cs, int pad, TIVec iv, double* __restrict__ partials) {
+    float acc[2] = {0.f, 0.f};
+    const int n = (int)(g.H / 4), stride = gridDim.x * blockDim.x;
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int c = t0; c < 2 * n; c += stride) {
+        const int colour = c >= n, h = 4 * (c - colour * n), at = h + colour * cs;
+        const Chunk<1> f = ld_chunk<1>(iv.rhs[0] + colour * g.H, h);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) acc[0] = __fmaf_rn(f.v[m], f.v[m], acc[0]);
+        st_chunk<1>(iv.r, at, f);
+        st_chunk<1>(iv.rh, at, f);
+        st_chunk<1>(iv.d, at, Chunk<1>{{0.f, 0.f, 0.f, 0.f}});
+    }
+    // zeros before, between and after the colours
+    float* const vecs[7] = {iv.r, iv.rh, iv.p, iv.v, iv.s, iv.t, iv.d};
+    for (int q = t0; q < pad; q += stride)
+#pragma unroll
+        for (int v = 0; v < 7; ++v) {
+            vecs[v][-1 - q] = 0.f;
+            vecs[v][g.H + q] = 0.f;
+            vecs[v][cs + g.H + q] = 0.f;
+        }
+    acc[1] = acc[0];
+    ti_block_sum<2>(acc, partials);
+}
+
+template <bool FIRST>
+__global__ void __launch_bounds__(kBlock) k_rw_v(RBGrid g, int cs, TIVec iv, const double* __restrict__ scal,
+                                                 double* __restrict__ partials) {
+    pdl_enter();
+    if (scal[TI_ANY] == 0.0) return;
+    float acc[1] = {0.f};
+    const int n = (int)(g.H / 4);
+    const float* const x = FIRST ? iv.r : iv.p;
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < 2 * n; c += gridDim.x * blockDim.x) {
+        const int colour = c >= n, ch = c - colour * n, at = 4 * ch + colour * cs;
+        const Chunk<1> p = ld_chunk<1>(x, at), rh = ld_chunk<1>(iv.rh, at);
+        Chunk<1> near;
+        Chunk<1> y = rb_links<1>(g, iv, colour, ch, SrcVec<1>{x + (colour ? 0 : cs)}, near);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            y.v[m] = p.v[m] + y.v[m];
+            acc[0] = __fmaf_rn(rh.v[m], y.v[m], acc[0]);
+        }
+        st_chunk<1>(iv.v, at, y);
+        if (FIRST) st_chunk<1>(iv.p, at, p);
+    }
+    ti_block_sum<1>(acc, partials);
+}
+
+__global__ void __launch_bounds__(kBlock) k_rw_t(RBGrid g, int cs, TIVec iv, const double* __restrict__ scal,
+                                                 double* __restrict__ partials) {
+    pdl_enter();
+    if (scal[TI_ANY] == 0.0) return;
+    float a[1], acc[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+    ti_scal<1>(scal, TI_ALPHA, a);
+    const int n = (int)(g.H / 4);
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < 2 * n; c += gridDim.x * blockDim.x) {
+        const int colour = c >= n, ch = c - colour * n, at = 4 * ch + colour * cs, other = colour ? 0 : cs;
+        const Chunk<1> rh = ld_chunk<1>(iv.rh, at), s = SrcS<1>{iv.r, iv.v, {-a[0]}}.chunk(at);
+        Chunk<1> near;
+        Chunk<1> t = rb_links<1>(g, iv, colour, ch, SrcS<1>{iv.r + other, iv.v + other, {-a[0]}}, near);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            t.v[m] = s.v[m] + t.v[m];
+            acc[0] = __fmaf_rn(t.v[m], s.v[m], acc[0]);
+            acc[1] = __fmaf_rn(t.v[m], t.v[m], acc[1]);
+            acc[2] = __fmaf_rn(rh.v[m], s.v[m], acc[2]);
+            acc[3] = __fmaf_rn(rh.v[m], t.v[m], acc[3]);
+            acc[4] = __fmaf_rn(s.v[m], s.v[m], acc[4]);
+        }
+        st_chunk<1>(iv.s, at, s);
+        st_chunk<1>(iv.t, at, t);
+    }
+    ti_block_sum<5>(acc, partials);
+}
+
+// x += d
+__global__ void __launch_bounds__(kBlock) k_rw_accum(RBGrid g, int cs, TIVec iv, double* __restrict__ x) {
+    pdl_enter();
+    const int n = (int)(g.H / 4);
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < 2 * n; c += gridDim.x * blockDim.x) {
+        const int colour = c >= n, ch = c - colour * n, h = 4 * ch;
+        const Chunk<1> d = ld_chunk<1>(iv.d, h + colour * cs);
+        const int row = (int)fdiv(g.div4, (unsigned int)ch), i = (int)fdiv(g.div_j, (unsigned int)row);
+        const int j = row - i * g.J, k0 = 2 * (h - row * g.K2p) + ((i + j + colour) & 1);
+        const long long base = (long long)i * g.si + (long long)j * g.sj;
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+            if (k0 + 2 * m < g.K) x[base + (k0 + 2 * m) * g.sk] += widen(d.v[m]);
+    }
+}
+
+__global__ void k_t_copy(long long n, const double* __restrict__ from, double* __restrict__ to) {
+    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < n; r += (long long)gridDim.x * blockDim.x)
+        to[r] = from[r];
 }
 
 __device__ __forceinline__ bool finite_d(double v) { return v == v && fabs(v) < INFINITY; }
@@ -1133,6 +1264,7 @@ static ls_status t_alloc(ls_ctx* c) {
             LS_CUDA(c, cudaMemsetAsync(c->trhs[q], 0, sizeof(float) * m, c->stream));
         }
     if (!c->tkind) LS_TRY(walloc_t(c, &c->tkind, n));
+    if (!c->t_hard) LS_TRY(dalloc_t(c, &c->t_hard, 1));
     return LS_OK;
 }
 
@@ -1149,53 +1281,73 @@ static TBuf make_tbuf(ls_ctx* c) {
 
 // Inner solve of the right-hand sides lane_q[0..NQ-1] (indices into trhs / x), each to its
 // relative tolerance tol[l]; the correction is added to x[lane_q[l]]. Returns the
-// iterations of each lane.
-template <int NQ>
+// iterations of each lane. WHOLE (one right-hand side): the whole system instead of the reduced one.
+template <int NQ, bool WHOLE>
 static ls_status inner_solve(ls_ctx* c, const TBuf& tb, const int lane_q[NQ], const double tol[NQ],
-                             int max_it, double* x[2], int its[NQ]) {
+                             int max_it, double* const x[2], int its[NQ]) {
+    static_assert(!WHOLE || NQ == 1, "the vectors hold both colours of one right-hand side");
     const Grid g = c->g;
     const RBGrid rb = tb.rb;
-    const int grid = grid_for(c, rb.H / (4 / NQ));
+    const int pad = (int)c->ti_pad, cs = (int)rb.H + pad;  // WHOLE: red follows black and a pad
+    const int grid = grid_for(c, WHOLE ? rb.H / 2 : rb.H / (4 / NQ));
     // the kernels with dots: four blocks per SM are resident together (up to 56 registers a
     // thread), and more would only add partial sums
     const int dgrid = std::min(grid, 4 * c->num_sms);
     TIVec iv;
     float** vecs[kTiVecs] = {&iv.r, &iv.rh, &iv.p, &iv.v, &iv.s, &iv.t, &iv.d, &iv.z};
-    for (int v = 0; v < kTiVecs; ++v) *vecs[v] = c->ti + (size_t)v * c->ti_stride + 2 * c->ti_pad;
-    iv.rhs[0] = c->trhs[lane_q[0]] + c->ti_pad;
-    iv.rhs[1] = c->trhs[NQ > 1 ? lane_q[1] : lane_q[0]] + c->ti_pad;
+    if (WHOLE) {  // seven vectors of 2 H + 3 pad elements in the room of eight of 2 (H + 2 pad)
+        for (int v = 0; v < kTiVecs - 1; ++v) *vecs[v] = c->ti + (size_t)v * (2 * (size_t)rb.H + 3 * pad) + pad;
+        iv.z = nullptr;
+    } else {
+        for (int v = 0; v < kTiVecs; ++v) *vecs[v] = c->ti + (size_t)v * c->ti_stride + 2 * pad;
+    }
+    iv.rhs[0] = c->trhs[lane_q[0]] + pad;
+    iv.rhs[1] = c->trhs[NQ > 1 ? lane_q[1] : lane_q[0]] + pad;
     for (int d = 0; d < 6; ++d) iv.o[d] = tb.o[d];
+    RBGrid el = rb;  // what the element-wise passes run over
+    if (WHOLE) el.H = cs + rb.H;
     const double t0 = tol[0] * tol[0], t1 = NQ > 1 ? tol[1] * tol[1] : 0.0;
-    LS_LAUNCH(c, k_rb_init<NQ>, dgrid, kBlock, 0, rb, (int)c->ti_pad, iv, c->partials);
+    const double* const scal = c->scal;
+    if constexpr (WHOLE) LS_LAUNCH(c, k_rw_init, dgrid, kBlock, 0, rb, cs, pad, iv, c->partials);
+    else LS_LAUNCH(c, k_rb_init<NQ>, dgrid, kBlock, 0, rb, pad, iv, c->partials);
     LS_LAUNCH_PDL(c, (k_ti_fin<PH_INIT, NQ>), 1, ti_fin_threads(ti_values(PH_INIT, NQ)), 0, (const double*)c->partials, dgrid,
                   c->scal, t0, t1);
-    // algorithmic bytes of the two operator applications: FP32 off-diagonals (24 per row)
-    // plus per lane 2 bytes for each half-length vector read or written once
+    auto apply_v = [&](bool first) -> ls_status {  // v of p (first: of r, which p takes)
+        Timed tm(c, LS_T_KRY_APPLY);
+        if constexpr (WHOLE) {
+            if (first) LS_LAUNCH_PDL(c, k_rw_v<true>, dgrid, kBlock, 0, rb, cs, iv, scal, c->partials);
+            else LS_LAUNCH_PDL(c, k_rw_v<false>, dgrid, kBlock, 0, rb, cs, iv, scal, c->partials);
+        } else {
+            LS_LAUNCH_PDL(c, k_rb_z<NQ>, grid, kBlock, 0, rb, iv, (const float*)(first ? iv.r : iv.p), scal);
+            if (first) LS_LAUNCH_PDL(c, (k_rb_v<NQ, true>), dgrid, kBlock, 0, rb, iv, scal, c->partials);
+            else LS_LAUNCH_PDL(c, (k_rb_v<NQ, false>), dgrid, kBlock, 0, rb, iv, scal, c->partials);
+        }
+        return LS_OK;
+    };
+    auto apply_t = [&]() -> ls_status {  // s and t
+        Timed tm(c, LS_T_KRY_APPLY);
+        if constexpr (WHOLE) {
+            LS_LAUNCH_PDL(c, k_rw_t, dgrid, kBlock, 0, rb, cs, iv, scal, c->partials);
+        } else {
+            LS_LAUNCH_PDL(c, k_rb_zs<NQ>, grid, kBlock, 0, rb, iv, scal);
+            LS_LAUNCH_PDL(c, k_rb_t<NQ>, dgrid, kBlock, 0, rb, iv, scal, c->partials);
+        }
+        return LS_OK;
+    };
+    // algorithmic bytes of the two operator applications: FP32 off-diagonals (24 per row) plus per
+    // lane 2 bytes for each half-length vector (WHOLE: 4 for each vector) read or written once
     const double v_bytes = (double)g.N * (24.0 + 12.0 * NQ);
-    const double st_bytes = (double)g.N * (24.0 + 18.0 * NQ);
+    const double st_bytes = (double)g.N * (24.0 + (WHOLE ? 20.0 : 18.0 * NQ));
     int it = 0, batch = 4;
     double sc[TI_STRIDE * 2 + 8];
     while (it < max_it) {
         const int nb = std::min(batch, max_it - it);
         for (int b = 0; b < nb; ++b, ++it) {
-            if (it > 0) LS_LAUNCH_PDL(c, k_rb_xp<NQ>, grid, kBlock, 0, rb, iv, (const double*)c->scal);
-            {
-                Timed tm(c, LS_T_KRY_APPLY);
-                LS_LAUNCH_PDL(c, k_rb_z<NQ>, grid, kBlock, 0, rb, iv, (const float*)(it == 0 ? iv.r : iv.p),
-                              (const double*)c->scal);
-                if (it == 0)
-                    LS_LAUNCH_PDL(c, (k_rb_v<NQ, true>), dgrid, kBlock, 0, rb, iv, (const double*)c->scal, c->partials);
-                else
-                    LS_LAUNCH_PDL(c, (k_rb_v<NQ, false>), dgrid, kBlock, 0, rb, iv, (const double*)c->scal,
-                                  c->partials);
-            }
+            if (it > 0) LS_LAUNCH_PDL(c, k_rb_xp<NQ>, grid, kBlock, 0, el, iv, scal);
+            LS_TRY(apply_v(it == 0));
             LS_LAUNCH_PDL(c, (k_ti_fin<PH_V, NQ>), 1, ti_fin_threads(ti_values(PH_V, NQ)), 0, (const double*)c->partials, dgrid,
                           c->scal, 0.0, 0.0);
-            {
-                Timed tm(c, LS_T_KRY_APPLY);
-                LS_LAUNCH_PDL(c, k_rb_zs<NQ>, grid, kBlock, 0, rb, iv, (const double*)c->scal);
-                LS_LAUNCH_PDL(c, k_rb_t<NQ>, dgrid, kBlock, 0, rb, iv, (const double*)c->scal, c->partials);
-            }
+            LS_TRY(apply_t());
             LS_LAUNCH_PDL(c, (k_ti_fin<PH_ST, NQ>), 1, ti_fin_threads(ti_values(PH_ST, NQ)), 0, (const double*)c->partials, dgrid,
                           c->scal, 0.0, 0.0);
         }
@@ -1214,15 +1366,16 @@ static ls_status inner_solve(ls_ctx* c, const TBuf& tb, const int lane_q[NQ], co
             }
         }
     }
-    LS_LAUNCH_PDL(c, k_rb_pending<NQ>, grid, kBlock, 0, rb, iv, (const double*)c->scal);
+    LS_LAUNCH_PDL(c, k_rb_pending<NQ>, grid, kBlock, 0, el, iv, scal);
     double* const xl[2] = {x[lane_q[0]], NQ > 1 ? x[lane_q[1]] : (double*)nullptr};
-    if (rb.axis == 2 && g.K % 2 == 0) LS_LAUNCH_PDL(c, (k_rb_accum<NQ, true>), grid, kBlock, 0, rb, iv, (const double*)c->scal, xl[0], xl[1]);
-    else LS_LAUNCH_PDL(c, (k_rb_accum<NQ, false>), grid, kBlock, 0, rb, iv, (const double*)c->scal, xl[0], xl[1]);
+    if constexpr (WHOLE) LS_LAUNCH_PDL(c, k_rw_accum, grid, kBlock, 0, rb, cs, iv, xl[0]);
+    else if (rb.axis == 2 && g.K % 2 == 0) LS_LAUNCH_PDL(c, (k_rb_accum<NQ, true>), grid, kBlock, 0, rb, iv, scal, xl[0], xl[1]);
+    else LS_LAUNCH_PDL(c, (k_rb_accum<NQ, false>), grid, kBlock, 0, rb, iv, scal, xl[0], xl[1]);
     for (int l = 0; l < NQ; ++l) its[l] = (int)sc[TI_STRIDE * l + TI_ITS];
     // the launches of a batch beyond the last iteration return at once and move nothing
     if (c->timing) {
         const int live = NQ > 1 ? std::max(its[0], its[NQ - 1]) : its[0];
-        c->timer_bytes[LS_T_KRY_APPLY] += live * (v_bytes + st_bytes) + (live > 0 ? 2.0 * NQ * g.N : 0.0);
+        c->timer_bytes[LS_T_KRY_APPLY] += live * (v_bytes + st_bytes) + (live > 0 ? (WHOLE ? 4.0 : 2.0) * NQ * g.N : 0.0);
     }
     return LS_OK;
 }
@@ -1252,30 +1405,34 @@ static ls_status mixed_solve(ls_ctx* c, const Rows<L>& rows, int nrhs, const dou
             c->t_valid = 0;
         }
         const int force = (!c->t_valid || memcmp(consts, c->t_consts, sizeof(consts)) != 0) ? 1 : 0;
+        if (force) LS_CUDA(c, cudaMemsetAsync(c->t_hard, 0, sizeof(int), c->stream));
+        c->t_valid = 0;  // until the rows, their marks and the count belong together again
         LS_TRY(wlist_reset(c));
         LS_LAUNCH(c, k_t_dirty<L>, grid, kBlock, 0, g, rows.label, rows.fx, rows.fy, rows.fz,
                   (L*)c->sht_label, c->sht_fx, c->sht_fy, c->sht_fz, c->dbits, force);
         const int per = scan_words(c->num_sms, g.N);
         LS_LAUNCH(c, k_t_scan, scan_grid(c->num_sms, g.N, per), kBlock, 0, g, (const unsigned int*)c->dbits, c->dwords,
                   per, c->wlist, c->wcount);
-        LS_LAUNCH(c, k_t_rows<L>, grid, kBlock, 0, rows, tb, (const int*)c->wlist, (const unsigned int*)c->wcount);
+        LS_LAUNCH(c, k_t_rows<L>, grid, kBlock, 0, rows, tb, force, (const int*)c->wlist, (const unsigned int*)c->wcount,
+                  c->t_hard);
         LS_LAUNCH(c, k_t_rhs, grid, kBlock, 0, g, rows.tc.inv_dt, rows.tc.in_val[0], rows.tc.in_val[1], tb, nrhs,
-                  f0, f1, (const double*)x0, (const double*)x1, c->partials);
+                  f0, f1, (const double*)x0, (const double*)x1, (const int*)c->t_hard, c->scal + S_RED0 + 8, c->partials);
         LS_TRY(finalize_sum(c, grid, 4, S_RED0 + 4));
         memcpy(c->t_consts, consts, sizeof(consts));
         c->t_valid = 1;
     } else {
+        LS_CUDA(c, cudaMemsetAsync(c->t_hard, 0, sizeof(int), c->stream));
         if (rows.mode == 0)
-            LS_LAUNCH(c, (k_t_setup<L, true>), grid, kBlock, 0, rows, tb, nrhs, f0, f1, c->partials);
+            LS_LAUNCH(c, (k_t_setup<L, true>), grid, kBlock, 0, rows, tb, nrhs, f0, f1, c->t_hard, c->partials);
         else
-            LS_LAUNCH(c, (k_t_setup<L, false>), grid, kBlock, 0, rows, tb, nrhs, f0, f1, c->partials);
+            LS_LAUNCH(c, (k_t_setup<L, false>), grid, kBlock, 0, rows, tb, nrhs, f0, f1, c->t_hard, c->partials);
         LS_TRY(finalize_sum(c, grid, 2, S_RED0 + 4));
-        LS_LAUNCH(c, k_set_ones, 1, 2, 0, c->scal + S_RED0 + 6);
+        LS_LAUNCH(c, k_t_counts, 1, 1, 0, (const int*)c->t_hard, c->scal + S_RED0 + 6);
         c->t_valid = 0;  // the row buffers now hold other rows
     }
     LS_LAUNCH(c, k_t_xid, grid, kBlock, 0, g, tb, x0, x1, nrhs);
-    double den[4];
-    LS_TRY(read_scalars(c, S_RED0 + 4, 4, den));
+    double den[5];
+    LS_TRY(read_scalars(c, S_RED0 + 4, 5, den));
     int mask = nrhs > 1 ? 3 : 1;
     int its[2] = {0, 0}, sweeps[2] = {0, 0}, reason[2] = {0, 0};
     // a system with b = 0 and x = 0 on every row is solved exactly: no residual pass
@@ -1288,6 +1445,25 @@ static ls_status mixed_solve(ls_ctx* c, const Rows<L>& rows, int nrhs, const dou
     }
     double rel[2] = {0.0, 0.0}, prev[2] = {INFINITY, INFINITY};
     int stagnant[2] = {0, 0}, floored[2] = {0, 0};
+    // Hard rows: the first solution is kept (without memory for it the reduced solve is all there is),
+    // and a lane whose reduced solve ends without convergence starts again from it on the whole
+    // system, with all of max_it.
+    bool whole[2] = {false, false}, kept[2] = {false, false};
+    double* const xs[2] = {x0, x1};
+    if (den[4] > 0.0)
+        for (int q = 0; q < nrhs; ++q) {
+            if (!((mask >> q) & 1)) continue;
+            if (!c->t_keep[q]) dalloc_t(c, &c->t_keep[q], (size_t)g.N);
+            kept[q] = c->t_keep[q] != nullptr;
+            if (kept[q]) LS_LAUNCH(c, k_t_copy, grid, kBlock, 0, g.N, (const double*)xs[q], c->t_keep[q]);
+        }
+    auto restart = [&](int q) {
+        if (!kept[q] || whole[q]) return false;
+        whole[q] = true;
+        its[q] = sweeps[q] = stagnant[q] = floored[q] = 0;
+        prev[q] = INFINITY;
+        return true;
+    };
     const int max_sweeps = 40;
     const double inner_floor = 1e-6;
     while (mask) {
@@ -1306,23 +1482,30 @@ static ls_status mixed_solve(ls_ctx* c, const Rows<L>& rows, int nrhs, const dou
         double h[4];
         LS_TRY(read_scalars(c, S_RED0, 4, h));
         int solve_mask = 0;
+        bool again = false;
         double tol[2] = {0.5, 0.5};
         for (int q = 0; q < nrhs; ++q) {
             if (!((mask >> q) & 1)) continue;
-            if (h[2 + q] > 0.0 || h[q] != h[q]) { reason[q] = -4; rel[q] = NAN; mask &= ~(1 << q); continue; }
-            rel[q] = den[q] > 0.0 ? sqrt(h[q] / den[q]) : sqrt(h[q]);
+            const bool bad = h[2 + q] > 0.0 || h[q] != h[q];
+            rel[q] = bad ? NAN : den[q] > 0.0 ? sqrt(h[q] / den[q]) : sqrt(h[q]);
             // A sweep aims at 0.2 rtol. One that the floor of the inner tolerance stopped above
             // that is followed by another (an iteration or two) while the residual still falls,
             // so that the margin holds at tight tolerances too.
             const bool refine = floored[q] && rel[q] > 0.3 * rtol && rel[q] <= 0.5 * prev[q] && its[q] < max_it &&
                                 sweeps[q] < max_sweeps;
-            if ((rel[q] <= rtol && !refine) || h[q] == 0.0) { reason[q] = 2; mask &= ~(1 << q); continue; }
-            if (its[q] >= max_it || sweeps[q] >= max_sweeps) { reason[q] = -3; mask &= ~(1 << q); continue; }
-            if (rel[q] > 0.5 * prev[q]) {
-                if (++stagnant[q] >= 6) { reason[q] = -3; mask &= ~(1 << q); continue; }
-            } else {
-                stagnant[q] = 0;
+            if (!bad && ((rel[q] <= rtol && !refine) || h[q] == 0.0)) { reason[q] = 2; mask &= ~(1 << q); continue; }
+            const bool still = rel[q] > 0.5 * prev[q];
+            if (bad || its[q] >= max_it || sweeps[q] >= max_sweeps || (still && stagnant[q] >= 5)) {
+                if (sweeps[q] > 0 && restart(q)) {
+                    LS_LAUNCH(c, k_t_copy, grid, kBlock, 0, g.N, (const double*)c->t_keep[q], xs[q]);
+                    again = true;
+                } else {
+                    reason[q] = bad ? -4 : -3;
+                    mask &= ~(1 << q);
+                }
+                continue;
             }
+            stagnant[q] = still ? stagnant[q] + 1 : 0;
             prev[q] = rel[q];
             // inner tolerance: what reaches rtol from here (with a margin), floored at what
             // the FP32 inner system still resolves (a relative 1e-6 is ~17 FP32 ulps)
@@ -1331,20 +1514,25 @@ static ls_status mixed_solve(ls_ctx* c, const Rows<L>& rows, int nrhs, const dou
             tol[q] = std::min(0.5, std::max(inner_floor, want));
             solve_mask |= 1 << q;
         }
-        if (!solve_mask) break;
-        int lane_q[2] = {0, 0}, nq = 0;
-        for (int q = 0; q < 2; ++q)
-            if ((solve_mask >> q) & 1) lane_q[nq++] = q;
-        const double ltol[2] = {tol[lane_q[0]], tol[lane_q[nq - 1]]};
-        int lits[2] = {0, 0};
+        if (!solve_mask && !again) break;
         const int budget = std::max(1, max_it - std::max(its[0], its[1]));
-        double* xs[2] = {x0, x1};
-        if (nq == 2) LS_TRY(inner_solve<2>(c, tb, lane_q, ltol, budget, xs, lits));
-        else LS_TRY(inner_solve<1>(c, tb, lane_q, ltol, budget, xs, lits));
-        for (int l = 0; l < nq; ++l) { its[lane_q[l]] += lits[l]; sweeps[lane_q[l]]++; }
+        int lane_q[2] = {0, 0}, nq = 0, lits[2] = {0, 0};
+        for (int q = 0; q < 2; ++q) {
+            if (!((solve_mask >> q) & 1)) continue;
+            sweeps[q]++;
+            if (!whole[q]) {
+                lane_q[nq++] = q;
+                continue;
+            }
+            LS_TRY((inner_solve<1, true>(c, tb, &q, &tol[q], budget, xs, lits)));
+            its[q] += lits[0];
+        }
+        const double ltol[2] = {tol[lane_q[0]], tol[lane_q[nq > 1 ? 1 : 0]]};
+        if (nq == 2) LS_TRY((inner_solve<2, false>(c, tb, lane_q, ltol, budget, xs, lits)));
+        else if (nq == 1) LS_TRY((inner_solve<1, false>(c, tb, lane_q, ltol, budget, xs, lits)));
+        for (int l = 0; l < nq; ++l) its[lane_q[l]] += lits[l];
     }
     ls_status st = LS_OK;
-    double* xs[2] = {x0, x1};
     for (int q = 0; q < nrhs; ++q) {
         double mm[2] = {0.0, -0.0};  // max x, max -x
         if (den[2 + q] != 0.0) {  // otherwise x = 0 on every row
