@@ -43,6 +43,11 @@ constexpr int kKSlot0 = 32;   // device scalar slots of the K-cycle FCG (5 per l
 // at 48x64x64 (24,576, 3,072, 384) took 48.8 ms without the 3,072-cell level and 46.7 with it.
 constexpr long long kFuseCells32 = 9000;
 constexpr long long kFuseCells64 = 8192;
+// FP64 with at most this many cells on the coarsest level keeps the level kernels: its 48 sweeps cost 48
+// cluster barriers, and one SM does them faster. Cold solves, fused and not: 40x40x40 (125 cells)
+// 10.3 and 8.1 ms, 128x160x120 (80) 41.4 and 33.1, 61x83x101 (168) 21.6 and 20.1, 48x48x48 (216) 10.2
+// and 10.0, 48x52x48 (252) 9.6 and 9.9, 64x48x48 (288) 12.3 and 13.5, 64x64x64 (512) 13.3 and 19.3.
+constexpr long long kFuseCoarsest64 = 232;
 constexpr int kUnionSpin = 1 << 20;  // bound on the union-find retry loop
 // learned coarse solver (LS_PRESS_LEARNED): the network solves level kLearnedLevel in place of
 // the V-cycle below the K-cycle levels
@@ -1276,7 +1281,8 @@ ls_status mg_apply(ls_ctx* c, const T* r, T* z, const T* dotv2, int* nblocks_out
     // the levels from `fuse` down run as one launch each time they are visited (k_mg_fused)
     size_t fuse = L + 1, fuse_smem = 0;
     FuseArgs<T> fa = {};
-    if (!learned && c->mg_cluster > 0) {
+    const bool small64 = sizeof(T) == 8 && c->mg_tail_cells < 0 && lv[L].g.N <= kFuseCoarsest64;
+    if (!learned && !small64 && c->mg_cluster > 0) {
         for (size_t l = L >= (size_t)kMaxFuse ? L + 1 - kMaxFuse : 1; l <= L && fuse > L; ++l) {
             if (lv[l].g.N > fuse_cells<T>(c)) continue;
             fa = {};
