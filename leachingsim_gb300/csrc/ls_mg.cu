@@ -36,12 +36,14 @@ constexpr int kCoarseSweeps = 48;
 constexpr double kProlongScale = 1.8;
 constexpr int kKLevels = 3;   // levels 1..kKLevels take a K-cycle coarse correction
 constexpr int kKSlot0 = 32;   // device scalar slots of the K-cycle FCG (5 per level)
-// Levels up to these sizes run fused (k_mg_fused). Beyond them 16 SMs take longer for a step than
-// the whole GPU and a launch: with bounds of 3,000 / 9,000 / 30,000 / 50,000 cells a run at
-// 64x64x64 (levels of 32,768, 4,096 and 512) took 74.9 / 73.9 / 74.8 / 74.8 ms, a step of the
-// 224x320x320 flow-through model (44,800, 5,600, 700, 100) 103.7 / 104.3 / 104.5 / 104.5; in FP64 a run
-// at 48x64x64 (24,576, 3,072, 384) took 48.8 ms without the 3,072-cell level and 46.7 with it.
-constexpr long long kFuseCells32 = 9000;
+// Levels up to these sizes run fused (k_mg_fused). FP32: one block with a cell per thread; a level of two
+// cells per thread, or one on the cluster, takes longer than its kernels do. With the largest fused
+// level just left out and taken in, ms: 80x80x80 (1,000 cells) 6.14 and 6.04; 61x83x101, implicit
+// saturation (1,144) 124.7 and 126.1; 101x77x95 (1,560) 7.8 and 8.1; 200x160x240 (1,950) 17.8 and
+// 19.5; 160x256x256 (2,560) 18.2 and 19.8; 64x64x64 with acid (4,096) 58.9 and 61.0; a fractured
+// step of 224x320x320 (5,600) 284 and 300; without any fused level 8.4, 165, 10.7, 21.4, 21.3, 69 and 303.
+// FP64 (48x64x64, 3,072 cells): 26.3 and 26.0.
+constexpr long long kFuseCells32 = 1024;
 constexpr long long kFuseCells64 = 8192;
 // FP64 with at most this many cells on the coarsest level keeps the level kernels: its 48 sweeps cost 48
 // cluster barriers, and one SM does them faster. Cold solves, fused and not: 40x40x40 (125 cells)
