@@ -215,6 +215,7 @@ struct RBGrid {
     int I, J, K, K2p, JK2;
     int axis;        // of the grid, along which the layout's rows run
     int si, sj, sk;  // strides of i, j and k in the voxel arrays
+    int pair;        // from the place of the grid's voxel (i, j, k), k even, to that of (i, j, k + 1)
     long long H;
     FastDiv div4, div2, div_j;  // by K2p / 4, K2p / 2 and J
 };
@@ -239,6 +240,7 @@ static RBGrid make_rb_axis(const Grid& g, int axis) {
     r.sk = stride[axis];
     r.K2p = (((r.K + 1) / 2 + 3) / 4) * 4;
     r.JK2 = r.J * r.K2p;
+    r.pair = axis == 2 ? 0 : r.K2p;
     r.H = (long long)r.I * r.JK2;
     r.div4 = make_fastdiv((unsigned int)(r.K2p / 4));
     r.div2 = make_fastdiv((unsigned int)(r.K2p / 2));
@@ -514,28 +516,26 @@ __global__ void __launch_bounds__(kBlock) k_t_resid(Grid g, TBuf tb, const doubl
         ld_rows<V>(tb.inv, r, inv);
         int colour;
         const int h = rb_index(tb.rb, i, j, k, colour);
-        // rows k and k + 1 (k even) differ in colour only, unless k is not the layout's row axis
-        const int h1 = tb.rb.axis == 2 ? h : h + tb.rb.K2p;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             if (!(MASK >> q & 1)) continue;
             const double* __restrict__ x = q ? x1 : x0;
             double b[V], xc[V], xim[V], xip[V], xjm[V], xjp[V];
             ld_rows<V>(tb.b[q], r, b);
-            ld_rows<V>(x, im, xim);
-            ld_rows<V>(x, jm, xjm);
             ld_rows<V>(x, r, xc);
-            ld_rows<V>(x, jp, xjp);
-            ld_rows<V>(x, ip, xip);
             const double xkm = x[km], xkp = x[kp];
+            ld_rows<V>(x, jm, xjm);
+            ld_rows<V>(x, jp, xjp);
+            ld_rows<V>(x, im, xim);
+            ld_rows<V>(x, ip, xip);
 #pragma unroll
             for (int e = 0; e < V; ++e) {
                 // the diagonal between the lower and the upper links, which have the other sign: taken
                 // first it doubles the partial sums, and their rounding kept the norm above 1.55e-16
                 // where it now reaches 1.25e-16 (long time steps, 32x40x40)
-                double a = __fma_rn(-c[2][e], xim[e], b[e]);
+                double a = __fma_rn(-c[6][e], e == 0 ? xkm : xc[0], b[e]);
                 a = __fma_rn(-c[4][e], xjm[e], a);
-                a = __fma_rn(-c[6][e], e == 0 ? xkm : xc[0], a);
+                a = __fma_rn(-c[2][e], xim[e], a);
                 a = __fma_rn(-c[0][e], xc[e], a);
                 a = __fma_rn(-c[5][e], e == V - 1 ? xkp : xc[V - 1], a);
                 a = __fma_rn(-c[3][e], xjp[e], a);
@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(kBlock) k_t_resid(Grid g, TBuf tb, const doubl
                 const double rv = a * inv[e];
                 // the inner right-hand side in FP32 rounded toward zero on the integer pipe (its
                 // rounding is the inner solve's business)
-                const long long at = (e ? colour ^ 1 : colour) * tb.rb.H + (e ? h1 : h);
+                const long long at = (e ? colour ^ 1 : colour) * tb.rb.H + h + (e ? tb.rb.pair : 0);
                 (q ? r1 : r0)[at] = d2f_rz(rv);
                 acc[q] = __fma_rn(rv, rv, acc[q]);
                 nan[q] += disnan(rv) ? 1 : 0;
