@@ -194,12 +194,11 @@ constexpr int kDzSkew = 7;
 // schedule does not change during a call, so a thread finds its voxel while the level before
 // still runs (programmatic dependent launch: the state is read after griddepcontrol.wait; the
 // next level is let in only then, since levels queued further ahead take the slots of the SMs
-// that should share the current one: 46 ms a call against 25). What a level then takes is the
+// that should share the current one). What a level then takes is the
 // update's chain: one round trip to L2, some 60 FP64 operations of the warp or two that an SM
 // holds, the hand-over to the next launch. A call at 338x338x283 (1,900 levels of 9,000 updates,
-// 20 sub-steps): 36.7 ms with each face's label, acid and division in turn and ordinary
-// launches; 24.8 with the reads together and dependent launches; 12.7 with the quotients from
-// one reciprocal (670 instructions a warp instead of 1,620). At 64x64x64: 7.8 -> 2.2 ms.
+// 20 sub-steps) takes 12.7 ms, against 36.7 with each face's label, acid and division in turn and
+// ordinary launches; at 64x64x64 2.2 against 7.8.
 template <typename L>
 __global__ void __launch_bounds__(kBlock) k_dz_skew(Grid g, DzConst dc, int level, int num_steps, int nlev,
                                                     const int* __restrict__ list, const int* __restrict__ tab,

@@ -483,7 +483,8 @@ __device__ __forceinline__ int lin_point(int s, int p, long long t, long long nu
 // One coordinate of the points t = 0 .. n of a line from s to p, |p - s| <= n < kExactSteps, in
 // integers: rem = (2 t |p - s| + n) mod 2n, pos the rounded point. An exact tie (rem = 0 behind the
 // start) rounds as the floating-point point does, so lin_point decides it; elsewhere the point is
-// 1/(2n) or more from a half, far beyond that point's rounding error of about n 2^-52.
+// 1/(2n) or more from a half, above 2^-21. lin_point's own rounding is below n 2^-52 < 2^-32 (step and
+// product) plus half an ulp of the coordinate, at most 2^-23 below 2^31: together below 2^-22.
 constexpr int kExactSteps = 1 << 20;
 struct LineAxis {
     int s, p, a, dir, n, rem, pos;

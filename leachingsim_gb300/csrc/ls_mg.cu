@@ -85,8 +85,8 @@ __device__ __forceinline__ T m_apply(const Grid& g, long long r, int i, int j, i
 
 // Resident blocks per SM of the passes that hold more than 32 registers and sum nothing, whose
 // grid is that many blocks per SM: with grid_for's 8 a second, partly filled wave followed (the
-// finest sweep with the correction at 338x338x283: 186 us, now 163). 4, 5 or 6: the step with
-// acid there takes 81.1, 80.8 or 81.1 ms. The passes that leave partial sums keep grid_for's
+// finest sweep with the correction at 338x338x283: 186 us, now 165). 4, 5 or 6 blocks: a step with
+// acid there differs by 0.4 %. The passes that leave partial sums keep grid_for's
 // grid, which is part of the order of their sums.
 constexpr int kPassBlocks = 5;
 static int pass_grid(const ls_ctx* c, long long n) { return std::min(grid_for(c, n), c->num_sms * kPassBlocks); }

@@ -3,8 +3,9 @@
 //
 // A K-cycle visits level 3 eight times and the levels below it as often, and a kernel there
 // runs for 3-9 us however few cells it has: launch, two memory round trips, drain. Here one
-// thread-block cluster runs the whole correction from some level down: the K-cycle FCG of that
-// level, the levels below it and the coarsest solve. Each block owns a slab of consecutive cells
+// launch runs the whole correction from some level down: the K-cycle FCG of that level, the
+// levels below it and the coarsest solve. FP32 takes levels of up to a cell per thread, in one block; FP64
+// and LS_MG_TAIL_CELLS above 2,048 take a thread-block cluster. Each of its blocks owns a slab of consecutive cells
 // of every level and holds its coefficients and vectors in shared memory; a new value of an
 // iterate also goes to the halos of the slabs on either side (distributed shared memory), so a
 // sweep reads local shared memory only, and a cluster barrier (about 1 us) ends it. Small levels
@@ -22,10 +23,10 @@
 //
 // What bounds it: a step's issue and shared-memory reads on one SM (a sweep over 1,144 cells 1.1
 // us), the cluster barrier (0.7-1 us), the coarsest sweeps' dependent chain (0.18 us each, 48 of
-// them). Whole runs against a kernel per step with a one-block V-cycle for levels up to 4,096
-// cells: 61x83x101, implicit saturation 259 -> 200 ms; 64x64x64 with acid 86.7 -> 72.4; 32x40x40
-// 13.9 -> 11.8; 48x64x64 with the FP64 solver 57.6 -> 46.8; a cold solve of 160x256x256 34.2 ->
-// 32.2.
+// them). A visit from a level of 320 cells down takes 17 us (160x256x256), from 700 down with its
+// K-cycle 29 (224x320x320). Against level kernels alone: 160x256x256 21.3 and 18.2 ms, 32x40x40
+// (ten steps) 12.2 and 11.0, 48x64x64 with the FP64 solver 30.1 and 26.0; which levels gain is at
+// kFuseCells32 in ls_mg.cu.
 #pragma once
 
 #include <cooperative_groups.h>

@@ -567,8 +567,9 @@ __global__ void __launch_bounds__(kBlock) k_t_resid(Grid g, TBuf tb, const doubl
 // eigenvalues of I + O at 1 -+ mu fold onto 1 - mu^2. The residual of the whole system is the
 // reduced one (its red half is zero by construction), so the stopping test is unchanged: ||r||
 // against ||f||. An iteration moves 94 bytes per voxel for one right-hand side (whole matrix:
-// 112). Against BiCGStab on the whole matrix a two-species solve of 97x128x121 to 1e-12 takes
-// 2.2 ms (4.7), a step at 338x338x283 21.0 ms (29.1) and with acid flowing in 124 ms (151).
+// 112). Two species to 1e-12 with all rows new: 1.46 ms at 97x128x121 (4.43 with BiCGStab on the
+// whole matrix), 18.7 at 338x338x283 (46.5); with unchanged rows 1.38 (4.67) and 16.8 (47.1).
+// Rows whose links outweigh their diagonal by far can defeat it: mixed_solve.
 //
 // NQ right-hand sides go together; with NQ = 2 they share the link loads and each vector
 // element is a float2 with one lane per right-hand side. Every vector has `pad` zero elements
